@@ -1123,9 +1123,9 @@ int upbd_set_fluid_next(upbd_sim* s, int32_t next) {
   return UPBD_OK;
 }
 
-// Solver._recomputeGroups, src/solver.js:488-499 — union-find with path
-// halving over alive constraints in constraint order, on the host over the
-// downloaded alive flags (the same sequential algorithm, so root ids match).
+// Solver._recomputeGroups, src/solver.js:488-499: the root labels of its
+// union-find over the alive constraints in constraint order
+// (upbd_groups.cuh), in scratch from the density pass's neighbour lists.
 int upbd_groups_device(upbd_sim* s, int32_t* d_group) {
   if (!s) return UPBD_ERR_INVALID;
   const int S = s->v.S, C = s->v.C;
@@ -1133,18 +1133,13 @@ int upbd_groups_device(upbd_sim* s, int32_t* d_group) {
   if (!d_group) return UPBD_ERR_INVALID;
   cudaSetDevice(s->device);
   cudaStream_t st = s->stream;
-  int32_t* par = reinterpret_cast<int32_t*>(s->v.tmp);  // the grid's scatter buffer, N >= S words
-  if (S <= GROUPS_SMEM_MAX) {
-    const size_t smem = (size_t)S * sizeof(int32_t);
-    if (smem > 48 * 1024)
-      UPBD_CK(s, cudaFuncSetAttribute(k_groups_replay<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    k_groups_replay<true><<<1, 32, smem, st>>>(s->v.cons, C, S, par);
-  } else {
-    k_groups_replay<false><<<1, 32, 0, st>>>(s->v.cons, C, S, par);
-  }
-  UPBD_KCK(s);
-  k_groups_label<<<blocks_for(S), 256, 0, st>>>(par, S, d_group);
+  const GroupScratch g = group_scratch(s->v.nbr, S, C);
+  k_groups_first<<<blocks_for((long long)S * GRP_LANES), 256, 0, st>>>(s->v.cons, s->v.adj, S, C, g);
+  k_groups_tree<<<blocks_for(S), 256, 0, st>>>(S, g);
+  k_groups_cross<<<blocks_for(C), 256, 0, st>>>(s->v.cons, C, S, g);
+  k_groups_join<<<1, GRP_BLOCK, 0, st>>>(s->v.cons, C, S, g);
+  k_groups_last<<<blocks_for(S), 256, 0, st>>>(S, g);
+  k_groups_label<<<blocks_for(S), 256, 0, st>>>(s->v.cons, S, g, d_group);
   UPBD_KCK(s);
   return UPBD_OK;
 }
