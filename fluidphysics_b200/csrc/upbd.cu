@@ -183,29 +183,47 @@ int launch_substep(upbd_sim* s, int last) {
     UPBD_KCK(s);
     return UPBD_OK;
   }
-  // With two or more plain Jacobi iterations (no tets, no solid contacts)
-  // each iteration is one launch that also applies (b_solid_solve's OUT), and
-  // the displacement pass applies the fluid's move itself. The iterations
-  // before the last read and write solid positions only (pos, sbuf), which no
+  // The solid solve is a sequence of phases (b_solid_solve's OUT): per
+  // iteration the distance solve, the tets and the solid contacts the scene
+  // has. With two or more, each phase is one launch that also applies, and
+  // the displacement pass applies the fluid's move itself. The phases before
+  // the last read and write solid positions only (pos, sbuf), which no
   // pass of the grid build or the fluid gathers writes, so they run on the
-  // side stream meanwhile; the last one also writes the solids' slot copies,
-  // so it waits for the grid build, and still runs beside density and
-  // displacement (they read fluid slots only), followed there by the contact
+  // side stream meanwhile, the contact phases once the grid is built and the
+  // contact cache collected from it; the last one also writes the solids'
+  // slot copies, so it waits for the grid build, and still runs beside density
+  // and displacement (they read fluid slots only), followed there by the contact
   // marks, which read the fluid's grid positions with a reach widened by the
   // displacement limit (the pass that applies the displacement marks the
   // particles that change cell). Eager per-kernel timing keeps one stream
   // and marks from the displaced fluid after the solve.
-  const bool fold = iters >= 2 && !tets && !scc && last >= UPBD_PASS_SOLID;
+  const int per = 1 + (tets ? 1 : 0) + (scc ? 1 : 0), phases = iters * per;
+  const bool fold = phases >= 2 && last >= UPBD_PASS_SOLID;
   const bool overlap = fold && !s->prof_on && s->side;
+  const int early = scc ? per - 1 : phases - 1;  // phases that need no grid
   const int solid_pad = ((v.S * GL + 31) / 32) * 32;  // lane threads of the solve, whole warps
+  const unsigned blk_gl = blocks_for((long long)v.S * GL), blk_gt = blocks_for((long long)v.S * GT);
+  auto solid_phase = [&](cudaStream_t ss, int q, bool mark) {
+    const int kind = q % per;
+    const bool lastq = q == phases - 1;
+    if (kind == 0) {
+      if (!lastq) PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_STEP><<<blocks_for(solid_pad), 256, 0, ss>>>(v, P, solid_pad, q));
+      else if (mark) PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_LAST><<<blocks_for(solid_pad), 256, 0, ss>>>(v, P, solid_pad, q));
+      else PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_FINAL><<<blocks_for(solid_pad), 256, 0, ss>>>(v, P, solid_pad, q));
+    } else if (tets && kind == 1) {
+      if (!lastq) PROF(s, K_SOLVE_TETS, k_solve_tets<false><<<blk_gt, 256, 0, ss>>>(v, P, q));
+      else PROF(s, K_SOLVE_TETS, k_solve_tets<true><<<blk_gt, 256, 0, ss>>>(v, P, q));
+    } else {
+      if (!lastq) PROF(s, K_SOLID_CONTACTS, k_solid_contacts<false><<<blk_gl, 256, 0, ss>>>(v, P, q));
+      else PROF(s, K_SOLID_CONTACTS, k_solid_contacts<true><<<blk_gl, 256, 0, ss>>>(v, P, q));
+    }
+    L++;
+  };
   PROF(s, K_INTEGRATE, k_integrate_count<true, true><<<blocks_for(v.N), 256, 0, st>>>(v, P));
   if (overlap) {
     UPBD_CK(s, cudaEventRecord(s->fork_ev, st));
     UPBD_CK(s, cudaStreamWaitEvent(s->side, s->fork_ev, 0));
-    for (int it = 0; it < iters - 1; it++) {
-      k_solid_solve<false, SOLVE_STEP><<<blocks_for(solid_pad), 256, 0, s->side>>>(v, P, solid_pad, it);
-      L++;
-    }
+    for (int q = 0; q < early; q++) solid_phase(s->side, q, false);
   }
   PROF(s, K_SCAN, k_scan<<<v.num_tiles, SCAN_THREADS, 0, st>>>(v));
   PROF(s, K_SCATTER, k_scatter<<<blocks_for(std::max(v.N, tile_words(v.num_tiles))), 256, 0, st>>>(v));
@@ -215,8 +233,11 @@ int launch_substep(upbd_sim* s, int last) {
   if (overlap) {
     UPBD_CK(s, cudaEventRecord(s->grid_ev, st));
     UPBD_CK(s, cudaStreamWaitEvent(s->side, s->grid_ev, 0));
-    k_solid_solve<false, SOLVE_FINAL><<<blocks_for(solid_pad), 256, 0, s->side>>>(v, P, solid_pad, iters - 1);
-    L++;
+    if (scc) {
+      k_collect_contacts<<<blocks_for((long long)v.S * 32), 256, 0, s->side>>>(v, P);
+      L++;
+    }
+    for (int q = early; q < phases; q++) solid_phase(s->side, q, false);
     // the contact marks from the solids' final positions and the fluid's
     // grid positions (reach widened by the displacement limit), so they run
     // here beside density and displacement rather than after them
@@ -243,49 +264,24 @@ int launch_substep(upbd_sim* s, int last) {
     L++;
     if (last < UPBD_PASS_SOLID) return UPBD_OK;
   }
-  if (scc) {
-    PROF(s, K_COLLECT, k_collect_contacts<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-    L++;
-  }
   // the contact marks ride on the last applyDeltaSolid when that is the last
   // position update of the solve; otherwise they get their own launch
-  const bool mark_in_apply = iters > 0 && !tets && !scc;
-  if (fold) {
-    if (overlap) {
-      UPBD_CK(s, cudaStreamWaitEvent(st, s->join_ev, 0));  // the solve and the marks
-    } else {
-      for (int it = 0; it < iters - 1; it++) {
-        PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_STEP><<<blocks_for(solid_pad), 256, 0, st>>>(v, P, solid_pad, it));
-        L++;
-      }
-      PROF(s, K_SOLID_SOLVE,
-           k_solid_solve<false, SOLVE_LAST><<<blocks_for(solid_pad), 256, 0, st>>>(v, P, solid_pad, iters - 1));
+  const bool mark_in_apply = iters > 0 && per == 1;
+  if (overlap) {
+    UPBD_CK(s, cudaStreamWaitEvent(st, s->join_ev, 0));  // the solve and the marks
+  } else if (fold) {
+    if (scc) {
+      PROF(s, K_COLLECT, k_collect_contacts<<<blocks_for((long long)v.S * 32), 256, 0, st>>>(v, P));
       L++;
     }
-  }
-  for (int it = 0; it < iters && !fold; it++) {
-    if (it == 0)
-      PROF(s, K_SOLID_SOLVE, k_solid_solve<true, SOLVE_DELTA>
-           <<<blocks_for((long long)solid_pad + v.F), 256, 0, st>>>(v, P, solid_pad, it));
-    else
-      PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_DELTA><<<blocks_for(solid_pad), 256, 0, st>>>(v, P, solid_pad, it));
-    if (mark_in_apply && it == iters - 1)
-      PROF(s, K_APPLY_SOLID, k_apply_solid<true><<<blocks_for((long long)v.S * GL), 256, 0, st>>>(v, P));
-    else
-      PROF(s, K_APPLY_SOLID, k_apply_solid<false><<<blocks_for(v.S), 256, 0, st>>>(v, P));
+    for (int q = 0; q < phases; q++) solid_phase(st, q, true);
+  } else if (phases == 1) {  // one plain iteration: split, it may not write what it reads
+    PROF(s, K_SOLID_SOLVE, k_solid_solve<true, SOLVE_DELTA>
+         <<<blocks_for((long long)solid_pad + v.F), 256, 0, st>>>(v, P, solid_pad, 0));
+    PROF(s, K_APPLY_SOLID, k_apply_solid<<<blk_gl, 256, 0, st>>>(v, P));
     L += 2;
-    if (tets) {
-      PROF(s, K_SOLVE_TETS, k_solve_tets<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-      PROF(s, K_APPLY_SOLID_CONTACTS, k_apply_solid_contacts<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-      L += 2;
-    }
-    if (scc) {
-      PROF(s, K_SOLID_CONTACTS, k_solid_contacts<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-      PROF(s, K_APPLY_SOLID_CONTACTS, k_apply_solid_contacts<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-      L += 2;
-    }
   }
-  if (!mark_in_apply && v.S > 0) {
+  if (!mark_in_apply && !overlap && v.S > 0) {
     PROF(s, K_APPLY_SOLID, k_contact_mark<32><<<blocks_for((long long)v.S * 32), 256, 0, st>>>(v, P));
     L++;
   }

@@ -45,6 +45,8 @@ enum Domain {
   D_SOLVE0,   // solve lanes rounded to warps + fluid (first iteration)
   D_SOLVE,    // solve lanes rounded to warps
   D_SGL,      // GL lanes per solid (apply + contact marks)
+  D_STL,      // GT lanes per solid (tets)
+  D_SW,       // a warp per solid (contact cache)
   D_S,        // solids
   D_BC,       // bond/tet updates rounded to warps + GL lanes per particle
   NUM_DOMAINS
@@ -129,28 +131,26 @@ __global__ void __launch_bounds__(256) kb_apply_fluid(BatchArgs a) {
   batch_loop<D_F, false>(a, UPBD_BODY { b_apply_fluid(v, P, vb); });
 }
 template <bool APPLY_FLUID, int OUT>
-__global__ void __launch_bounds__(256, 6) kb_solid_solve(BatchArgs a, int it) {
+__global__ void __launch_bounds__(256, 6) kb_solid_solve(BatchArgs a, int q) {
   batch_loop<APPLY_FLUID ? D_SOLVE0 : D_SOLVE, false, true>(
-      a, UPBD_BODY { b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad_of(v.S), it, vb); });
+      a, UPBD_BODY { b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad_of(v.S), q, vb); });
 }
-template <bool MARK>
 __global__ void __launch_bounds__(256) kb_apply_solid(BatchArgs a) {
-  batch_loop<MARK ? D_SGL : D_S, false>(a, UPBD_BODY { b_apply_solid<MARK>(v, P, vb); });
+  batch_loop<D_SGL, false>(a, UPBD_BODY { b_apply_solid(v, P, vb); });
 }
 __global__ void __launch_bounds__(256) kb_contact_mark(BatchArgs a) {
   batch_loop<D_SGL, false>(a, UPBD_BODY { b_contact_mark(v, P, vb); });
 }
 __global__ void __launch_bounds__(256) kb_collect_contacts(BatchArgs a) {
-  batch_loop<D_S, false>(a, UPBD_BODY { b_collect_contacts(v, P, vb); });
+  batch_loop<D_SW, false>(a, UPBD_BODY { b_collect_contacts(v, P, vb); });
 }
-__global__ void __launch_bounds__(256) kb_solid_contacts(BatchArgs a) {
-  batch_loop<D_S, false>(a, UPBD_BODY { b_solid_contacts(v, P, vb); });
+template <bool LAST>
+__global__ void __launch_bounds__(256) kb_solid_contacts(BatchArgs a, int q) {
+  batch_loop<D_SGL, false>(a, UPBD_BODY { b_solid_contacts<LAST>(v, P, q, vb); });
 }
-__global__ void __launch_bounds__(256) kb_apply_solid_contacts(BatchArgs a) {
-  batch_loop<D_S, false>(a, UPBD_BODY { b_apply_solid_contacts(v, P, vb); });
-}
-__global__ void __launch_bounds__(256) kb_solve_tets(BatchArgs a) {
-  batch_loop<D_S, false>(a, UPBD_BODY { b_solve_tets(v, P, vb); });
+template <bool LAST>
+__global__ void __launch_bounds__(256) kb_solve_tets(BatchArgs a, int q) {
+  batch_loop<D_STL, false>(a, UPBD_BODY { b_solve_tets<LAST>(v, P, q, vb); });
 }
 __global__ void __launch_bounds__(256) kb_bond_contacts(BatchArgs a, int tets) {
   batch_loop<D_BC, false>(a, UPBD_BODY {
@@ -199,6 +199,8 @@ void scene_blocks(const SimView& v, bool tets, int bt, uint32_t out[NUM_DOMAINS]
   out[D_SOLVE0] = ceil_div((long long)sp + v.F, bt);
   out[D_SOLVE] = ceil_div(sp, bt);
   out[D_SGL] = ceil_div((long long)v.S * GL, bt);
+  out[D_STL] = ceil_div((long long)v.S * GT, bt);
+  out[D_SW] = ceil_div((long long)v.S * 32, bt);
   out[D_S] = ceil_div(v.S, bt);
   out[D_BC] = ceil_div((long long)bond_pad_of(v.C, nt) + (long long)v.N * GL, bt);
 }
@@ -429,8 +431,11 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
   const bool tets = (b->desc.features & UPBD_FEAT_TETS) != 0;
   const bool scc = (b->desc.features & UPBD_FEAT_SOLID_CONTACTS) != 0;
   const int iters = b->desc.solid_iters;
-  const bool mark_in_apply = iters > 0 && !tets && !scc;
-  const bool fold = iters >= 2 && !tets && !scc;  // solve + apply in one launch per iteration
+  // the solve's phases, each one launch that also applies where there are two
+  // or more (b_solid_solve's OUT; the single-scene launch_substep)
+  const int per = 1 + (tets ? 1 : 0) + (scc ? 1 : 0), phases = iters * per;
+  const bool mark_in_apply = iters > 0 && per == 1;
+  const bool fold = phases >= 2;
   for (int k = 0; k < nsub; k++) {
     BLAUNCH(b, K_INTEGRATE, kb_integrate_count<true, true><<<G, BT, 0, st>>>(a));
     BLAUNCH(b, K_SCAN, kb_scan<<<G, SCAN_THREADS, 0, st>>>(a));
@@ -442,24 +447,24 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
     else
       BLAUNCH(b, K_DISP, kb_disp<false><<<G, BT, 0, st>>>(a));
     if (iters == 0) BLAUNCH(b, K_APPLY_FLUID, kb_apply_fluid<<<G, BT, 0, st>>>(a));
-    if (scc) BLAUNCH(b, K_COLLECT, kb_collect_contacts<<<G, BT, 0, st>>>(a));
-    for (int it = 0; it < iters && fold; it++) {  // each iteration one launch (b_solid_solve's OUT)
-      if (it < iters - 1) BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_STEP><<<G, BT, 0, st>>>(a, it)));
-      else BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_LAST><<<G, BT, 0, st>>>(a, it)));
+    if (scc && fold) BLAUNCH(b, K_COLLECT, kb_collect_contacts<<<G, BT, 0, st>>>(a));
+    for (int q = 0; q < phases && fold; q++) {
+      const int kind = q % per;
+      const bool lastq = q == phases - 1;
+      if (kind == 0) {
+        if (!lastq) BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_STEP><<<G, BT, 0, st>>>(a, q)));
+        else BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_LAST><<<G, BT, 0, st>>>(a, q)));
+      } else if (tets && kind == 1) {
+        if (!lastq) BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<false><<<G, BT, 0, st>>>(a, q));
+        else BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<true><<<G, BT, 0, st>>>(a, q));
+      } else {
+        if (!lastq) BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<false><<<G, BT, 0, st>>>(a, q));
+        else BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<true><<<G, BT, 0, st>>>(a, q));
+      }
     }
-    for (int it = 0; it < iters && !fold; it++) {
-      if (it == 0) BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<true, SOLVE_DELTA><<<G, BT, 0, st>>>(a, it)));
-      else BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_DELTA><<<G, BT, 0, st>>>(a, it)));
-      if (mark_in_apply && it == iters - 1) BLAUNCH(b, K_APPLY_SOLID, kb_apply_solid<true><<<G, BT, 0, st>>>(a));
-      else BLAUNCH(b, K_APPLY_SOLID, kb_apply_solid<false><<<G, BT, 0, st>>>(a));
-      if (tets) {
-        BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<<<G, BT, 0, st>>>(a));
-        BLAUNCH(b, K_APPLY_SOLID_CONTACTS, kb_apply_solid_contacts<<<G, BT, 0, st>>>(a));
-      }
-      if (scc) {
-        BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<<<G, BT, 0, st>>>(a));
-        BLAUNCH(b, K_APPLY_SOLID_CONTACTS, kb_apply_solid_contacts<<<G, BT, 0, st>>>(a));
-      }
+    if (phases == 1) {  // one plain iteration: split
+      BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<true, SOLVE_DELTA><<<G, BT, 0, st>>>(a, 0)));
+      BLAUNCH(b, K_APPLY_SOLID, kb_apply_solid<<<G, BT, 0, st>>>(a));
     }
     if (!mark_in_apply) BLAUNCH(b, K_APPLY_SOLID, kb_contact_mark<<<G, BT, 0, st>>>(a));
     BLAUNCH(b, K_BOND_CONTACTS, kb_bond_contacts<<<G, BT, 0, st>>>(a, tets ? 1 : 0));

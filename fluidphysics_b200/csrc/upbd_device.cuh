@@ -121,6 +121,10 @@ struct SimView {
   uint32_t* tet_idx;   // 4 per tet
   float* tet_vol;      // rest volume, negative = dead
   const uint32_t* tet_adj;  // [S+1 offsets][4NT ids]
+  // CSR-parallel (scenes that solve tets): the corners of tet ids[k] and its
+  // pair scale 1 / max(tet degree of a corner) (both static)
+  const uint4* tet_rec;
+  const float* tet_scale;
   // Bucket-ordered copies, slot e matching entries[e]: neighbour gathers read
   // a candidate's data with one load at its slot instead of entries -> pos.
   // Every pass that moves a particle also writes its slot's copy.
@@ -236,6 +240,8 @@ constexpr int GL = 8;
 constexpr int GLF = 4;
 constexpr uint32_t NL = 32;  // density-pass neighbour-list entries kept per fluid lane (GLF * NL per particle)
 constexpr int DL = 2;        // threads per particle in the displacement pass
+constexpr int GT = 16;       // lanes per solid in the tet solve
+constexpr uint32_t CL_NEAR = 0x80000000u;  // contact cache entry flag: a lattice neighbour (solids stay below 2^31)
 
 // xsph sums over the fluid candidates within H at its own time, after the
 // displacement, contact and bounds passes moved the fluid. The density pass

@@ -72,12 +72,11 @@ __global__ void __launch_bounds__(256) k_apply_fluid(SimView v, const DevParams*
   b_apply_fluid(v, P, blockIdx.x);
 }
 template <bool APPLY_FLUID, int OUT>
-__global__ void __launch_bounds__(256) k_solid_solve(SimView v, const DevParams* __restrict__ P, int solid_pad, int it) {
-  b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad, it, blockIdx.x);
+__global__ void __launch_bounds__(256) k_solid_solve(SimView v, const DevParams* __restrict__ P, int solid_pad, int q) {
+  b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad, q, blockIdx.x);
 }
-template <bool MARK>
 __global__ void __launch_bounds__(256) k_apply_solid(SimView v, const DevParams* __restrict__ P) {
-  b_apply_solid<MARK>(v, P, blockIdx.x);
+  b_apply_solid(v, P, blockIdx.x);
 }
 template <int G, bool FROM_GRID = false>
 __global__ void __launch_bounds__(256) k_contact_mark(SimView v, const DevParams* __restrict__ P) {
@@ -86,14 +85,13 @@ __global__ void __launch_bounds__(256) k_contact_mark(SimView v, const DevParams
 __global__ void __launch_bounds__(256) k_collect_contacts(SimView v, const DevParams* __restrict__ P) {
   b_collect_contacts(v, P, blockIdx.x);
 }
-__global__ void __launch_bounds__(256) k_solid_contacts(SimView v, const DevParams* __restrict__ P) {
-  b_solid_contacts(v, P, blockIdx.x);
+template <bool LAST>
+__global__ void __launch_bounds__(256) k_solid_contacts(SimView v, const DevParams* __restrict__ P, int q) {
+  b_solid_contacts<LAST>(v, P, q, blockIdx.x);
 }
-__global__ void __launch_bounds__(256) k_apply_solid_contacts(SimView v, const DevParams* __restrict__ P) {
-  b_apply_solid_contacts(v, P, blockIdx.x);
-}
-__global__ void __launch_bounds__(256) k_solve_tets(SimView v, const DevParams* __restrict__ P) {
-  b_solve_tets(v, P, blockIdx.x);
+template <bool LAST>
+__global__ void __launch_bounds__(256) k_solve_tets(SimView v, const DevParams* __restrict__ P, int q) {
+  b_solve_tets<LAST>(v, P, q, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_bond_contacts(SimView v, const DevParams* __restrict__ P, int nb, int nt,
                                                        int nb_pad, int nc) {

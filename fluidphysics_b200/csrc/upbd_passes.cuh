@@ -496,20 +496,40 @@ __device__ __forceinline__ void mark_fluid_near(const SimView& v, const DevParam
 //
 // OUT selects what the solve does with solid i's correction:
 //   SOLVE_DELTA  writes delta[i] for b_apply_solid (the reference's split).
-//   SOLVE_STEP   applies it too (applyDeltaSolid, src/gpu/wgsl.js:361-366)
-//                into a ping-pong copy of the solid positions: iteration `it`
-//                reads pos (it 0) or sbuf[(it-1)&1] and writes sbuf[it&1],
-//                inactive solids carried over unchanged.
-//   SOLVE_LAST   applies it into pos and the slot copy, then marks the fluid
-//                near the final position (b_apply_solid<true>'s work).
+//   SOLVE_STEP   applies it too (applyDeltaSolid, src/gpu/wgsl.js:361-366) as
+//                one phase of the folded solve (below).
+//   SOLVE_LAST   the last phase: applies it into pos and the slot copy, then
+//                marks the fluid near the final position (b_apply_solid's
+//                work).
 //   SOLVE_FINAL  as SOLVE_LAST without the marks (b_contact_mark follows).
-// Every solve reads the previous iteration's positions only, as with the
-// split passes, and pos + omega * delta is the same expression, so the
-// folded iterations give the split ones' results bit for bit; they need at
-// least two iterations (the first may not write what it reads).
+//
+// The folded solve is a sequence of Q >= 2 phases: per iteration the distance
+// solve, then the tet solve and the solid contacts where the scene has them,
+// each with its apply. Phase q reads the positions phase q - 1 left and writes
+// the other of two copies (solid_src, solid_store): pos -> sbuf[0] -> sbuf[1]
+// -> sbuf[0] ... -> pos and the slot copy, inactive solids carried over. Every
+// phase reads its predecessor's positions only, as the split passes do, with
+// the same expressions, so the results are the split passes' bit for bit.
+// (One phase alone may not write what it reads: that case stays split.)
+// A phase is a launch of a few microseconds of dependent loads, so what
+// counts is their number: with tets and contacts 24 a substep of 8 iterations
+// instead of 48.
 constexpr int SOLVE_DELTA = 0, SOLVE_STEP = 1, SOLVE_LAST = 2, SOLVE_FINAL = 3;
+__device__ __forceinline__ const real4* solid_src(const SimView& v, int q) {
+  return q == 0 ? v.pos : v.sbuf + (size_t)((q - 1) & 1) * v.S;
+}
+template <bool LAST>
+__device__ __forceinline__ void solid_store(const SimView& v, int q, int i, bool act, const real4& p) {
+  if (!LAST) {
+    v.sbuf[(size_t)(q & 1) * v.S + i] = p;
+  } else if (act) {
+    v.pos[i] = p;
+    v.spos[v.slot[i]] = p;
+  }
+}
+
 template <bool APPLY_FLUID, int OUT = SOLVE_DELTA>
-__device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams* __restrict__ P, int solid_pad, int it,
+__device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams* __restrict__ P, int solid_pad, int q,
                                               uint32_t vb) {
   const int t = UPBD_VTID;
   if (t >= solid_pad) {
@@ -528,7 +548,7 @@ __device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams*
   const int i = t / GL;
   const int lane = threadIdx.x & (GL - 1);
   const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
-  const real4* __restrict__ pos = (OUT == SOLVE_DELTA || it == 0) ? v.pos : v.sbuf + (size_t)((it - 1) & 1) * v.S;
+  const real4* __restrict__ pos = (OUT == SOLVE_DELTA) ? v.pos : solid_src(v, q);
   const real4 pi = (i < v.S) ? pos[i] : make_real4(0.f, 0.f, 0.f, 0.f);
   real cx = 0.f, cy = 0.f, cz = 0.f;
   if (act) {
@@ -571,37 +591,23 @@ __device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams*
   if (act) {
     p.x = p.x + cx * w; p.y = p.y + cy * w; p.z = p.z + cz * w;
   }
-  if (OUT == SOLVE_STEP) {
-    if (i < v.S && lane == 0) v.sbuf[(size_t)(it & 1) * v.S + i] = p;
-    return;
-  }
-  if (act && lane == 0) {
-    v.pos[i] = p;
-    v.spos[v.slot[i]] = p;
-  }
+  if (i < v.S && lane == 0) solid_store<OUT != SOLVE_STEP>(v, q, i, act, p);
   if (OUT == SOLVE_LAST && P->use_mark) mark_fluid_near(v, P, act ? p : make_real4(0.f, 0.f, 0.f, 0.f), act, lane);
 }
 
-// applyDeltaSolid, src/gpu/wgsl.js:361-366. With MARK (last iteration of the
-// solve) GL lanes per solid also mark the fluid near its final position for
-// the contacts pass; the fluid positions are final by then.
-template <bool MARK>
+// applyDeltaSolid, src/gpu/wgsl.js:361-366, of a solve of one split
+// iteration: GL lanes per solid, which also mark the fluid near its final
+// position for the contacts pass; the fluid positions are final by then.
 __device__ __forceinline__ void b_apply_solid(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
   const int t = UPBD_VTID;
-  const int i = MARK ? t / GL : t;
+  const int i = t / GL;
   const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
-  if (!MARK && !act) return;
   const real w = P->omega;
   real4 p = make_real4(0.f, 0.f, 0.f, 0.f);
   if (act) {
     p = v.pos[i];
     const real4 d = v.delta[i];
     p.x = p.x + d.x * w; p.y = p.y + d.y * w; p.z = p.z + d.z * w;
-  }
-  if (!MARK) {
-    v.pos[i] = p;
-    v.spos[v.slot[i]] = p;
-    return;
   }
   const int lane = threadIdx.x & (GL - 1);
   if (act && lane == 0) {
@@ -643,99 +649,148 @@ __device__ __forceinline__ bool lattice_adjacent(const SimView& v, uint32_t i, u
   return abs(ax - bx) <= 1 && abs(ay - by) <= 1 && abs(az - bz) <= 1;
 }
 
-// isBonded, src/gpu/wgsl.js:599-607
-__device__ __forceinline__ bool is_bonded(const SimView& v, uint32_t i, uint32_t j) {
-  const uint32_t* ids = v.adj + v.S + 1;
-  for (uint32_t k = v.adj[i]; k < v.adj[i + 1]; k++) {
-    if (!UPBD_IDX_OK(v, ids[k], v.C)) continue;
-    const uint4 c = v.cons[ids[k]];
-    if (c.w != 0u && (c.x == j || c.y == j)) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ real solid_rsum(const SimView& v, const DevParams* __restrict__ P,
-                                            uint32_t i, uint32_t j) {
+// solidRsum: the contact distance of two solids, lattice neighbours or not
+__device__ __forceinline__ real solid_rsum(const DevParams* __restrict__ P, bool near) {
   const real rsum = 2.0f * P->solid_radius;
-  if (lattice_adjacent(v, i, j)) return mn(rsum, P->spacing * 0.97f);
+  if (near) return mn(rsum, P->spacing * 0.97f);
   return rsum;
 }
 
-// collectContacts, src/gpu/wgsl.js:532-560
+// collectContacts, src/gpu/wgsl.js:532-560, a warp per solid: the lanes take
+// 32 candidates of the solids' part of the 27 buckets at a time, in sequence
+// order, and a ballot gives each kept one its place, so the cache holds what
+// one invocation of the reference would list (the first C_K kept candidates).
+// A candidate's position is its slot copy (the solve writes the copies only at
+// its end). The solid's alive neighbours (at most 26, one per lane) are looked
+// up by shuffles. Entries carry CL_NEAR for lattice neighbours, whose contact
+// distance differs (solid_rsum), so the iterations need no index arithmetic.
+// Bound by the latency of its three or four dependent loads. One thread per
+// solid, as a chain of ~70 candidates with a constraint scan for each in
+// range, took 710 us a launch on 8,512 solids (B200, event-timed).
 __device__ __forceinline__ void b_collect_contacts(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const int i = UPBD_VTID;
-  if (i >= v.S) return;
-  uint32_t cnt = 0;
-  if (v.flags[i] & F_ACTIVE) {
-    const real4 pi = v.pos[i];
-    const real margin = 2.0f * P->solid_radius;
-    const uint32_t mask = (uint32_t)v.T - 1u;
-    CellHash ch;
-    ch.init(pi.x, pi.y, pi.z, P->inv_cell);
-    for (int a = 0; a < 3; a++)
-      for (int b = 0; b < 3; b++)
-        for (int c = 0; c < 3; c++) {
-          const uint32_t hb = ch.bucket(a, b, c, mask);
-          const uint32_t e1 = v.start[hb + 1];
-          for (uint32_t e = v.start[hb]; e < e1; e++) {
-            const uint32_t j = v.entries[e];
-            if (j == (uint32_t)i || j >= (uint32_t)v.S || cnt >= C_K) continue;
-            const real4 pj = v.pos[j];
-            const real ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
-            const real lim = solid_rsum(v, P, i, j) + margin;
-            if (dot3(ex, ey, ez, ex, ey, ez) >= lim * lim) continue;
-            if (is_bonded(v, i, j)) continue;
-            v.clist[(size_t)i * C_K + cnt] = j;
-            cnt++;
-          }
-        }
+  const unsigned FULL = 0xffffffffu;
+  const int i = (int)(UPBD_VTID >> 5), lane = (int)(threadIdx.x & 31);
+  if (i >= v.S) return;  // whole warps
+  if (!(v.flags[i] & F_ACTIVE)) {
+    if (lane == 0) v.ccount[i] = 0u;
+    return;
   }
-  v.ccount[i] = cnt;
-}
-
-// solidContacts, src/gpu/wgsl.js:562-585
-__device__ __forceinline__ void b_solid_contacts(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const int i = UPBD_VTID;
-  if (i >= v.S) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
   const real4 pi = v.pos[i];
-  const real wi = pi.w;
-  real cx = 0.f, cy = 0.f, cz = 0.f;
-  const uint32_t n = v.ccount[i];
-  for (uint32_t k = 0; k < n; k++) {
-    const uint32_t j = v.clist[(size_t)i * C_K + k];
-    if (!UPBD_IDX_OK(v, j, v.S)) continue;
-    const real4 pj = v.pos[j];
-    const real ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
-    const real rsum = solid_rsum(v, P, i, j);
-    const real d2 = dot3(ex, ey, ez, ex, ey, ez);
-    if (d2 >= rsum * rsum || d2 < 1e-12f) continue;
-    const real wsum = wi + pj.w;
-    if (wsum == 0.f) continue;
-    const real d = r_sqrt(d2);
-    const real f = (rsum - d) / d * wi / wsum * 0.5f;
-    cx = cx + ex * f; cy = cy + ey * f; cz = cz + ez * f;
+  CellHash ch;
+  group_cell_hash<32>(pi.x, pi.y, pi.z, P->inv_cell, ch);
+  const int row = (int)(threadIdx.x >> 5) * (32 / GLF);
+  const uint32_t run = walk_tables<1, 32>(v, ch, lane, true, row);
+  const uint32_t st = v.adj[i], en = v.adj[i + 1];
+  const real margin = 2.0f * P->solid_radius;
+  const real wide = 2.0f * P->solid_radius + margin, wide2 = wide * wide;  // no contact distance is larger
+  uint32_t cnt = 0, k = 0, next = s_walk_off[row][1], base = s_walk_base[row][0];
+  for (uint32_t c0 = 0; c0 < run && cnt < C_K; c0 += 32) {
+    const uint32_t c = c0 + (uint32_t)lane;
+    uint32_t j = (uint32_t)i;
+    bool keep = false, near = false;
+    if (c < run) {
+      while (c >= next) {
+        k++;
+        next = s_walk_off[row][k + 1];
+        base = s_walk_base[row][k];
+      }
+      const uint32_t e = base + c;
+      if (UPBD_IDX_OK(v, e, v.N)) {
+        const uint32_t jj = v.entries[e];
+        const real4 pj = v.spos[e];
+        const real ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
+        const real d2 = dot3(ex, ey, ez, ex, ey, ez);
+        if (jj != (uint32_t)i && jj < (uint32_t)v.S && !(d2 >= wide2)) {
+          near = lattice_adjacent(v, (uint32_t)i, jj);
+          const real lim = solid_rsum(P, near) + margin;
+          j = jj;
+          keep = !(d2 >= lim * lim);
+        }
+      }
+    }
+    // isBonded, src/gpu/wgsl.js:599-607: only lattice neighbours are
+    if (__any_sync(FULL, keep && near)) {
+      bool bonded = false;
+      for (uint32_t q0 = st; q0 < en; q0 += 32) {
+        uint32_t other = 0xffffffffu;
+        if (q0 + (uint32_t)lane < en) {
+          const uint32_t ci = v.adj[v.S + 1 + q0 + lane];
+          if (UPBD_IDX_OK(v, ci, v.C) && v.cons[ci].w != 0u) other = v.adj_other[q0 + lane];
+        }
+        const int m = (int)min(32u, en - q0);
+        for (int l = 0; l < m; l++) {  // every lane takes part in every shuffle
+          const uint32_t o = __shfl_sync(FULL, other, l);
+          bonded = bonded | (o == j);
+        }
+      }
+      keep = keep && !bonded;
+    }
+    const unsigned kept = __ballot_sync(FULL, keep);
+    const uint32_t at = cnt + (uint32_t)__popc(kept & ((1u << lane) - 1u));
+    if (keep && at < C_K) v.clist[(size_t)i * C_K + at] = j | (near ? CL_NEAR : 0u);
+    cnt = min(cnt + (uint32_t)__popc(kept), C_K);
   }
-  v.delta[i] = make_real4(cx, cy, cz, 1.0f);
+  if (lane == 0) v.ccount[i] = cnt;
+  __syncwarp();  // the next call may rewrite this warp's tables
 }
 
-// applySolidContacts, src/gpu/wgsl.js:587-596
-__device__ __forceinline__ void b_apply_solid_contacts(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const int i = UPBD_VTID;
-  if (i >= v.S) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
+// Clamp of applySolidContacts (src/gpu/wgsl.js:587-596) on a correction of
+// solid position p: the apply of the tet and contact phases.
+__device__ __forceinline__ real4 apply_clamped(const DevParams* __restrict__ P, real4 p, real dx, real dy, real dz) {
   const real maxC = 0.5f * P->solid_radius;
-  const real4 dd = v.delta[i];
-  real dx = dd.x, dy = dd.y, dz = dd.z;
   const real m2 = dot3(dx, dy, dz, dx, dy, dz);
   if (m2 > maxC * maxC) {
     const real f = maxC / r_sqrt(m2);
     dx = dx * f; dy = dy * f; dz = dz * f;
   }
-  real4 p = v.pos[i];
   p.x = p.x + dx; p.y = p.y + dy; p.z = p.z + dz;
-  v.pos[i] = p;
-  v.spos[v.slot[i]] = p;
+  return p;
+}
+
+// solidContacts + applySolidContacts, src/gpu/wgsl.js:562-596, as a phase of
+// the folded solve: GL lanes per solid take the cache's entries side by side,
+// then every lane adds the terms up in the cache's order (one fused or one
+// rounded multiply-add per term, as the one-thread loop). An uncut lattice
+// lists about six entries a solid, so one round.
+template <bool LAST>
+__device__ __forceinline__ void b_solid_contacts(const SimView& v, const DevParams* __restrict__ P, int q, uint32_t vb) {
+  const unsigned FULL = 0xffffffffu;
+  const int i = (int)(UPBD_VTID / GL), lane = (int)(threadIdx.x & (GL - 1));
+  const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
+  const real4* __restrict__ pos = solid_src(v, q);
+  const real4 pi = (i < v.S) ? pos[i] : make_real4(0.f, 0.f, 0.f, 0.f);
+  const real wi = pi.w;
+  real cx = 0.f, cy = 0.f, cz = 0.f;
+  const uint32_t n = act ? v.ccount[i] : 0u;
+  for (uint32_t k0 = 0; __any_sync(FULL, k0 < n); k0 += GL) {
+    real ex = 0.f, ey = 0.f, ez = 0.f, f = 0.f;
+    bool hit = false;
+    if (k0 + (uint32_t)lane < n) {
+      const uint32_t e = v.clist[(size_t)i * C_K + k0 + lane], j = e & ~CL_NEAR;
+      if (UPBD_IDX_OK(v, j, v.S)) {
+        const real4 pj = pos[j];
+        const real dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const real rsum = solid_rsum(P, (e & CL_NEAR) != 0u);
+        const real d2 = dot3(dx, dy, dz, dx, dy, dz);
+        const real wsum = wi + pj.w;
+        hit = !(d2 >= rsum * rsum || d2 < 1e-12f) && wsum != 0.f;
+        if (hit) {
+          const real d = r_sqrt(d2);
+          ex = dx; ey = dy; ez = dz;
+          f = (rsum - d) / d * wi / wsum * 0.5f;
+        }
+      }
+    }
+    if (!__any_sync(FULL, hit)) continue;
+#pragma unroll
+    for (int l = 0; l < GL; l++) {
+      const real fl = __shfl_sync(FULL, f, l, GL);
+      cx = cx + __shfl_sync(FULL, ex, l, GL) * fl;
+      cy = cy + __shfl_sync(FULL, ey, l, GL) * fl;
+      cz = cz + __shfl_sync(FULL, ez, l, GL) * fl;
+    }
+  }
+  if (i < v.S && lane == 0) solid_store<LAST>(v, q, i, act, act ? apply_clamped(P, pi, cx, cy, cz) : pi);
 }
 
 __device__ __forceinline__ void cross3(real ax, real ay, real az, real bx, real by, real bz,
@@ -745,65 +800,87 @@ __device__ __forceinline__ void cross3(real ax, real ay, real az, real bx, real 
   z = ax * by - ay * bx;
 }
 
-// solveTets, src/gpu/wgsl.js:423-468
-__device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const int i = UPBD_VTID;
-  if (i >= v.S) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
-  const uint32_t* ids = v.tet_adj + v.S + 1;
-  real cx = 0.f, cy = 0.f, cz = 0.f;
-  for (uint32_t k = v.tet_adj[i]; k < v.tet_adj[i + 1]; k++) {
-    const uint32_t t = ids[k];
-    if (!UPBD_IDX_OK(v, t, v.NT)) continue;
-    const uint32_t ia = v.tet_idx[4 * t], ib = v.tet_idx[4 * t + 1], ic = v.tet_idx[4 * t + 2],
-                   id = v.tet_idx[4 * t + 3];
-    if (!UPBD_IDX_OK(v, ia, v.S) || !UPBD_IDX_OK(v, ib, v.S) || !UPBD_IDX_OK(v, ic, v.S) ||
-        !UPBD_IDX_OK(v, id, v.S))
-      continue;
-    const real V0 = v.tet_vol[t];
-    if (V0 <= 0.f) continue;
-    const real4 pa = v.pos[ia], pb = v.pos[ib], pc = v.pos[ic], pd = v.pos[id];
-    const real bax = pb.x - pa.x, bay = pb.y - pa.y, baz = pb.z - pa.z;
-    const real cax = pc.x - pa.x, cay = pc.y - pa.y, caz = pc.z - pa.z;
-    const real dax = pd.x - pa.x, day = pd.y - pa.y, daz = pd.z - pa.z;
-    real xx, xy, xz;
-    cross3(bax, bay, baz, cax, cay, caz, xx, xy, xz);
-    const real V = dot3(xx, xy, xz, dax, day, daz) / 6.0f;
-    const real Cv = V - V0;
-    real gbx, gby, gbz, gcx, gcy, gcz, gdx, gdy, gdz;
-    cross3(cax, cay, caz, dax, day, daz, gbx, gby, gbz);
-    gbx = gbx / 6.0f; gby = gby / 6.0f; gbz = gbz / 6.0f;
-    cross3(dax, day, daz, bax, bay, baz, gcx, gcy, gcz);
-    gcx = gcx / 6.0f; gcy = gcy / 6.0f; gcz = gcz / 6.0f;
-    cross3(bax, bay, baz, cax, cay, caz, gdx, gdy, gdz);
-    gdx = gdx / 6.0f; gdy = gdy / 6.0f; gdz = gdz / 6.0f;
-    const real gax = -((gbx + gcx) + gdx), gay = -((gby + gcy) + gdy), gaz = -((gbz + gcz) + gdz);
-    const real w = pa.w;
-    const real denom = w * (dot3(gax, gay, gaz, gax, gay, gaz) + dot3(gbx, gby, gbz, gbx, gby, gbz) +
-                             dot3(gcx, gcy, gcz, gcx, gcy, gcz) + dot3(gdx, gdy, gdz, gdx, gdy, gdz));
-    if (denom < 1e-12f) continue;
-    const real dl = -Cv / denom;
-    const uint32_t da = v.tet_adj[ia + 1] - v.tet_adj[ia], db = v.tet_adj[ib + 1] - v.tet_adj[ib];
-    const uint32_t dc = v.tet_adj[ic + 1] - v.tet_adj[ic], dd = v.tet_adj[id + 1] - v.tet_adj[id];
-    const uint32_t m1 = (da < db) ? db : da, m2 = (dc < dd) ? dd : dc;
-    uint32_t dm = (m1 < m2) ? m2 : m1;
-    if (dm < 1u) dm = 1u;
-    const real s = 1.0f / (real)dm;
-    real gx = gax, gy = gay, gz = gaz;
-    if ((uint32_t)i == ib) { gx = gbx; gy = gby; gz = gbz; }
-    else if ((uint32_t)i == ic) { gx = gcx; gy = gcy; gz = gcz; }
-    else if ((uint32_t)i == id) { gx = gdx; gy = gdy; gz = gdz; }
-    const real f = w * dl * s;
-    real c1x = gx * f, c1y = gy * f, c1z = gz * f;
-    const real cl2 = dot3(c1x, c1y, c1z, c1x, c1y, c1z);
-    const real lim = 0.5f * P->solid_radius;
-    if (cl2 > lim * lim) {
-      const real g = lim / r_sqrt(cl2);
-      c1x = c1x * g; c1y = c1y * g; c1z = c1z * g;
-    }
-    cx = cx + c1x; cy = cy + c1y; cz = cz + c1z;
+// solveTets, src/gpu/wgsl.js:423-468: corner i's correction from one tet with
+// corners q, rest volume V0 and pair scale s
+__device__ __forceinline__ void tet_corner(const DevParams* __restrict__ P, const real4* __restrict__ pos, uint32_t i,
+                                           const uint4& q, real V0, real s, real& ox, real& oy, real& oz) {
+  ox = 0.f; oy = 0.f; oz = 0.f;
+  const real4 pa = pos[q.x], pb = pos[q.y], pc = pos[q.z], pd = pos[q.w];
+  const real bax = pb.x - pa.x, bay = pb.y - pa.y, baz = pb.z - pa.z;
+  const real cax = pc.x - pa.x, cay = pc.y - pa.y, caz = pc.z - pa.z;
+  const real dax = pd.x - pa.x, day = pd.y - pa.y, daz = pd.z - pa.z;
+  real xx, xy, xz;
+  cross3(bax, bay, baz, cax, cay, caz, xx, xy, xz);
+  const real V = dot3(xx, xy, xz, dax, day, daz) / 6.0f;
+  const real Cv = V - V0;
+  real gbx, gby, gbz, gcx, gcy, gcz, gdx, gdy, gdz;
+  cross3(cax, cay, caz, dax, day, daz, gbx, gby, gbz);
+  gbx = gbx / 6.0f; gby = gby / 6.0f; gbz = gbz / 6.0f;
+  cross3(dax, day, daz, bax, bay, baz, gcx, gcy, gcz);
+  gcx = gcx / 6.0f; gcy = gcy / 6.0f; gcz = gcz / 6.0f;
+  cross3(bax, bay, baz, cax, cay, caz, gdx, gdy, gdz);
+  gdx = gdx / 6.0f; gdy = gdy / 6.0f; gdz = gdz / 6.0f;
+  const real gax = -((gbx + gcx) + gdx), gay = -((gby + gcy) + gdy), gaz = -((gbz + gcz) + gdz);
+  const real w = pa.w;
+  const real denom = w * (dot3(gax, gay, gaz, gax, gay, gaz) + dot3(gbx, gby, gbz, gbx, gby, gbz) +
+                           dot3(gcx, gcy, gcz, gcx, gcy, gcz) + dot3(gdx, gdy, gdz, gdx, gdy, gdz));
+  if (denom < 1e-12f) return;
+  const real dl = -Cv / denom;
+  real gx = gax, gy = gay, gz = gaz;
+  if (i == q.y) { gx = gbx; gy = gby; gz = gbz; }
+  else if (i == q.z) { gx = gcx; gy = gcy; gz = gcz; }
+  else if (i == q.w) { gx = gdx; gy = gdy; gz = gdz; }
+  const real f = w * dl * s;
+  real c1x = gx * f, c1y = gy * f, c1z = gz * f;
+  const real cl2 = dot3(c1x, c1y, c1z, c1x, c1y, c1z);
+  const real lim = 0.5f * P->solid_radius;
+  if (cl2 > lim * lim) {
+    const real g = lim / r_sqrt(cl2);
+    c1x = c1x * g; c1y = c1y * g; c1z = c1z * g;
   }
-  v.delta[i] = make_real4(cx, cy, cz, 1.0f);
+  ox = c1x; oy = c1y; oz = c1z;
+}
+
+// solveTets + its apply, a phase of the folded solve: GT lanes per solid
+// compute the corrections of its next GT tets side by side (corners and pair
+// scale in one row per incidence), then every lane adds them up in the CSR's
+// order, so the sum is the one-thread loop's. Bound by latency (record ->
+// corners -> arithmetic): inner solids have 8 or 32 tets, so one or two rounds
+// of 16 lanes; one thread per solid, 32 tets in a chain, took 34 us a launch
+// on 8,512 solids (B200, event-timed).
+template <bool LAST>
+__device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* __restrict__ P, int q, uint32_t vb) {
+  const unsigned FULL = 0xffffffffu;
+  const int i = (int)(UPBD_VTID / GT), lane = (int)(threadIdx.x & (GT - 1));
+  const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
+  const real4* __restrict__ pos = solid_src(v, q);
+  const uint32_t* __restrict__ ids = v.tet_adj + v.S + 1;
+  real cx = 0.f, cy = 0.f, cz = 0.f;
+  const uint32_t st = act ? v.tet_adj[i] : 0u, en = act ? v.tet_adj[i + 1] : 0u;
+  for (uint32_t k0 = st; __any_sync(FULL, k0 < en); k0 += GT) {
+    const uint32_t k = k0 + (uint32_t)lane;
+    real ox = 0.f, oy = 0.f, oz = 0.f;
+    if (k < en) {
+      const uint4 c = __ldg(&v.tet_rec[k]);
+      const uint32_t t = __ldg(&ids[k]);
+      const real s = __ldg(&v.tet_scale[k]);
+      if (UPBD_IDX_OK(v, t, v.NT) && UPBD_IDX_OK(v, c.x, v.S) && UPBD_IDX_OK(v, c.y, v.S) && UPBD_IDX_OK(v, c.z, v.S) &&
+          UPBD_IDX_OK(v, c.w, v.S)) {
+        const real V0 = v.tet_vol[t];
+        if (!(V0 <= 0.f)) tet_corner(P, pos, (uint32_t)i, c, V0, s, ox, oy, oz);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < GT; l++) {
+      cx = cx + __shfl_sync(FULL, ox, l, GT);
+      cy = cy + __shfl_sync(FULL, oy, l, GT);
+      cz = cz + __shfl_sync(FULL, oz, l, GT);
+    }
+  }
+  if (i < v.S && lane == 0) {
+    const real4 pi = pos[i];
+    solid_store<LAST>(v, q, i, act, act ? apply_clamped(P, pi, cx, cy, cz) : pi);
+  }
 }
 
 // -------------------------------------------- bond update + contacts

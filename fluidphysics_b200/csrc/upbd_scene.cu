@@ -20,7 +20,6 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
   const double maxD2 = 3 * sp * sp + 1e-9;
   std::vector<uint32_t> ca, cb;
   std::vector<double> crest;
-  std::vector<std::vector<uint32_t>> inc(out.S);
   int id = 0;
   auto add_lattice = [&](int dim, const double* c) {
     const int base = id;
@@ -45,12 +44,9 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
                 if (b <= a) continue;
                 const double d2 = (double)(dx * dx + dy * dy + dz * dz) * sp * sp;
                 if (d2 > maxD2) continue;
-                const uint32_t cidx = (uint32_t)ca.size();
                 ca.push_back(a);
                 cb.push_back(b);
                 crest.push_back(std::sqrt(d2));
-                inc[a].push_back(cidx);
-                inc[b].push_back(cidx);
               }
   };
   auto signed_vol = [&](int a, int b, int c, int e) {
@@ -99,13 +95,20 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
     std::memcpy(&bits, &r, 4);
     out.cons[c] = make_uint4(ca[c], cb[c], bits, 1u);
   }
-  out.adj.assign(out.S + 1 + 2 * (size_t)C, 0);
-  uint32_t off = 0;
-  for (int i = 0; i < out.S; i++) {
-    out.adj[i] = off;
-    for (uint32_t c : inc[i]) out.adj[out.S + 1 + off++] = c;
-  }
-  out.adj[out.S] = off;
+  // CSR of the ids incident to each solid, ascending: count, prefix, fill
+  auto csr = [&](std::vector<uint32_t>& adj, size_t n, auto&& each) {
+    adj.assign(out.S + 1 + n, 0);
+    each([&](uint32_t i, uint32_t) { adj[i + 1]++; });
+    for (int i = 0; i < out.S; i++) adj[i + 1] += adj[i];
+    std::vector<uint32_t> at(adj.begin(), adj.begin() + out.S);
+    each([&](uint32_t i, uint32_t id) { adj[out.S + 1 + at[i]++] = id; });
+  };
+  csr(out.adj, 2 * (size_t)C, [&](auto&& put) {
+    for (int c = 0; c < C; c++) {
+      put(ca[c], (uint32_t)c);
+      put(cb[c], (uint32_t)c);
+    }
+  });
   // CSR-parallel static data of the Jacobi gather: the other endpoint of each
   // incident constraint and the pair scale 1/max(deg_i, deg_j) of
   // src/gpu/wgsl.js:340-354 (endpoints and degrees never change)
@@ -122,16 +125,21 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
     }
   }
   const int NT = (int)out.tet_vol.size();
-  std::vector<std::vector<uint32_t>> tinc(out.S);
-  for (int t = 0; t < NT; t++)
-    for (int q = 0; q < 4; q++) tinc[out.tet_idx[4 * t + q]].push_back(t);
-  out.tet_adj.assign(out.S + 1 + 4 * (size_t)NT, 0);
-  off = 0;
-  for (int i = 0; i < out.S; i++) {
-    out.tet_adj[i] = off;
-    for (uint32_t t : tinc[i]) out.tet_adj[out.S + 1 + off++] = t;
+  csr(out.tet_adj, 4 * (size_t)NT, [&](auto&& put) {
+    for (int t = 0; t < NT; t++)
+      for (int q = 0; q < 4; q++) put(out.tet_idx[4 * t + q], (uint32_t)t);
+  });
+  // CSR-parallel static data of the tet gather: the corners and the pair
+  // scale 1/max(tet degree) of src/gpu/wgsl.js:444-452
+  out.tet_rec.resize(4 * (size_t)NT);
+  out.tet_scale.resize(4 * (size_t)NT);
+  for (size_t k = 0; k < 4 * (size_t)NT; k++) {
+    const uint32_t* q = &out.tet_idx[4 * (size_t)out.tet_adj[out.S + 1 + k]];
+    uint32_t dm = 1;
+    for (int c = 0; c < 4; c++) dm = std::max(dm, out.tet_adj[q[c] + 1] - out.tet_adj[q[c]]);
+    out.tet_rec[k] = make_uint4(q[0], q[1], q[2], q[3]);
+    out.tet_scale[k] = 1.0f / (float)dm;
   }
-  out.tet_adj[out.S] = off;
 }
 
 namespace {
@@ -158,6 +166,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   v.T = d.table_size;
   v.num_tiles = (v.T + SCAN_TILE - 1) / SCAN_TILE;
   const bool scc = (d.features & UPBD_FEAT_SOLID_CONTACTS) != 0;
+  const bool tets = (d.features & UPBD_FEAT_TETS) != 0;
   Carver cv;
   SceneLayout L{};
   L.pos = cv.take<real4>(v.N);
@@ -190,6 +199,8 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.ascl = cv.take<float>(std::max<size_t>(hs.adj_scale.size(), 1));
   L.ccount = cv.take<uint32_t>(scc ? std::max(v.S, 1) : 1);
   L.clist = cv.take<uint32_t>(scc ? (size_t)std::max(v.S, 1) * C_K : 1);
+  L.trec = cv.take<uint4>(tets ? std::max<size_t>(hs.tet_rec.size(), 1) : 1);
+  L.tscl = cv.take<float>(tets ? std::max<size_t>(hs.tet_scale.size(), 1) : 1);
   L.sbuf = cv.take<real4>(2 * (size_t)std::max(v.S, 1));
   L.sfp = cv.take<real4>(v.N);
   L.smove = cv.take<float>(v.N);
@@ -201,6 +212,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
 #else
   L.conv = 0;
 #endif
+  L.tets = tets;
   L.bytes = cv.off;
   return L;
 }
@@ -234,6 +246,8 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.ncount = (uint32_t*)(base + L.ncount);
   v.adj_other = (const uint32_t*)(base + L.aoth);
   v.adj_scale = (const float*)(base + L.ascl);
+  v.tet_rec = L.tets ? (const uint4*)(base + L.trec) : nullptr;
+  v.tet_scale = L.tets ? (const float*)(base + L.tscl) : nullptr;
   v.ccount = (uint32_t*)(base + L.ccount);
   v.clist = (uint32_t*)(base + L.clist);
   v.sbuf = (real4*)(base + L.sbuf);
@@ -317,6 +331,10 @@ cudaError_t upload_scene(const HostScene& hs, const SimView& v, cudaStream_t st)
     e = cudaMemcpyAsync((void*)v.tet_adj, hs.tet_adj.data(), hs.tet_adj.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && !hs.tet_idx.empty())
     e = cudaMemcpyAsync(v.tet_idx, hs.tet_idx.data(), hs.tet_idx.size() * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && v.tet_rec && !hs.tet_rec.empty())
+    e = cudaMemcpyAsync((void*)v.tet_rec, hs.tet_rec.data(), hs.tet_rec.size() * sizeof(uint4), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && v.tet_rec && !hs.tet_scale.empty())
+    e = cudaMemcpyAsync((void*)v.tet_scale, hs.tet_scale.data(), hs.tet_scale.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = state_to_device((real*)v.pos, (const float*)hs.pos.data(), hs.pos.size(), 4, v, st);
   if (e == cudaSuccess) e = state_to_device((real*)v.prev, (const float*)hs.pos.data(), hs.pos.size(), 4, v, st);
   if (e == cudaSuccess && v.C > 0)
@@ -406,6 +424,8 @@ cudaError_t upload_prepared(const PreparedScene& ps, const SimView& v, cudaStrea
   if (e == cudaSuccess) e = up((void*)v.adj_scale, L.adj_scale.data(), L.adj_scale.size() * 4);
   if (e == cudaSuccess) e = up((void*)v.tet_adj, L.tet_adj.data(), L.tet_adj.size() * 4);
   if (e == cudaSuccess) e = up(v.tet_idx, L.tet_idx.data(), L.tet_idx.size() * 4);
+  if (e == cudaSuccess && v.tet_rec) e = up((void*)v.tet_rec, L.tet_rec.data(), L.tet_rec.size() * sizeof(uint4));
+  if (e == cudaSuccess && v.tet_rec) e = up((void*)v.tet_scale, L.tet_scale.data(), L.tet_scale.size() * 4);
   if (e == cudaSuccess) e = up(v.cons, L.cons.data(), L.cons.size() * 16);
   if (e == cudaSuccess) e = up(v.tet_vol, L.tet_vol.data(), L.tet_vol.size() * 4);
   auto rows = [&](real4* dst, const std::vector<float4>& src, size_t n) {

@@ -23,6 +23,8 @@ struct HostScene {
   std::vector<uint32_t> tet_idx;
   std::vector<float> tet_vol;
   std::vector<uint32_t> tet_adj;
+  std::vector<uint4> tet_rec;     // per tet_adj id: the tet's corners
+  std::vector<float> tet_scale;   // per tet_adj id: 1 / max(tet degree of a corner)
   int S = 0, N1 = 0, N = 0;
 };
 
@@ -34,8 +36,9 @@ void build_scene(const upbd_scene_desc& d, HostScene& out);
 struct SceneLayout {
   size_t pos, prev, vel, delta, dens, flags, cons, adj, counts, start, entries, tmp, ticket, cell, tiles;
   size_t tidx, tvol, tadj, mark, spos, sdens, svel, slot, fend, nbr, ncount, aoth, ascl, ccount, clist;
-  size_t sbuf, sfp, smove, bmove, scr, par, conv;
+  size_t trec, tscl, sbuf, sfp, smove, bmove, scr, par, conv;
   size_t bytes;
+  bool tets;  // the scene solves tets: trec and tscl hold their data
 };
 
 // Fills the sizes of v from the descriptor and host scene (full or
