@@ -60,7 +60,7 @@ struct ProfRec {
 struct upbd_sim {
   upbd_scene_desc desc{};
   upbd_params prm{};
-  int device = 0;
+  int device = 0, num_sms = 0;
   SimView v{};
   DevParams hp{};              // host mirror of the device uniforms
   DevParams* dparams = nullptr;
@@ -248,8 +248,11 @@ int launch_substep(upbd_sim* s, int last) {
     UPBD_CK(s, cudaEventRecord(s->join_ev, s->side));
   }
   if (last < UPBD_PASS_DENSITY) return UPBD_OK;
-  const long long fl = (long long)v.N * GLF;  // lane-parallel fluid gathers over the slots
-  PROF(s, K_DENSITY, k_density<<<blocks_for(fl), 256, 0, st>>>(v, P));
+  // places of a density block's window: at least two blocks an SM where the
+  // scene has them
+  uint32_t window = WINDOW_MAX;
+  while (window > 16 && (long long)v.N < 2ll * s->num_sms * window) window /= 2;
+  PROF(s, K_DENSITY, k_density<<<blocks_for(v.N, (int)window), 256, 8 * STAGE_WARP, st>>>(v, P, window));
   L++;
   if (last < UPBD_PASS_DISP) return UPBD_OK;
   if (fold)  // DL threads per slot
@@ -509,6 +512,7 @@ int upbd_create(const upbd_scene_desc* desc, const upbd_params* params, upbd_sim
   s->desc = *desc;
   s->prm = *params;
   s->device = desc->device;
+  s->num_sms = prop.multiProcessorCount;
   HostScene hs;
   build_scene(*desc, hs);
   SimView& v = s->v;

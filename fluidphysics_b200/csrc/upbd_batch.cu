@@ -39,7 +39,8 @@ enum Domain {
   D_N,        // particles (integrate/count, rankfix, apply+bounds+velocity)
   D_TILES,    // scan tiles of the bucket table (SCAN_THREADS per block)
   D_SCATTER,  // max(particles, scan tiles)
-  D_FGL,      // GLF lanes per grid slot (density, xsph)
+  D_CHUNK,    // windows of half a block's threads in grid slots (density)
+  D_FGL,      // GLF lanes per grid slot (xsph)
   D_DISP,     // DL threads per grid slot (displacement)
   D_F,        // fluid particles (apply, xsph apply, active count)
   D_SOLVE0,   // solve lanes rounded to warps + fluid (first iteration)
@@ -118,10 +119,8 @@ __global__ void __launch_bounds__(256) kb_scatter(BatchArgs a) {
 __global__ void __launch_bounds__(256) kb_rankfix(BatchArgs a) {
   batch_loop<D_N, false, true>(a, UPBD_BODY { b_rankfix(v, vb); });
 }
-// density and the solve are latency-bound: at most 40 registers (6 CTAs of
-// 256 per SM) hides more of it than the few spilled values cost
-__global__ void __launch_bounds__(256, 6) kb_density(BatchArgs a) {
-  batch_loop<D_FGL, false, true>(a, UPBD_BODY { b_density(v, P, vb); });
+__global__ void __launch_bounds__(256, 5) kb_density(BatchArgs a) {
+  batch_loop<D_CHUNK, true, true>(a, UPBD_BODY { b_density(v, P, blockDim.x / 2, vb); });
 }
 template <bool APPLY>
 __global__ void __launch_bounds__(256) kb_disp(BatchArgs a) {
@@ -130,6 +129,8 @@ __global__ void __launch_bounds__(256) kb_disp(BatchArgs a) {
 __global__ void __launch_bounds__(256) kb_apply_fluid(BatchArgs a) {
   batch_loop<D_F, false>(a, UPBD_BODY { b_apply_fluid(v, P, vb); });
 }
+// the solve is latency-bound: at most 40 registers (6 CTAs of 256 per SM)
+// hides more of it than the few spilled values cost
 template <bool APPLY_FLUID, int OUT>
 __global__ void __launch_bounds__(256, 6) kb_solid_solve(BatchArgs a, int q) {
   batch_loop<APPLY_FLUID ? D_SOLVE0 : D_SOLVE, false, true>(
@@ -193,6 +194,7 @@ void scene_blocks(const SimView& v, bool tets, int bt, uint32_t out[NUM_DOMAINS]
   out[D_N] = ceil_div(v.N, bt);
   out[D_TILES] = (uint32_t)std::max(v.num_tiles, 1);
   out[D_SCATTER] = ceil_div(std::max(v.N, tile_words(v.num_tiles)), bt);
+  out[D_CHUNK] = ceil_div(v.N, bt / 2);
   out[D_FGL] = ceil_div((long long)v.N * GLF, bt);
   out[D_DISP] = ceil_div((long long)v.N * DL, bt);
   out[D_F] = ceil_div(v.F, bt);
@@ -441,7 +443,7 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
     BLAUNCH(b, K_SCAN, kb_scan<<<G, SCAN_THREADS, 0, st>>>(a));
     BLAUNCH(b, K_SCATTER, kb_scatter<<<G, BT, 0, st>>>(a));
     BLAUNCH(b, K_RANKFIX, kb_rankfix<<<G, BT, 0, st>>>(a));
-    BLAUNCH(b, K_DENSITY, kb_density<<<G, BT, 0, st>>>(a));
+    BLAUNCH(b, K_DENSITY, kb_density<<<G, BT, (BT / 32) * STAGE_WARP, st>>>(a));
     if (fold)  // the displacement pass applies the fluid's move (b_disp<true>)
       BLAUNCH(b, K_DISP, kb_disp<true><<<G, BT, 0, st>>>(a));
     else

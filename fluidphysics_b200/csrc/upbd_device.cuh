@@ -70,6 +70,10 @@ __device__ __forceinline__ float r_fabs(float x) { return fabsf(x); }
 __device__ __forceinline__ double r_fabs(double x) { return fabs(x); }
 __device__ __forceinline__ float r_fmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double r_fmax(double a, double b) { return fmax(a, b); }
+__device__ __forceinline__ float r_mul(float a, float b) { return __fmul_rn(a, b); }  // never fused with an add
+__device__ __forceinline__ double r_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float r_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double r_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float r_fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double r_fdiv(double a, double b) { return a / b; }
 // a float no smaller than x (movement bounds kept as float bits); x >= 0
@@ -128,7 +132,7 @@ struct SimView {
   // Bucket-ordered copies, slot e matching entries[e]: neighbour gathers read
   // a candidate's data with one load at its slot instead of entries -> pos.
   // Every pass that moves a particle also writes its slot's copy.
-  real4* spos;         // position + inverse mass
+  real4* spos;         // position + inverse mass (fluid, until the bounds pass: + slot)
   real2* sdens;        // (rho, rho_near) of the density pass
   real4* svel;         // velocity after velocityUpdate
   uint32_t* slot;      // slot of particle i in this substep's grid
@@ -240,6 +244,9 @@ constexpr int GL = 8;
 constexpr int GLF = 4;
 constexpr uint32_t NL = 32;  // density-pass neighbour-list entries kept per fluid lane (GLF * NL per particle)
 constexpr int DL = 2;        // threads per particle in the displacement pass
+constexpr uint32_t CHUNK = 32 / GLF;  // fluid particles of one cell that a warp takes in the density pass
+constexpr int CHUNK_SHIFT = 28;       // chunk place: slot, above it the size of the chunk that starts there
+constexpr uint32_t CHUNK_SLOT = (1u << CHUNK_SHIFT) - 1u;  // a scene of 2^28 slots would need 240 GB
 constexpr int GT = 16;       // lanes per solid in the tet solve
 constexpr uint32_t CL_NEAR = 0x80000000u;  // contact cache entry flag: a lattice neighbour (solids stay below 2^31)
 
@@ -470,14 +477,37 @@ __device__ __forceinline__ float approx_sqrt(float x) {
 }
 __device__ __forceinline__ double approx_sqrt(double x) { return sqrt(x); }
 
-__device__ __forceinline__ uint32_t cell_of(real px, real py, real pz, double inv, uint32_t mask) {
+// Bucket of the cell at p; key: a second hash of the cell that tells most
+// cells of one bucket apart.
+__device__ __forceinline__ uint32_t cell_of(real px, real py, real pz, double inv, uint32_t mask, uint32_t& key) {
   const double cx = floor(__dmul_rn((double)px, inv));
   const double cy = floor(__dmul_rn((double)py, inv));
   const double cz = floor(__dmul_rn((double)pz, inv));
   const int32_t a = js_toint32(__dmul_rn(cx, 92837111.0));
   const int32_t b = js_toint32(__dmul_rn(cy, 689287499.0));
   const int32_t c = js_toint32(__dmul_rn(cz, 283923481.0));
+  key = (uint32_t)a + 3u * (uint32_t)b + 5u * (uint32_t)c;
   return (uint32_t)(a ^ b ^ c) & mask;
+}
+
+// The slot of a fluid particle in the w of its slot copy.
+__device__ __forceinline__ real slot_pack(float, uint32_t e) { return __uint_as_float(e); }
+__device__ __forceinline__ uint32_t slot_unpack(float w) { return __float_as_uint(w); }
+#ifdef UPBD_FP64_BUILD
+__device__ __forceinline__ real slot_pack(double, uint32_t e) { return (double)e; }
+__device__ __forceinline__ uint32_t slot_unpack(double w) { return (uint32_t)w; }
+#endif
+
+// Words of the grid build and the density pass that live in arrays the bounds
+// pass writes: smove holds the cell keys by particle (count -> rank fix-up),
+// svel the bucket members with their keys (scatter -> rank fix-up), behind them
+// the chunk places (rank fix-up -> density) and the fluid's masses by slot
+// (rank fix-up -> displacement).
+__device__ __forceinline__ uint32_t* cell_keys(const SimView& v) { return reinterpret_cast<uint32_t*>(v.smove); }
+__device__ __forceinline__ float* slot_mass(const SimView& v) { return reinterpret_cast<float*>(v.svel) + 3 * (size_t)v.N; }
+__device__ __forceinline__ uint2* bucket_pairs(const SimView& v) { return reinterpret_cast<uint2*>(v.svel); }
+__device__ __forceinline__ uint32_t* chunk_places(const SimView& v) {
+  return reinterpret_cast<uint32_t*>(v.svel) + 2 * (size_t)v.N;
 }
 
 // std::max / std::min / clamp with the operand order of the oracle (so -0.0

@@ -61,8 +61,9 @@ __global__ void __launch_bounds__(256) k_integrate_count(SimView v, const DevPar
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(SimView v) { b_scan(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_scatter(SimView v) { b_scatter(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_rankfix(SimView v) { b_rankfix(v, blockIdx.x); }
-__global__ void __launch_bounds__(256) k_density(SimView v, const DevParams* __restrict__ P) {
-  b_density(v, P, blockIdx.x);
+// 5 CTAs of 256 per SM: 48 registers (with 6 and 40 a launch took 32.2 us instead of 31.1)
+__global__ void __launch_bounds__(256, 5) k_density(SimView v, const DevParams* __restrict__ P, uint32_t window) {
+  b_density(v, P, window, blockIdx.x);
 }
 template <bool APPLY>
 __global__ void __launch_bounds__(256) k_disp(SimView v, const DevParams* __restrict__ P) {

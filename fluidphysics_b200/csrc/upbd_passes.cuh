@@ -75,8 +75,10 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
     if (i >= v.S) v.mark[i] = 0u;  // contact marks of this substep start clear
   }
   if (COUNT) {
-    const uint32_t h = cell_of(p4.x, p4.y, p4.z, P->inv_cell, (uint32_t)v.T - 1u);
+    uint32_t key;
+    const uint32_t h = cell_of(p4.x, p4.y, p4.z, P->inv_cell, (uint32_t)v.T - 1u, key);
     v.cell[i] = h;
+    if (v.smove) cell_keys(v)[i] = key;
     v.ticket[i] = atomicAdd(&v.counts[h], 1u);
     const int rep = (i >> 5) & (tile_reps(v.num_tiles) - 1);  // a power of two
     atomicAdd(&v.tile_sum[rep * v.num_tiles + (int)(h / SCAN_TILE)], 1u);
@@ -178,6 +180,7 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb) {
 
 // Scatter by ticket (gridScatter, src/gpu/wgsl.js:238-245, without its
 // second atomic), and clear the tile totals for the next count.
+// In a scene the particle's cell key goes along, for the rank fix-up.
 __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i < tile_words(v.num_tiles)) v.tile_sum[i] = 0u;
@@ -185,32 +188,64 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
   if (!(v.flags[i] & F_ACTIVE)) return;
   const uint32_t h = v.cell[i];
   const uint32_t at = v.start[h] + v.ticket[i];
-  if (UPBD_IDX_OK(v, at, v.N)) v.tmp[at] = (uint32_t)i;
+  if (!UPBD_IDX_OK(v, at, v.N)) return;
+  if (v.spos) bucket_pairs(v)[at] = make_uint2((uint32_t)i, cell_keys(v)[i]);
+  else v.tmp[at] = (uint32_t)i;  // the stateless grid build
 }
 
 // Deterministic membership: particle i goes to start[h] + #{j in bucket : j > i},
 // i.e. descending index inside a bucket, the order Solver._buildGrid's
 // `--cellStart[h]` scatter leaves (src/solver.js:182-183).
+//
+//
+// In a scene it also lays out the density pass's chunks: up to CHUNK fluid
+// particles of one bucket and one cell (bucket mates of another cell, found in
+// one bucket of seven in a settled pool, would need candidates of their own).
+// Inside a bucket the fluid's slots are listed by (cell key, slot) at the
+// bucket's places of chunk_places, the first of each chunk with the chunk's
+// size in the bits above CHUNK_SHIFT. The slot copy of a fluid particle carries
+// its slot where the mass would be, for the density pass's lists; the mass goes
+// to slot_mass.
 __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i >= v.N) return;
   if (!(v.flags[i] & F_ACTIVE)) return;
   const uint32_t h = v.cell[i];
   const uint32_t s = v.start[h], e = v.start[h + 1];
-  uint32_t rank = 0, solids = 0;
   if (!UPBD_IDX_OK(v, e, (uint32_t)v.N + 1u)) return;
+  uint32_t rank = 0;
+  if (!v.spos) {  // the stateless grid build has no bucket-ordered copies
+    for (uint32_t k = s; k < e; k++) rank += (v.tmp[k] > (uint32_t)i) ? 1u : 0u;
+    if (UPBD_IDX_OK(v, s + rank, v.N)) v.entries[s + rank] = (uint32_t)i;
+    return;
+  }
+  real4 p = v.pos[i];
+  const uint32_t key = cell_keys(v)[i];
+  const uint2* __restrict__ pairs = bucket_pairs(v);
+  uint32_t solids = 0, before = 0, mates = 0, rank_in = 0;
   for (uint32_t k = s; k < e; k++) {
-    const uint32_t j = v.tmp[k];
-    rank += (j > (uint32_t)i) ? 1u : 0u;
-    solids += (j < (uint32_t)v.S) ? 1u : 0u;
+    const uint2 j = pairs[k];
+    const bool ahead = j.x > (uint32_t)i, solid = j.x < (uint32_t)v.S, mate = !solid && j.y == key;
+    rank += ahead ? 1u : 0u;
+    solids += solid ? 1u : 0u;
+    before += (!solid && j.y < key) ? 1u : 0u;
+    mates += mate ? 1u : 0u;
+    rank_in += (mate && ahead) ? 1u : 0u;
   }
-  if (!UPBD_IDX_OK(v, s + rank, v.N)) return;
-  v.entries[s + rank] = (uint32_t)i;
-  if (v.spos) {  // the stateless grid build has no bucket-ordered copies
-    v.slot[i] = s + rank;
-    v.spos[s + rank] = v.pos[i];
-    v.fend[h] = e - solids;  // every member writes the same value
+  const uint32_t slot = s + rank;
+  if (!UPBD_IDX_OK(v, slot, v.N)) return;
+  v.entries[slot] = (uint32_t)i;
+  v.slot[i] = slot;
+  v.fend[h] = e - solids;  // every member writes the same value
+  if (i >= v.S) {
+    const uint32_t n = (rank_in % CHUNK == 0u) ? min(CHUNK, mates - rank_in) : 0u;
+    chunk_places(v)[s + before + rank_in] = slot | (n << CHUNK_SHIFT);
+    slot_mass(v)[slot] = (float)p.w;
+    p.w = slot_pack(real(0), slot);
+  } else {
+    chunk_places(v)[slot] = 0u;  // solids follow the fluid: no chunk starts there
   }
+  v.spos[slot] = p;
 }
 
 // ------------------------------------------------------------------ fluid
@@ -231,58 +266,254 @@ __device__ __forceinline__ void slot_group(const SimView& v, uint32_t t, uint32_
 
 // fluidDensity, src/gpu/wgsl.js:254-279. Every grid entry is active (the
 // grid is built from the active particles of this substep, before bounds).
-__device__ __forceinline__ void b_density(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const uint32_t t = UPBD_VTID;
-  const int lane = threadIdx.x & (GLF - 1);
-  uint32_t myslot, i;
-  bool act;
-  slot_group(v, t, myslot, i, act);
-  if (!__any_sync(0xffffffffu, act)) return;  // a warp of solid slots (or past the active count)
-  real rho = 0.f, rhoNear = 0.f;
-  const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
-  CellHash ch;
-  group_cell_hash<GLF>(pi.x, pi.y, pi.z, P->inv_cell, ch);
+//
+// A warp takes one chunk (rank fix-up): up to CHUNK fluid particles of one
+// cell, GLF lanes each. They share their 27 buckets, so the warp looks them up
+// once, a lane a bucket, and copies their fluid to shared memory (four lanes a
+// bucket, asynchronous 16-byte copies that bring the slot along); each
+// particle's lanes then test their shares there: no cursor, no branch, one
+// 16-byte shared load and eight operations a candidate, a bit kept for each
+// candidate within the list radius. The bits (one candidate in five) are then
+// walked with the square root, the sums and the list entry. The order is
+// lane_strided's (candidate c to lane c mod GLF, each lane in sequence), so are
+// the sums. A round stages at most STAGE candidates; longer sequences take more
+// rounds, and particles whose cell is another one after all (equal keys)
+// another turn. A block's warps share out the chunks that start in its window of
+// places: 128 for large scenes (two to three chunks a warp in a settled pool,
+// so that uneven chunks even out), fewer where that would leave SMs idle.
+// Bound by the latency of the shared loads, square roots and shuffles between
+// its instructions (54 % of the issue slots of an active SM). On the default
+// scene's settled pool (65,536 fluid, 120 candidates and 22 listed each; B200,
+// event-timed) a launch takes 29.8 us; a walk of each group of GLF lanes with its
+// own cursor, 46 instructions a candidate, took 42.8 us; on the large scene 121
+// against 173 us. With half a warp a chunk of 4 it took 40 us (the set-up is
+// shared by half as many), with a warp over 8 consecutive slots of several cells
+// 73 us.
+constexpr uint32_t STAGE = 4096 / sizeof(real4);     // 256 candidates a warp and round (FP64: 128)
+constexpr size_t STAGE_WARP = STAGE * sizeof(real4);  // dynamic shared bytes per warp
+constexpr uint32_t WINDOW_MAX = 128;                  // places of a block's window
+
+__device__ __forceinline__ void copy_row_async(real4* dst, const real4* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll
+  for (int k = 0; k < (int)sizeof(real4); k += 16)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + k), "l"((const char*)src + k) : "memory");
+}
+__device__ __forceinline__ void copy_rows_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Squared distance inside the gathers: the product build's rounding is spelled
+// out (the compiler may fuse either product first), the parity build's
+// operations are the reference's.
+__device__ __forceinline__ real dist2(real ex, real ey, real ez) {
+#ifdef UPBD_PARITY_BUILD
+  return dot3(ex, ey, ez, ex, ey, ez);
+#else
+  return r_fma(ez, ez, r_fma(ex, ex, ey * ey));
+#endif
+}
+
+// bits << 1, plus 1 where d2 is below lim (the parity build: not at or above)
+__device__ __forceinline__ uint32_t push_listed(uint32_t bits, real d2, real lim) {
+#if defined(UPBD_PARITY_BUILD) || defined(UPBD_FP64_BUILD)
+  return (bits << 1) | (d2 >= lim ? 0u : 1u);
+#else
+  return __funnelshift_l(__float_as_uint(d2 - lim), bits, 1);  // the sign of the difference (a NaN's is clear)
+#endif
+}
+
+// threadIdx.x in a register: read once, not again wherever a lane is needed
+__device__ __forceinline__ int thread_index() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
+// One round's copies: candidates q0 .. of the sequence whose bucket k starts at
+// place off (lane k) and slot s0 and ends at end. CLIP: only those below q0 +
+// STAGE, else all there are.
+template <bool CLIP>
+__device__ __forceinline__ void stage_rows(const SimView& v, real4* sx, int L, uint32_t s0, uint32_t off, uint32_t end,
+                                           uint32_t q0) {
+  const unsigned FULL = 0xffffffffu;
+  const real4* __restrict__ spos = v.spos;
+  const uint32_t NS = (uint32_t)v.N;
+#pragma unroll
+  for (int r = 0; r < 4; r++) {  // buckets 8 r + L / 4, rows L mod 4 and every fourth after it
+    const int src = 8 * r + L / 4;
+    uint32_t o = __shfl_sync(FULL, off, src), hi = __shfl_sync(FULL, end, src);
+    const uint32_t sb = __shfl_sync(FULL, s0, src) - o;
+    if (CLIP) {
+      o = max(o, q0);
+      hi = min(hi, q0 + STAGE);
+    }
+    uint32_t k = o + (uint32_t)(L & 3);
+    do {
+#pragma unroll
+      for (int m = 0; m < 2; m++, k += 4)
+        if (k < hi) {
+          if (UPBD_IDX_OK(v, sb + k, NS)) copy_row_async(&sx[CLIP ? k - q0 : k], &spos[sb + k]);
+          else sx[CLIP ? k - q0 : k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never listed (reported)
+        }
+    } while (__any_sync(FULL, k < hi));
+  }
+}
+
+// window <= min(WINDOW_MAX, blockDim), at most 256 threads a block.
+__device__ __forceinline__ void b_density(const SimView& v, const DevParams* __restrict__ P, uint32_t window,
+                                          uint32_t vb) {
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  __shared__ uint32_t s_chunk[WINDOW_MAX], s_fill[WINDOW_MAX / 32], s_next;
+  const unsigned FULL = 0xffffffffu;
+  const int tid = thread_index();
+  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1), g = L / GLF;
+  // the window's chunks
+  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  if (first >= nact) return;
+  const uint32_t place = first + (uint32_t)tid;
+  uint32_t word = 0, before = 0;
+  if ((uint32_t)wid * 32u < window) {
+    if ((uint32_t)tid < window && place < nact) word = chunk_places(v)[place] >> CHUNK_SHIFT;
+    const unsigned b = __ballot_sync(FULL, word != 0u);
+    if (L == 0) s_fill[wid] = (uint32_t)__popc(b);
+    before = (uint32_t)__popc(b & ((1u << L) - 1u));
+  }
+  if (tid == 0) s_next = blockDim.x >> 5;
+  __syncthreads();
+  uint32_t chunks = 0;
+#pragma unroll
+  for (int w = 0; w < (int)(WINDOW_MAX / 32); w++)
+    if ((uint32_t)w * 32u < window) {
+      if (w == wid && word) s_chunk[chunks + before] = (uint32_t)tid | (word << 8);
+      chunks += s_fill[w];
+    }
+  __syncthreads();
+  real4* __restrict__ sx = reinterpret_cast<real4*>(s_stage + wid * STAGE_WARP);
+  const double inv = P->inv_cell;
   const real H = P->fluid_h, H2 = H * H;
   const real HS = H * (1.0f + XSKIN), HS2 = HS * HS;  // list radius (for xsph)
-  const real4* __restrict__ spos = v.spos;
-  // lane l's c-th listed candidate goes to row l*NL + c, column myslot
   const uint32_t NS = (uint32_t)v.N;
-  uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
-  uint32_t cnt = 0;
 #ifndef UPBD_PARITY_BUILD
   const real invH = 1.0f / H;
 #endif
-  lane_strided<0, GLF>(v, ch, lane, act, [&](uint32_t e) { return spos[e]; }, [&](uint32_t e, const real4& pj) {
-    const real ex = pj.x - pi.x, ey = pj.y - pi.y, ez = pj.z - pi.z;
-    const real d2 = dot3(ex, ey, ez, ex, ey, ez);
+  for (uint32_t c = (uint32_t)wid; c < chunks;) {
+    const uint32_t d = s_chunk[c];
+    const bool act = (uint32_t)g < (d >> 8);
+    const uint32_t myslot = act ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
+    const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
+    // lane l's c-th listed candidate goes to row l*NL + c, column myslot
+    uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
+    uint32_t cnt = 0;
+    real rho = 0.f, rhoNear = 0.f;
+    const double ca = floor(__dmul_rn((double)(lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z)), inv));
+    unsigned rem = __ballot_sync(FULL, act);  // particles whose cell has not had its turn
+    do {
+      // the first remaining particle and those of its cell
+      const int ll = __ffs((int)rem) - 1;
+      const bool other = !(ca == __shfl_sync(FULL, ca, ll + lane));
+      unsigned turn = ~__ballot_sync(FULL, other);
+      turn &= (turn >> 1) & (turn >> 2) & 0x11111111u;  // groups with all three coordinates equal
+      turn = ((turn * 15u) | (15u << ll)) & rem;
+      rem &= ~turn;
+      // its cell's hash components, one per lane (CellHash::init's values), and
+      // the range of bucket L
+      const int axis = (L < 9) ? L / 3 : 2;
+      const double cl = __shfl_sync(FULL, ca, ll + axis);
+      const double K = (axis == 0) ? 92837111.0 : ((axis == 1) ? 689287499.0 : 283923481.0);
+      const int32_t comp = js_toint32(__dmul_rn(__dadd_rn(cl, (double)(L - 3 * axis - 1)), K));
+      const int ka = L / 9, kb = (L - 9 * ka) / 3, kc = L - 9 * ka - 3 * kb;
+      const uint32_t hb = (uint32_t)(__shfl_sync(FULL, comp, ka) ^ __shfl_sync(FULL, comp, 3 + kb) ^
+                                     __shfl_sync(FULL, comp, 6 + kc)) & ((uint32_t)v.T - 1u);
+      uint32_t s0 = 0, n = 0;
+      if (L < 27) {
+        s0 = __ldg(&v.start[hb]);
+        n = __ldg(&v.fend[hb]) - s0;
+      }
+      uint32_t end = n;  // inclusive scan in cell order
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, end, o);
+        if (L >= o) end += y;
+      }
+      const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
+      for (uint32_t q0 = 0; q0 < total; q0 += STAGE) {
+        if (total <= STAGE) stage_rows<false>(v, sx, L, s0, off, end, 0u);
+        else stage_rows<true>(v, sx, L, s0, off, end, q0);
+        copy_rows_wait();
+        __syncwarp();
+        const uint32_t len = min(total - q0, STAGE);
+        const uint32_t mine = (turn >> L & 1u) ? (len + (GLF - 1) - lane) / GLF : 0u;  // this lane's share
+        const real4* __restrict__ row = sx + lane;
+        for (uint32_t u0 = 0; u0 * GLF < len; u0 += 32, row += 32 * GLF) {
+          // up to 32 candidates a lane, the first one's bit on top
+          const uint32_t steps = min((len + (GLF - 1)) / GLF - u0, 32u);
+          uint32_t bits = 0;
+          const real4* __restrict__ r4 = row;
+          for (uint32_t u = 0; u < steps; u += 4, r4 += 4 * GLF) {  // reads past the share stay in the warp's rows
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const real4 pj = r4[k * GLF];
+              const real d2 = dist2(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z);
+              bits = push_listed(bits, d2, HS2);
+            }
+          }
+          bits <<= (32u - ((steps + 3u) & ~3u)) & 31u;
+          const uint32_t own = (mine > u0) ? mine - u0 : 0u;  // drop the rows past the share
+          if (own < 32u) bits &= ~(0xffffffffu >> own);
+          // two listed candidates at a time: their loads and square roots overlap
+          while (bits) {
+            const int k0 = __clz((int)bits);
+            bits &= ~(0x80000000u >> k0);
+            const int k1 = bits ? __clz((int)bits) : k0;
+            const bool two = bits != 0u;
+            bits &= ~(0x80000000u >> k1);
+            const real4 p0 = row[k0 * GLF], p1 = row[k1 * GLF];
+            const real d0 = dist2(p0.x - pi.x, p0.y - pi.y, p0.z - pi.z);
+            const real d1 = dist2(p1.x - pi.x, p1.y - pi.y, p1.z - pi.z);
+            const uint32_t e0 = slot_unpack(p0.w), e1 = slot_unpack(p1.w);
+            const bool use0 = e0 != myslot, use1 = two && e1 != myslot;
+            const bool in0 = d0 < H2, in1 = d1 < H2;
+            if (use0) {
+              if (cnt < NL) nbr[cnt * NS] = e0 | (in0 ? NBR_IN : 0u);  // for fluidDisp (same positions) and xsph
+              cnt++;
+            }
+            if (use1) {
+              if (cnt < NL) nbr[cnt * NS] = e1 | (in1 ? NBR_IN : 0u);
+              cnt++;
+            }
 #ifdef UPBD_PARITY_BUILD
-    if (e == myslot) return;
-    if (d2 >= HS2) return;
-    if (cnt < NL) nbr[cnt * NS] = e | ((d2 < H2) ? NBR_IN : 0u);  // for fluidDisp (same positions) and xsph
-    cnt++;
-    if (d2 >= H2) return;
-    const real q = 1.0f - r_sqrt(d2) / H;
-    rho = rho + q * q;
-    rhoNear = rhoNear + q * q * q;
+            if (use0 && !(d0 >= H2)) {
+              const real q = 1.0f - r_sqrt(d0) / H;
+              rho = rho + q * q;
+              rhoNear = rhoNear + q * q * q;
+            }
+            if (use1 && !(d1 >= H2)) {
+              const real q = 1.0f - r_sqrt(d1) / H;
+              rho = rho + q * q;
+              rhoNear = rhoNear + q * q * q;
+            }
 #else
-    // branch-free: every lane of the warp takes the same path per candidate
-    const bool in = (e != myslot) && (d2 < H2);
-    const bool listed = (e != myslot) && (d2 < HS2);
-    const real q = 1.0f - approx_sqrt(d2) * invH;
-    const real qq = in ? q * q : 0.0f;
-    rho = rho + qq;
-    rhoNear = rhoNear + qq * q;
-    if (listed && cnt < NL) nbr[cnt * NS] = e | (in ? NBR_IN : 0u);  // for fluidDisp (same positions) and xsph
-    cnt += listed ? 1u : 0u;
+            const real q0_ = r_fma(-approx_sqrt(d0), invH, real(1.0f)), q1_ = r_fma(-approx_sqrt(d1), invH, real(1.0f));
+            const real qq0 = (use0 && in0) ? r_mul(q0_, q0_) : real(0.0f), qq1 = (use1 && in1) ? r_mul(q1_, q1_) : real(0.0f);
+            rho = rho + qq0;
+            rhoNear = r_fma(qq0, q0_, rhoNear);
+            rho = rho + qq1;
+            rhoNear = r_fma(qq1, q1_, rhoNear);
 #endif
-  });
-  if (act) v.ncount[lane * NS + myslot] = cnt;
-  rho = lane_sum<GLF>(rho);
-  rhoNear = lane_sum<GLF>(rhoNear);
-  if (act && lane == 0) {
-    const real2 d = make_real2(rho, rhoNear);
-    v.density[i] = d;
-    v.sdens[myslot] = d;
+          }
+        }
+        __syncwarp();  // the next round rewrites the rows
+      }
+    } while (rem);
+    if (act) v.ncount[lane * NS + myslot] = cnt;
+    rho = lane_sum<GLF>(rho);
+    rhoNear = lane_sum<GLF>(rhoNear);
+    if (act && lane == 0) {
+      const real2 dd = make_real2(rho, rhoNear);
+      v.density[v.entries[myslot]] = dd;
+      v.sdens[myslot] = dd;
+    }
+    if (L == 0) c = atomicAdd(&s_next, 1u);
+    c = __shfl_sync(FULL, c, 0);
   }
 }
 
@@ -424,14 +655,19 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
     sz = sz + __shfl_xor_sync(0xffffffffu, sz, d);
   }
   if (!act || h != 0) return;
+#ifdef UPBD_FP64_BUILD
+  const real w = v.pos[i].w;
+#else
+  const real w = slot_mass(v)[e0];
+#endif
   const real maxTotal = 0.35f * H;
   const real s2 = dot3(sx, sy, sz, sx, sy, sz);
   if (s2 > maxTotal * maxTotal) {
     const real f = maxTotal / r_sqrt(s2);
     sx = sx * f; sy = sy * f; sz = sz * f;
   }
-  if (APPLY) {  // pi is pos[i]: the grid build copied it and nothing moved it since
-    const real4 p = make_real4(pi.x + sx, pi.y + sy, pi.z + sz, pi.w);
+  if (APPLY) {  // pi is pos[i] (but for its w): the grid build copied it and nothing moved it since
+    const real4 p = make_real4(pi.x + sx, pi.y + sy, pi.z + sz, w);
     v.pos[i] = p;
     v.sfp[e0] = p;
     mark_if_cell_changed(v, P, (int)i, pi, p);

@@ -20,6 +20,23 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
   const double maxD2 = 3 * sp * sp + 1e-9;
   std::vector<uint32_t> ca, cb;
   std::vector<double> crest;
+  // 13 of a solid's 26 neighbours have a larger index, five tets to a cell
+  ca.reserve(13 * (size_t)out.S);
+  cb.reserve(13 * (size_t)out.S);
+  crest.reserve(13 * (size_t)out.S);
+  out.tet_idx.reserve(20 * (size_t)out.S);
+  out.tet_vol.reserve(5 * (size_t)out.S);
+  struct Neighbour {
+    int dx, dy, dz;
+    double rest;
+  };
+  std::vector<Neighbour> fwd;
+  for (int dx = -1; dx <= 1; dx++)
+    for (int dy = -1; dy <= 1; dy++)
+      for (int dz = -1; dz <= 1; dz++) {
+        const double d2 = (double)(dx * dx + dy * dy + dz * dz) * sp * sp;
+        if ((dx * 3 + dy) * 3 + dz > 0 && d2 <= maxD2) fwd.push_back({dx, dy, dz, std::sqrt(d2)});
+      }
   int id = 0;
   auto add_lattice = [&](int dim, const double* c) {
     const int base = id;
@@ -31,23 +48,20 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
                                     (float)(c[2] - half + iz * sp), (float)(1 / d.solid_mass));
           id++;
         }
+    // a solid's 13 neighbours of larger index, in ascending index: (dx, dy, dz)
+    // after (0, 0, 0) in lexicographic order
     for (int ix = 0; ix < dim; ix++)
       for (int iy = 0; iy < dim; iy++)
-        for (int iz = 0; iz < dim; iz++)
-          for (int dx = -1; dx <= 1; dx++)
-            for (int dy = -1; dy <= 1; dy++)
-              for (int dz = -1; dz <= 1; dz++) {
-                const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
-                if (jx < 0 || jy < 0 || jz < 0 || jx >= dim || jy >= dim || jz >= dim) continue;
-                const int a = base + (ix * dim + iy) * dim + iz;
-                const int b = base + (jx * dim + jy) * dim + jz;
-                if (b <= a) continue;
-                const double d2 = (double)(dx * dx + dy * dy + dz * dz) * sp * sp;
-                if (d2 > maxD2) continue;
-                ca.push_back(a);
-                cb.push_back(b);
-                crest.push_back(std::sqrt(d2));
-              }
+        for (int iz = 0; iz < dim; iz++) {
+          const uint32_t a = (uint32_t)(base + (ix * dim + iy) * dim + iz);
+          for (const Neighbour& o : fwd) {
+            const int jx = ix + o.dx, jy = iy + o.dy, jz = iz + o.dz;
+            if (jx < 0 || jy < 0 || jz < 0 || jx >= dim || jy >= dim || jz >= dim) continue;
+            ca.push_back(a);
+            cb.push_back((uint32_t)(base + (jx * dim + jy) * dim + jz));
+            crest.push_back(o.rest);
+          }
+        }
   };
   auto signed_vol = [&](int a, int b, int c, int e) {
     auto comp = [&](int p, int q, int k) {
@@ -96,50 +110,35 @@ void build_scene(const upbd_scene_desc& d, HostScene& out) {
     out.cons[c] = make_uint4(ca[c], cb[c], bits, 1u);
   }
   // CSR of the ids incident to each solid, ascending: count, prefix, fill
-  auto csr = [&](std::vector<uint32_t>& adj, size_t n, auto&& each) {
-    adj.assign(out.S + 1 + n, 0);
-    each([&](uint32_t i, uint32_t) { adj[i + 1]++; });
-    for (int i = 0; i < out.S; i++) adj[i + 1] += adj[i];
-    std::vector<uint32_t> at(adj.begin(), adj.begin() + out.S);
-    each([&](uint32_t i, uint32_t id) { adj[out.S + 1 + at[i]++] = id; });
-  };
-  csr(out.adj, 2 * (size_t)C, [&](auto&& put) {
-    for (int c = 0; c < C; c++) {
-      put(ca[c], (uint32_t)c);
-      put(cb[c], (uint32_t)c);
-    }
-  });
+  out.adj.assign(out.S + 1 + 2 * (size_t)C, 0);
+  for (int c = 0; c < C; c++) {
+    out.adj[ca[c] + 1]++;
+    out.adj[cb[c] + 1]++;
+  }
+  for (int i = 0; i < out.S; i++) out.adj[i + 1] += out.adj[i];
   // CSR-parallel static data of the Jacobi gather: the other endpoint of each
   // incident constraint and the pair scale 1/max(deg_i, deg_j) of
   // src/gpu/wgsl.js:340-354 (endpoints and degrees never change)
-  out.adj_other.assign(2 * (size_t)C, 0);
-  out.adj_scale.assign(2 * (size_t)C, 0.f);
-  for (int i = 0; i < out.S; i++) {
-    const uint32_t degI = out.adj[i + 1] - out.adj[i];
-    for (uint32_t k = out.adj[i]; k < out.adj[i + 1]; k++) {
-      const uint32_t c = out.adj[out.S + 1 + k];
-      const uint32_t other = (ca[c] == (uint32_t)i) ? cb[c] : ca[c];
-      const uint32_t degJ = out.adj[other + 1] - out.adj[other];
-      out.adj_other[k] = other;
-      out.adj_scale[k] = 1.0f / (float)((degI < degJ) ? degJ : degI);
-    }
+  out.adj_other.resize(2 * (size_t)C);
+  out.adj_scale.resize(2 * (size_t)C);
+  std::vector<uint32_t> at(out.adj.begin(), out.adj.begin() + out.S);
+  for (int c = 0; c < C; c++) {
+    const uint32_t a = ca[c], b = cb[c];
+    const uint32_t da = out.adj[a + 1] - out.adj[a], db = out.adj[b + 1] - out.adj[b];
+    const float scale = 1.0f / (float)((da < db) ? db : da);
+    const uint32_t ka = at[a]++, kb = at[b]++;
+    out.adj[out.S + 1 + ka] = out.adj[out.S + 1 + kb] = (uint32_t)c;
+    out.adj_other[ka] = b;
+    out.adj_other[kb] = a;
+    out.adj_scale[ka] = out.adj_scale[kb] = scale;
   }
   const int NT = (int)out.tet_vol.size();
-  csr(out.tet_adj, 4 * (size_t)NT, [&](auto&& put) {
-    for (int t = 0; t < NT; t++)
-      for (int q = 0; q < 4; q++) put(out.tet_idx[4 * t + q], (uint32_t)t);
-  });
-  // CSR-parallel static data of the tet gather: the corners and the pair
-  // scale 1/max(tet degree) of src/gpu/wgsl.js:444-452
-  out.tet_rec.resize(4 * (size_t)NT);
-  out.tet_scale.resize(4 * (size_t)NT);
-  for (size_t k = 0; k < 4 * (size_t)NT; k++) {
-    const uint32_t* q = &out.tet_idx[4 * (size_t)out.tet_adj[out.S + 1 + k]];
-    uint32_t dm = 1;
-    for (int c = 0; c < 4; c++) dm = std::max(dm, out.tet_adj[q[c] + 1] - out.tet_adj[q[c]]);
-    out.tet_rec[k] = make_uint4(q[0], q[1], q[2], q[3]);
-    out.tet_scale[k] = 1.0f / (float)dm;
-  }
+  out.tet_adj.assign(out.S + 1 + 4 * (size_t)NT, 0);
+  for (size_t k = 0; k < 4 * (size_t)NT; k++) out.tet_adj[out.tet_idx[k] + 1]++;
+  for (int i = 0; i < out.S; i++) out.tet_adj[i + 1] += out.tet_adj[i];
+  at.assign(out.tet_adj.begin(), out.tet_adj.begin() + out.S);
+  for (int t = 0; t < NT; t++)
+    for (int c = 0; c < 4; c++) out.tet_adj[out.S + 1 + at[out.tet_idx[4 * (size_t)t + c]]++] = (uint32_t)t;
 }
 
 namespace {
@@ -199,8 +198,8 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.ascl = cv.take<float>(std::max<size_t>(hs.adj_scale.size(), 1));
   L.ccount = cv.take<uint32_t>(scc ? std::max(v.S, 1) : 1);
   L.clist = cv.take<uint32_t>(scc ? (size_t)std::max(v.S, 1) * C_K : 1);
-  L.trec = cv.take<uint4>(tets ? std::max<size_t>(hs.tet_rec.size(), 1) : 1);
-  L.tscl = cv.take<float>(tets ? std::max<size_t>(hs.tet_scale.size(), 1) : 1);
+  L.trec = cv.take<uint4>(tets ? std::max<size_t>(4 * (size_t)v.NT, 1) : 1);
+  L.tscl = cv.take<float>(tets ? std::max<size_t>(4 * (size_t)v.NT, 1) : 1);
   L.sbuf = cv.take<real4>(2 * (size_t)std::max(v.S, 1));
   L.sfp = cv.take<real4>(v.N);
   L.smove = cv.take<float>(v.N);
@@ -321,6 +320,30 @@ cudaError_t state_to_f32(float* dst_dev, const real* src, size_t rows, int comps
 }
 #endif
 
+namespace {
+// The tet gather's static rows, one per CSR entry: the corners of its tet and
+// the pair scale 1/max(tet degree) of src/gpu/wgsl.js:444-452 (degrees in a
+// box lattice are powers of two, so the scale is exact in any type).
+__global__ void k_tet_rows(SimView v, uint4* rec, float* scale) {
+  const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (k >= 4 * v.NT) return;
+  const uint32_t t = v.tet_adj[v.S + 1 + k];
+  uint32_t q[4], dm = 1;
+  for (int c = 0; c < 4; c++) {
+    q[c] = v.tet_idx[4 * t + c];
+    dm = max(dm, v.tet_adj[q[c] + 1] - v.tet_adj[q[c]]);
+  }
+  rec[k] = make_uint4(q[0], q[1], q[2], q[3]);
+  scale[k] = 1.0f / (float)dm;
+}
+
+cudaError_t fill_tet_rows(const SimView& v, cudaStream_t st) {
+  if (!v.tet_rec || v.NT == 0) return cudaSuccess;
+  k_tet_rows<<<(4 * v.NT + 255) / 256, 256, 0, st>>>(v, (uint4*)v.tet_rec, (float*)v.tet_scale);
+  return cudaPeekAtLastError();
+}
+}  // namespace
+
 cudaError_t upload_scene(const HostScene& hs, const SimView& v, cudaStream_t st) {
   cudaError_t e = cudaMemcpyAsync((void*)v.adj, hs.adj.data(), hs.adj.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && !hs.adj_other.empty())
@@ -331,10 +354,7 @@ cudaError_t upload_scene(const HostScene& hs, const SimView& v, cudaStream_t st)
     e = cudaMemcpyAsync((void*)v.tet_adj, hs.tet_adj.data(), hs.tet_adj.size() * 4, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && !hs.tet_idx.empty())
     e = cudaMemcpyAsync(v.tet_idx, hs.tet_idx.data(), hs.tet_idx.size() * 4, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && v.tet_rec && !hs.tet_rec.empty())
-    e = cudaMemcpyAsync((void*)v.tet_rec, hs.tet_rec.data(), hs.tet_rec.size() * sizeof(uint4), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && v.tet_rec && !hs.tet_scale.empty())
-    e = cudaMemcpyAsync((void*)v.tet_scale, hs.tet_scale.data(), hs.tet_scale.size() * 4, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = fill_tet_rows(v, st);
   if (e == cudaSuccess) e = state_to_device((real*)v.pos, (const float*)hs.pos.data(), hs.pos.size(), 4, v, st);
   if (e == cudaSuccess) e = state_to_device((real*)v.prev, (const float*)hs.pos.data(), hs.pos.size(), 4, v, st);
   if (e == cudaSuccess && v.C > 0)
@@ -424,8 +444,7 @@ cudaError_t upload_prepared(const PreparedScene& ps, const SimView& v, cudaStrea
   if (e == cudaSuccess) e = up((void*)v.adj_scale, L.adj_scale.data(), L.adj_scale.size() * 4);
   if (e == cudaSuccess) e = up((void*)v.tet_adj, L.tet_adj.data(), L.tet_adj.size() * 4);
   if (e == cudaSuccess) e = up(v.tet_idx, L.tet_idx.data(), L.tet_idx.size() * 4);
-  if (e == cudaSuccess && v.tet_rec) e = up((void*)v.tet_rec, L.tet_rec.data(), L.tet_rec.size() * sizeof(uint4));
-  if (e == cudaSuccess && v.tet_rec) e = up((void*)v.tet_scale, L.tet_scale.data(), L.tet_scale.size() * 4);
+  if (e == cudaSuccess) e = fill_tet_rows(v, st);
   if (e == cudaSuccess) e = up(v.cons, L.cons.data(), L.cons.size() * 16);
   if (e == cudaSuccess) e = up(v.tet_vol, L.tet_vol.data(), L.tet_vol.size() * 4);
   auto rows = [&](real4* dst, const std::vector<float4>& src, size_t n) {

@@ -23,8 +23,6 @@ struct HostScene {
   std::vector<uint32_t> tet_idx;
   std::vector<float> tet_vol;
   std::vector<uint32_t> tet_adj;
-  std::vector<uint4> tet_rec;     // per tet_adj id: the tet's corners
-  std::vector<float> tet_scale;   // per tet_adj id: 1 / max(tet degree of a corner)
   int S = 0, N1 = 0, N = 0;
 };
 
