@@ -27,8 +27,7 @@ constexpr uint32_t C_K = 40u;           // solid contact cache width, src/gpu/wg
 constexpr int SCAN_THREADS = 256;       // 8 counts per thread (SCAN_TILE / 8)
 
 // scratch words (device)
-constexpr int SCR_PICK_T = 0;      // uint64 bits of the best t (words 0-1)
-constexpr int SCR_PICK_I = 2;      // best index
+constexpr int SCR_PICK = 0;        // pick blocks finished (last-block pattern)
 constexpr int SCR_CUT = 3;         // constraints cut by the last wedge
 constexpr int SCR_ACTIVE = 4;      // active-fluid partial sums
 constexpr int SCR_DONE = 5;        // blocks finished (last-block pattern)
@@ -38,6 +37,8 @@ constexpr int SCR_WORDS = 16;
 // mapped host words
 constexpr int HM_ACTIVE = 0;
 constexpr int HM_HEALTH = 1;
+constexpr int HM_PICK_T = 2;  // pick: uint64 bits of the smallest t (words 2-3)
+constexpr int HM_PICK_I = 4;  // and the index there
 constexpr int HM_WORDS = 8;
 
 // Scalar type of the particle state and of the pass arithmetic: float in
@@ -102,7 +103,6 @@ struct DevParams {
   float4 emit_pos, emit_dir, emit_side, emit_up;
   float4 grab_c;
   double cut_o[4], cut_d1[4], cut_d2[4];
-  double pick_o[4], pick_d[4];  // pick_o[3] = max perpendicular distance
 };
 
 // Device pointers and sizes of one scene (passed by value to kernels).

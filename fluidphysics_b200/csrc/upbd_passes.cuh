@@ -23,6 +23,16 @@ namespace upbd {
 // integrate (src/gpu/wgsl.js:121-160) fused with gridCount
 // (src/gpu/wgsl.js:173-178). The count keeps each particle's arrival ticket
 // and bumps its scan tile's total, so the scan needs no second pass.
+__device__ __forceinline__ void count_particle(const SimView& v, double inv_cell, int i, const real4& p) {
+  uint32_t key;
+  const uint32_t h = cell_of(p.x, p.y, p.z, inv_cell, (uint32_t)v.T - 1u, key);
+  v.cell[i] = h;
+  if (v.smove) cell_keys(v)[i] = key;
+  v.ticket[i] = atomicAdd(&v.counts[h], 1u);
+  const int rep = (i >> 5) & (tile_reps(v.num_tiles) - 1);  // a power of two
+  atomicAdd(&v.tile_sum[rep * v.num_tiles + (int)(h / SCAN_TILE)], 1u);
+}
+
 template <bool INTEGRATE, bool COUNT>
 __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
   const int i = UPBD_VTID;
@@ -74,15 +84,7 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
     v.pos[i] = p4;
     if (i >= v.S) v.mark[i] = 0u;  // contact marks of this substep start clear
   }
-  if (COUNT) {
-    uint32_t key;
-    const uint32_t h = cell_of(p4.x, p4.y, p4.z, P->inv_cell, (uint32_t)v.T - 1u, key);
-    v.cell[i] = h;
-    if (v.smove) cell_keys(v)[i] = key;
-    v.ticket[i] = atomicAdd(&v.counts[h], 1u);
-    const int rep = (i >> 5) & (tile_reps(v.num_tiles) - 1);  // a power of two
-    atomicAdd(&v.tile_sum[rep * v.num_tiles + (int)(h / SCAN_TILE)], 1u);
-  }
+  if (COUNT) count_particle(v, P->inv_cell, i, p4);
 }
 
 // ------------------------------------------------------------ exclusive scan
@@ -91,8 +93,9 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
 // totals of tiles < b (the count's tile counters, all replicas), writes
 // start[], and clears the counts it read. The counts and the earlier totals
 // are loaded up front so that their latencies overlap, and one block barrier
-// publishes both per-warp sums.
-__device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb) {
+// publishes both per-warp sums. COUNTS: the counts themselves go to counts_out.
+template <bool COUNTS = false>
+__device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* __restrict__ counts_out = nullptr) {
   __shared__ uint32_t s_scan[SCAN_THREADS / 32];  // per-warp sums of this tile's counts
   __shared__ uint32_t s_prev[SCAN_THREADS / 32];  // per-warp sums of earlier tiles' totals
   const int tid = threadIdx.x;
@@ -101,7 +104,8 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb) {
   // 16-byte rows when the tile is whole and the arrays allow it (start[] may
   // be a caller's buffer at any 4-byte offset)
   const bool vec = t0 + 8 <= (long long)v.T && ((reinterpret_cast<uintptr_t>(v.counts) | reinterpret_cast<uintptr_t>(v.start) |
-                                                 reinterpret_cast<uintptr_t>(v.fend)) & 15u) == 0;
+                                                 reinterpret_cast<uintptr_t>(v.fend) |
+                                                 reinterpret_cast<uintptr_t>(counts_out)) & 15u) == 0;
   uint32_t c[8];
   if (vec) {
     const uint4 a = *reinterpret_cast<const uint4*>(v.counts + t0);
@@ -155,6 +159,10 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb) {
       *reinterpret_cast<uint4*>(v.fend + t0) = a;
       *reinterpret_cast<uint4*>(v.fend + t0 + 4) = b;
     }
+    if (COUNTS) {
+      *reinterpret_cast<uint4*>(counts_out + t0) = make_uint4(c[0], c[1], c[2], c[3]);
+      *reinterpret_cast<uint4*>(counts_out + t0 + 4) = make_uint4(c[4], c[5], c[6], c[7]);
+    }
     const uint4 z = make_uint4(0u, 0u, 0u, 0u);  // ready for the next count
     *reinterpret_cast<uint4*>(v.counts + t0) = z;
     *reinterpret_cast<uint4*>(v.counts + t0 + 4) = z;
@@ -169,6 +177,7 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb) {
       if (idx < v.T) {
         v.start[idx] = r[k];
         if (v.fend) v.fend[idx] = r[k];
+        if (COUNTS) counts_out[idx] = c[k];
         v.counts[idx] = 0u;
         if (v.bmove) v.bmove[idx] = 0u;
       }
