@@ -38,16 +38,22 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
   const int i = UPBD_VTID;
   if (i >= v.N) return;
   uint32_t f = v.flags[i];
+  real4 p4 = v.pos[i], vv, pv;
+  issued(f);
+  issued(p4);
+  if (INTEGRATE) {
+    vv = v.vel[i];
+    pv = v.prev[i];
+    issued(vv);
+    issued(pv);
+  }
   if (!(f & F_ACTIVE)) return;
-  real4 p4 = v.pos[i];
   if (INTEGRATE) {
     const real h = P->h;
-    const real4 vv = v.vel[i];
     const real vx = vv.x, vz = vv.z;
     const real vy = vv.y + P->gravity * h;
     const real px = p4.x, py = p4.y, pz = p4.z;
     real nx = px + vx * h, ny = py + vy * h, nz = pz + vz * h;
-    const real4 pv = v.prev[i];
     real tw = pv.w;
     bool slipped = false;
     if (f & F_GRABBED) {
@@ -194,11 +200,15 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i < tile_words(v.num_tiles)) v.tile_sum[i] = 0u;
   if (i >= v.N) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
-  const uint32_t h = v.cell[i];
-  const uint32_t at = v.start[h] + v.ticket[i];
+  const uint32_t f = v.flags[i], h = v.cell[i], ticket = v.ticket[i], key = v.spos ? cell_keys(v)[i] : 0u;
+  issued(f);
+  issued(h);
+  issued(ticket);
+  issued(key);
+  if (!(f & F_ACTIVE)) return;
+  const uint32_t at = v.start[h] + ticket;
   if (!UPBD_IDX_OK(v, at, v.N)) return;
-  if (v.spos) bucket_pairs(v)[at] = make_uint2((uint32_t)i, cell_keys(v)[i]);
+  if (v.spos) bucket_pairs(v)[at] = make_uint2((uint32_t)i, key);
   else v.tmp[at] = (uint32_t)i;  // the stateless grid build
 }
 
@@ -218,8 +228,12 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
 __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i >= v.N) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
-  const uint32_t h = v.cell[i];
+  const uint32_t f = v.flags[i], h = v.cell[i];
+  real4 p = v.pos[i];
+  issued(f);
+  issued(h);
+  issued(p);
+  if (!(f & F_ACTIVE)) return;
   const uint32_t s = v.start[h], e = v.start[h + 1];
   if (!UPBD_IDX_OK(v, e, (uint32_t)v.N + 1u)) return;
   uint32_t rank = 0;
@@ -228,7 +242,6 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
     if (UPBD_IDX_OK(v, s + rank, v.N)) v.entries[s + rank] = (uint32_t)i;
     return;
   }
-  real4 p = v.pos[i];
   const uint32_t key = cell_keys(v)[i];
   const uint2* __restrict__ pairs = bucket_pairs(v);
   uint32_t solids = 0, before = 0, mates = 0, rank_in = 0;
@@ -258,20 +271,11 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
 }
 
 // ------------------------------------------------------------------ fluid
-// The fluid-fluid gathers run GLF lanes per particle (see lane_strided): a
-// warp holds 32/GLF particles, every lane reaches the shuffles, and lane 0
-// writes. Groups take the particles in slot order (group g: the particle at
-// slot g of this substep's grid, entries[g]): the particles of one bucket sit
-// in consecutive slots and share their 27 neighbour buckets, so a warp's
-// candidate loads mostly hit L1. A particle's own arithmetic does not depend
-// on which group runs it. Groups whose slot holds a solid, or lies past the
-// active count start[T], have no work.
-__device__ __forceinline__ void slot_group(const SimView& v, uint32_t t, uint32_t& e0, uint32_t& i, bool& fluid) {
-  e0 = t / GLF;
-  const uint32_t nact = __ldg(&v.start[v.T]);
-  i = (e0 < nact) ? v.entries[e0] : 0u;
-  fluid = e0 < nact && i >= (uint32_t)v.S;
-}
+// The fluid-fluid gathers run GLF lanes per particle (see lane_strided); lane 0
+// writes. They take the particles by grid slot: the particles of one bucket sit
+// in consecutive slots and share their 27 neighbour buckets. A particle's own
+// arithmetic does not depend on which group runs it. Groups whose slot holds a
+// solid, or lies past the active count start[T], have no work.
 
 // fluidDensity, src/gpu/wgsl.js:254-279. Every grid entry is active (the
 // grid is built from the active particles of this substep, before bounds).
@@ -559,8 +563,22 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
   constexpr int LPT = GLF / DL;  // lanes' lists per thread
   const uint32_t e0 = UPBD_VTID / DL;
   const int h = (int)(threadIdx.x & (DL - 1));
+  const real4* __restrict__ spos = v.spos;
+  const real2* __restrict__ sdens = v.sdens;
+  const uint32_t NS = (uint32_t)v.N, eld = min(e0, NS - 1u);
   const uint32_t nact = __ldg(&v.start[v.T]);
-  const uint32_t i = (e0 < nact) ? v.entries[e0] : 0u;
+  const uint32_t i = v.entries[eld];
+  const real4 pi = spos[eld];
+  const real2 di = sdens[eld];
+  uint32_t cnt[LPT];
+#pragma unroll
+  for (int u = 0; u < LPT; u++) cnt[u] = v.ncount[(size_t)(h * LPT + u) * NS + eld];
+  issued(nact);
+  issued(i);
+  issued(pi);
+  issued(di);
+#pragma unroll
+  for (int u = 0; u < LPT; u++) issued(cnt[u]);
   const bool act = e0 < nact && i >= (uint32_t)v.S;
   if (DL > 1) {
     if (!__any_sync(0xffffffffu, act)) return;
@@ -569,13 +587,9 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
   }
   const real H = P->fluid_h, H2 = H * H;
   real sx = 0.f, sy = 0.f, sz = 0.f;
-  const real4* __restrict__ spos = v.spos;
-  const real2* __restrict__ sdens = v.sdens;
-  const real4 pi = act ? spos[e0] : make_real4(0.f, 0.f, 0.f, 0.f);
   if (act) {
     const real maxPair = 0.05f * H;
     const real k = P->stiffness, kn = P->near_stiffness, rho0 = P->rest_density;
-    const real2 di = sdens[e0];
     const real Pi = k * (di.x - rho0);
     const real PNi = kn * di.y;
 #ifndef UPBD_PARITY_BUILD
@@ -604,15 +618,10 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
 #endif
       sx = sx - ex * f; sy = sy - ey * f; sz = sz - ez * f;
     };
-    const uint32_t NS = (uint32_t)v.N;
     const int l0 = h * LPT;
-    uint32_t cnt[LPT];
     bool over = false;
 #pragma unroll
-    for (int u = 0; u < LPT; u++) {
-      cnt[u] = v.ncount[(l0 + u) * NS + e0];
-      over = over || cnt[u] > NL;
-    }
+    for (int u = 0; u < LPT; u++) over = over || cnt[u] > NL;
     if (!over) {
       const uint32_t* __restrict__ nbr = v.nbr + e0;
 #pragma unroll
@@ -792,15 +801,25 @@ __device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams*
   }
   const int i = t / GL;
   const int lane = threadIdx.x & (GL - 1);
-  const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
   const real4* __restrict__ pos = (OUT == SOLVE_DELTA) ? v.pos : solid_src(v, q);
-  const real4 pi = (i < v.S) ? pos[i] : make_real4(0.f, 0.f, 0.f, 0.f);
+  real4 pi = make_real4(0.f, 0.f, 0.f, 0.f);
+  uint32_t fl = 0, st = 0, en = 0;
+  if (i < v.S) {
+    fl = v.flags[i];
+    pi = pos[i];
+    st = v.adj[i];
+    en = v.adj[i + 1];
+    issued(fl);
+    issued(pi);
+    issued(st);
+    issued(en);
+  }
+  const bool act = (fl & F_ACTIVE) != 0u;
   real cx = 0.f, cy = 0.f, cz = 0.f;
   if (act) {
     const real wi = pi.w;
     const real h = P->h;
     const real alpha = P->compliance / (h * h);
-    const uint32_t st = v.adj[i], en = v.adj[i + 1];
     const uint32_t* __restrict__ ids = v.adj + v.S + 1;
     const uint4* __restrict__ cons = v.cons;
 #pragma unroll 2
@@ -1001,17 +1020,29 @@ template <bool LAST>
 __device__ __forceinline__ void b_solid_contacts(const SimView& v, const DevParams* __restrict__ P, int q, uint32_t vb) {
   const unsigned FULL = 0xffffffffu;
   const int i = (int)(UPBD_VTID / GL), lane = (int)(threadIdx.x & (GL - 1));
-  const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
   const real4* __restrict__ pos = solid_src(v, q);
-  const real4 pi = (i < v.S) ? pos[i] : make_real4(0.f, 0.f, 0.f, 0.f);
+  real4 pi = make_real4(0.f, 0.f, 0.f, 0.f);
+  uint32_t fl = 0, n = 0, e = 0;
+  if (i < v.S) {
+    fl = v.flags[i];
+    n = v.ccount[i];
+    pi = pos[i];
+    e = v.clist[(size_t)i * C_K + lane];  // the first round's entry, should there be one
+    issued(fl);
+    issued(n);
+    issued(pi);
+    issued(e);
+  }
+  const bool act = (fl & F_ACTIVE) != 0u;
+  if (!act) n = 0;
   const real wi = pi.w;
   real cx = 0.f, cy = 0.f, cz = 0.f;
-  const uint32_t n = act ? v.ccount[i] : 0u;
   for (uint32_t k0 = 0; __any_sync(FULL, k0 < n); k0 += GL) {
     real ex = 0.f, ey = 0.f, ez = 0.f, f = 0.f;
     bool hit = false;
     if (k0 + (uint32_t)lane < n) {
-      const uint32_t e = v.clist[(size_t)i * C_K + k0 + lane], j = e & ~CL_NEAR;
+      if (k0 > 0) e = v.clist[(size_t)i * C_K + k0 + lane];
+      const uint32_t j = e & ~CL_NEAR;
       if (UPBD_IDX_OK(v, j, v.S)) {
         const real4 pj = pos[j];
         const real dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
@@ -1097,11 +1128,23 @@ template <bool LAST>
 __device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* __restrict__ P, int q, uint32_t vb) {
   const unsigned FULL = 0xffffffffu;
   const int i = (int)(UPBD_VTID / GT), lane = (int)(threadIdx.x & (GT - 1));
-  const bool act = i < v.S && (v.flags[i] & F_ACTIVE);
   const real4* __restrict__ pos = solid_src(v, q);
   const uint32_t* __restrict__ ids = v.tet_adj + v.S + 1;
+  real4 pi = make_real4(0.f, 0.f, 0.f, 0.f);
+  uint32_t fl = 0, st = 0, en = 0;
+  if (i < v.S) {
+    fl = v.flags[i];
+    st = v.tet_adj[i];
+    en = v.tet_adj[i + 1];
+    pi = pos[i];
+    issued(fl);
+    issued(st);
+    issued(en);
+    issued(pi);
+  }
+  const bool act = (fl & F_ACTIVE) != 0u;
+  if (!act) en = st;
   real cx = 0.f, cy = 0.f, cz = 0.f;
-  const uint32_t st = act ? v.tet_adj[i] : 0u, en = act ? v.tet_adj[i + 1] : 0u;
   for (uint32_t k0 = st; __any_sync(FULL, k0 < en); k0 += GT) {
     const uint32_t k = k0 + (uint32_t)lane;
     real ox = 0.f, oy = 0.f, oz = 0.f;
@@ -1122,10 +1165,7 @@ __device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* 
       cz = cz + __shfl_sync(FULL, oz, l, GT);
     }
   }
-  if (i < v.S && lane == 0) {
-    const real4 pi = pos[i];
-    solid_store<LAST>(v, q, i, act, act ? apply_clamped(P, pi, cx, cy, cz) : pi);
-  }
+  if (i < v.S && lane == 0) solid_store<LAST>(v, q, i, act, act ? apply_clamped(P, pi, cx, cy, cz) : pi);
 }
 
 // -------------------------------------------- bond update + contacts
@@ -1181,9 +1221,16 @@ __device__ __forceinline__ void tet_update(const SimView& v, const DevParams* __
 // walk (their correction is zero either way).
 __device__ __forceinline__ void contacts_lane(const SimView& v, const DevParams* __restrict__ P, int i, int lane,
                                               int nc) {
-  const bool act = i < nc && (v.flags[i] & F_ACTIVE);
+  uint32_t fl = 0, mk = 0;
+  if (i < nc) {
+    fl = v.flags[i];
+    mk = v.mark[i];
+    issued(fl);
+    issued(mk);
+  }
+  const bool act = (fl & F_ACTIVE) != 0u;
   const bool iSolid = i < v.S;
-  const bool walk = act && (iSolid || !P->use_mark || v.mark[i] != 0u);
+  const bool walk = act && (iSolid || !P->use_mark || mk != 0u);
   const unsigned FULL = 0xffffffffu;
   if (!__any_sync(FULL, walk)) {  // most fluid warps: nothing near a solid, no hash to compute
     if (act && lane == 0) v.delta[i] = make_real4(0.f, 0.f, 0.f, 0.f);
@@ -1285,16 +1332,21 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
                                                           int stage, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i >= v.N) return;
-  uint32_t f = v.flags[i];
+  const uint32_t f = v.flags[i], sl = v.slot[i];
+  real4 p = v.pos[i];
+  const real4 dd = v.delta[i], pv = v.prev[i], ov = v.vel[i];
+  issued(f);
+  issued(sl);
+  issued(p);
+  issued(dd);
+  issued(pv);
+  issued(ov);
   if (!(f & F_ACTIVE)) return;
   const bool iSolid = i < v.S;
   const real r = iSolid ? P->solid_radius : P->fluid_radius;
-  real4 p = v.pos[i];
-  const uint32_t sl = v.slot[i];
   const real4 o = iSolid ? p : v.spos[sl];  // a fluid particle's density-pass position, read before any store
   // applyDeltaAll
   {
-    const real4 dd = v.delta[i];
     real dx = dd.x, dy = dd.y, dz = dd.z;
     const real m2 = dot3(dx, dy, dz, dx, dy, dz);
     if (m2 > r * r) {
@@ -1310,7 +1362,6 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
     return;
   }
   // bounds
-  const real4 pv = v.prev[i];
   real px = p.x, py = p.y, pz = p.z;
   if (py < r) {
     py = r;
@@ -1346,7 +1397,7 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
   if (culled) {
     // xsph still reads a culled neighbour's velocity (src/gpu/wgsl.js:761
     // does not test its flag): its slot keeps the unchanged velocity
-    v.svel[sl] = v.vel[i];
+    v.svel[sl] = ov;
     return;
   }
   // velocityUpdate
@@ -1362,8 +1413,7 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
     vx = vx * q; vy = vy * q; vz = vz * q;
   }
   if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz)) atomicOr(&v.scratch[SCR_HEALTH], 1u);
-  const real vw = v.vel[i].w;
-  const real4 nv = make_real4(vx, vy, vz, vw);
+  const real4 nv = make_real4(vx, vy, vz, ov.w);
   v.vel[i] = nv;
   v.svel[sl] = nv;
 }
@@ -1427,13 +1477,25 @@ template <bool APPLY, int ROLE = 0>
 __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
   const uint32_t t = UPBD_VTID;
   const int lane = threadIdx.x & (GLF - 1);
-  uint32_t myslot, i;
-  bool fluid;
-  slot_group(v, t, myslot, i, fluid);
+  const uint32_t NS = (uint32_t)v.N, myslot = t / GLF, eld = min(myslot, NS - 1u);
+  const uint32_t nact = __ldg(&v.start[v.T]), i = v.entries[eld];
+  real4 pi = v.spos[eld];
+  float sm = v.smove[eld];
+  uint32_t cnt = v.ncount[(size_t)lane * NS + eld];
+  issued(nact);
+  issued(i);
+  issued(pi);
+  issued(sm);
+  issued(cnt);
+  const bool fluid = myslot < nact && i >= (uint32_t)v.S;
   const bool act = fluid && (v.flags[i] & F_ACTIVE);
   if (!__any_sync(0xffffffffu, act)) return;
   real sx = 0.f, sy = 0.f, sz = 0.f, m = 0.f;
-  const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
+  if (!act) {
+    pi = make_real4(0.f, 0.f, 0.f, 0.f);
+    sm = 0.f;
+    cnt = 0u;
+  }
   const real H = P->fluid_h, H2 = H * H;
   const real4* __restrict__ spos = v.spos;
   const real4* __restrict__ svel = v.svel;
@@ -1455,10 +1517,7 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
   // overflowed. The scene's largest recorded movement bounds every bucket's,
   // so when it passes the buckets are not looked at (nor hashed, unless the
   // group walks).
-  const uint32_t NS = (uint32_t)v.N;
   const real allow = xsph_allowance(P), rec = XMOVE_REC * allow;
-  const real sm = act ? v.smove[myslot] : 0.f;
-  const uint32_t cnt = act ? v.ncount[lane * NS + myslot] : 0u;
   uint32_t over = (cnt > NL) ? 1u : 0u;
 #pragma unroll
   for (int d = 1; d < GLF; d <<= 1) over |= __shfl_xor_sync(0xffffffffu, over, d);
