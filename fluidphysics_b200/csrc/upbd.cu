@@ -248,7 +248,7 @@ int launch_substep(upbd_sim* s, int last) {
     UPBD_CK(s, cudaEventRecord(s->join_ev, s->side));
   }
   if (last < UPBD_PASS_DENSITY) return UPBD_OK;
-  // places of a density block's window: at least two blocks an SM where the
+  // places of a density or xsph block's window: at least two blocks an SM where the
   // scene has them
   uint32_t window = WINDOW_MAX;
   while (window > 16 && (long long)v.N < 2ll * s->num_sms * window) window /= 2;
@@ -313,28 +313,10 @@ int launch_substep(upbd_sim* s, int last) {
     L += 2;
   }
   if (last < UPBD_PASS_XSPH) return UPBD_OK;
-  if (last < UPBD_PASS_XSPH_APPLY) {  // stop with the result in delta, as the reference's xsph pass leaves it
-    PROF(s, K_XSPH, k_xsph<false><<<blocks_for((long long)v.N * GLF), 256, 0, st>>>(v, P));
-    L++;
-    return UPBD_OK;
-  }
-  if (!s->prof_on && s->side) {
-    // xsph as two launches side by side: the groups that walk on the side
-    // stream (its launch first, so its long warps start early) and those that
-    // read their lists on the main stream, each launch with the registers its
-    // own form needs. Eager per-kernel timing keeps the one launch of both
-    // forms.
-    UPBD_CK(s, cudaEventRecord(s->fork_ev, st));
-    UPBD_CK(s, cudaStreamWaitEvent(s->side, s->fork_ev, 0));
-    k_xsph<true, 2><<<blocks_for((long long)v.N * GLF), 256, 0, s->side>>>(v, P);
-    UPBD_CK(s, cudaEventRecord(s->join_ev, s->side));
-    k_xsph<true, 1><<<blocks_for((long long)v.N * GLF), 256, 0, st>>>(v, P);
-    UPBD_CK(s, cudaStreamWaitEvent(st, s->join_ev, 0));
-    L += 2;
-    UPBD_KCK(s);
-    return UPBD_OK;
-  }
-  PROF(s, K_XSPH, k_xsph<true><<<blocks_for((long long)v.N * GLF), 256, 0, st>>>(v, P));
+  if (last < UPBD_PASS_XSPH_APPLY)  // stop with the result in delta, as the reference's xsph pass leaves it
+    PROF(s, K_XSPH, k_xsph<false><<<blocks_for(v.N, (int)window), 256, 8 * STAGE_WARP, st>>>(v, P, window));
+  else
+    PROF(s, K_XSPH, k_xsph<true><<<blocks_for(v.N, (int)window), 256, 8 * STAGE_WARP, st>>>(v, P, window));
   L++;
   UPBD_KCK(s);
   return UPBD_OK;

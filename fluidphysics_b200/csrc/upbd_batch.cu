@@ -39,8 +39,7 @@ enum Domain {
   D_N,        // particles (integrate/count, rankfix, apply+bounds+velocity)
   D_TILES,    // scan tiles of the bucket table (SCAN_THREADS per block)
   D_SCATTER,  // max(particles, scan tiles)
-  D_CHUNK,    // windows of half a block's threads in grid slots (density)
-  D_FGL,      // GLF lanes per grid slot (xsph)
+  D_CHUNK,    // windows of half a block's threads in grid slots (density, xsph)
   D_DISP,     // DL threads per grid slot (displacement)
   D_F,        // fluid particles (apply, xsph apply, active count)
   D_SOLVE0,   // solve lanes rounded to warps + fluid (first iteration)
@@ -172,8 +171,8 @@ __global__ void __launch_bounds__(256) kb_solid_visc_apply(BatchArgs a) {
     if (P->solid_viscosity > 0.f) b_solid_visc_apply(v, vb);
   });
 }
-__global__ void __launch_bounds__(256) kb_xsph(BatchArgs a) {
-  batch_loop<D_FGL, false>(a, UPBD_BODY { b_xsph<true>(v, P, vb); });
+__global__ void __launch_bounds__(256, 4) kb_xsph(BatchArgs a) {
+  batch_loop<D_CHUNK, true, true>(a, UPBD_BODY { b_xsph<true>(v, P, blockDim.x / 2, vb); });
 }
 __global__ void __launch_bounds__(256) kb_count_active(BatchArgs a) {
   batch_loop<D_F, true>(a, UPBD_BODY { b_count_active(v, vb, nblk); });
@@ -195,7 +194,6 @@ void scene_blocks(const SimView& v, bool tets, int bt, uint32_t out[NUM_DOMAINS]
   out[D_TILES] = (uint32_t)std::max(v.num_tiles, 1);
   out[D_SCATTER] = ceil_div(std::max(v.N, tile_words(v.num_tiles)), bt);
   out[D_CHUNK] = ceil_div(v.N, bt / 2);
-  out[D_FGL] = ceil_div((long long)v.N * GLF, bt);
   out[D_DISP] = ceil_div((long long)v.N * DL, bt);
   out[D_F] = ceil_div(v.F, bt);
   out[D_SOLVE0] = ceil_div((long long)sp + v.F, bt);
@@ -475,7 +473,7 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
       BLAUNCH(b, K_SOLID_VISC, kb_solid_visc<<<G, BT, 0, st>>>(a));
       BLAUNCH(b, K_SOLID_VISC, kb_solid_visc_apply<<<G, BT, 0, st>>>(a));
     }
-    BLAUNCH(b, K_XSPH, kb_xsph<<<G, BT, 0, st>>>(a));  // writes the blended velocity itself
+    BLAUNCH(b, K_XSPH, kb_xsph<<<G, BT, (BT / 32) * STAGE_WARP, st>>>(a));  // writes the blended velocity itself
   }
   BLAUNCH(b, K_COUNT_ACTIVE, kb_count_active<<<G, BT, 0, st>>>(a));
   const cudaError_t e = cudaPeekAtLastError();

@@ -132,9 +132,12 @@ struct SimView {
   // Bucket-ordered copies, slot e matching entries[e]: neighbour gathers read
   // a candidate's data with one load at its slot instead of entries -> pos.
   // Every pass that moves a particle also writes its slot's copy.
-  real4* spos;         // position + inverse mass (fluid, until the bounds pass: + slot)
+  real4* spos;         // position + inverse mass (fluid: + slot)
   real2* sdens;        // (rho, rho_near) of the density pass
-  real4* svel;         // velocity after velocityUpdate
+  // Row pairs (2 N rows): position + slot and velocity of the fluid particle at
+  // slot e after the bounds pass, at 2 e and 2 e + 1, for xsph. Until that
+  // pass the memory serves earlier ones (bucket_pairs, slot_mass, sfp).
+  real4* pvrow;
   uint32_t* slot;      // slot of particle i in this substep's grid
   // Inside a bucket, entries run in descending index, so fluid (indices >= S)
   // precede solids: fend[h] splits bucket h into [start[h], fend[h]) fluid and
@@ -158,7 +161,7 @@ struct SimView {
   real4* sbuf;         // 2 x S: solid positions between folded solve iterations
   // Slot-ordered fluid positions after applyDeltaFluid: the contact passes
   // (marks, solid-fluid contacts) read the fluid there, while spos keeps the
-  // positions the fluid gathers saw until the bounds pass rewrites it.
+  // positions the fluid gathers saw (the second half of pvrow's memory).
   real4* sfp;
   uint32_t* ccount;
   uint32_t* clist;
@@ -361,7 +364,7 @@ __device__ __forceinline__ uint32_t walk_tables(const SimView& v, const CellHash
   return run;
 }
 
-template <int PART, int G = GL, int U = 1, class Load, class Use>
+template <int PART, int G = GL, class Load, class Use>
 __device__ __forceinline__ void lane_strided(const SimView& v, const CellHash& ch, int lane, bool walk, Load&& load,
                                              Use&& use) {
   static_assert(G <= 32 && GLF <= G, "walk tables are sized for GLF..32 lanes");
@@ -373,96 +376,18 @@ __device__ __forceinline__ void lane_strided(const SimView& v, const CellHash& c
   const int g = (int)(threadIdx.x >> 5) * (32 / GLF) + (int)(threadIdx.x & 31) / G;
   const uint32_t run = walk_tables<PART, G>(v, ch, lane, walk, g);
   uint32_t k = 0, next = s_off[g][1], base = s_base[g][0];
-  if (U == 1) {
-    // one candidate per step: where every group walks, unrolling to keep
-    // several loads in flight costs more in registers (occupancy) than it
-    // wins in latency on B200
-    for (uint32_t c = (uint32_t)lane; c < run; c += G) {
-      while (c >= next) {  // next non-empty cell (the total ends the sequence)
-        k++;
-        next = s_off[g][k + 1];
-        base = s_base[g][k];
-      }
-      const uint32_t e = base + c;
-      if (UPBD_IDX_OK(v, e, v.N)) use(e, load(e));
+  // one candidate per step: unrolling to keep several loads in flight costs
+  // more in registers (occupancy) than it wins in latency
+  for (uint32_t c = (uint32_t)lane; c < run; c += G) {
+    while (c >= next) {  // next non-empty cell (the total ends the sequence)
+      k++;
+      next = s_off[g][k + 1];
+      base = s_base[g][k];
     }
-  } else {
-    // U candidates per step, their loads in flight together (for the few
-    // groups that walk while the rest of the kernel reads lists)
-    for (uint32_t c0 = (uint32_t)lane; c0 < run; c0 += G * U) {
-      uint32_t e[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const uint32_t c = c0 + (uint32_t)(u * G);
-        if (c < run) {
-          while (c >= next) {
-            k++;
-            next = s_off[g][k + 1];
-            base = s_base[g][k];
-          }
-          e[u] = base + c;
-          if (!UPBD_IDX_OK(v, e[u], v.N)) e[u] = 0u;  // out of range: slot 0 instead (reported)
-        } else {
-          e[u] = e[0];  // c0 < run: a valid slot, loaded again and not used
-        }
-      }
-      decltype(load(0u)) x[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) x[u] = load(e[u]);
-#pragma unroll
-      for (int u = 0; u < U; u++)
-        if (c0 + (uint32_t)(u * G) < run) use(e[u], x[u]);
-    }
+    const uint32_t e = base + c;
+    if (UPBD_IDX_OK(v, e, v.N)) use(e, load(e));
   }
   __syncwarp();  // the next call may rewrite this group's cells
-}
-
-// The same walk for warps where only a few groups walk: for each walking
-// group in turn, all 32 lanes of the warp load its next 32 candidates (one
-// each, all in flight together) into shared memory, and the group's lanes
-// then use them in their own order (lane l: candidates l, l+G, ..., as in
-// lane_strided, so the results are the same bit for bit). Every lane of the
-// warp must call it; at most 256 threads per block.
-template <int PART, int G, class Load, class Use>
-__device__ __forceinline__ void lane_staged(const SimView& v, const CellHash& ch, int lane, bool walk, Load&& load,
-                                            Use&& use) {
-  static_assert(G <= 32 && GLF <= G && 32 % G == 0, "walk tables are sized for GLF..32 lanes");
-  using X = decltype(load(0u));
-  __shared__ X s_x[256 / 32][32];
-  __shared__ uint32_t s_e[256 / 32][32];
-  auto& s_base = s_walk_base;
-  auto& s_off = s_walk_off;
-  const int w = (int)(threadIdx.x >> 5), L = (int)(threadIdx.x & 31);
-  const int g = w * (32 / GLF) + L / G;
-  walk_tables<PART, G>(v, ch, lane, walk, g);
-  unsigned todo = __ballot_sync(0xffffffffu, walk && lane == 0);  // one bit per walking group
-  while (todo) {
-    const int first = __ffs(todo) - 1;  // the group's lane 0
-    todo &= todo - 1u;
-    const int gw = w * (32 / GLF) + first / G;
-    const bool mine = (L / G) == (first / G);
-    const uint32_t run = s_off[gw][27];
-    uint32_t k = 0, next = s_off[gw][1], base = s_base[gw][0];
-    for (uint32_t c0 = 0; c0 < run; c0 += 32) {
-      const uint32_t c = c0 + (uint32_t)L;
-      if (c < run) {
-        while (c >= next) {
-          k++;
-          next = s_off[gw][k + 1];
-          base = s_base[gw][k];
-        }
-        uint32_t e = base + c;
-        if (!UPBD_IDX_OK(v, e, v.N)) e = 0u;  // out of range: slot 0 instead (reported)
-        s_e[w][L] = e;
-        s_x[w][L] = load(e);
-      }
-      __syncwarp();
-      if (mine)
-        for (uint32_t j = (uint32_t)lane; j < 32u && c0 + j < run; j += G) use(s_e[w][j], s_x[w][j]);
-      __syncwarp();
-    }
-  }
-  __syncwarp();  // the next call may rewrite this warp's rows
 }
 
 // Square roots inside the gathers' candidate loops. The parity build keeps
@@ -512,17 +437,38 @@ __device__ __forceinline__ void issued(const real4& x) {
 }
 __device__ __forceinline__ void issued(const real2& x) { issued(x.x); }
 
+// A row pair with one 32-byte access (the pair is 32-byte aligned).
+__device__ __forceinline__ void load_row_pair(const float4* src, float4& a, float4& b) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(src));
+}
+__device__ __forceinline__ void store_row_pair(float4* dst, const float4& a, const float4& b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(a.x), "f"(a.y), "f"(a.z),
+               "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+#ifdef UPBD_FP64_BUILD
+__device__ __forceinline__ void load_row_pair(const real4* src, real4& a, real4& b) {
+  a = src[0];
+  b = src[1];
+}
+__device__ __forceinline__ void store_row_pair(real4* dst, const real4& a, const real4& b) {
+  dst[0] = a;
+  dst[1] = b;
+}
+#endif
+
 // Words of the grid build and the density pass that live in arrays the bounds
 // pass writes: smove holds the cell keys by particle (count -> rank fix-up),
-// svel the bucket members with their keys (scatter -> rank fix-up), behind them
-// the chunk places (rank fix-up -> density) and the fluid's masses by slot
-// (rank fix-up -> displacement).
+// pvrow the bucket members with their keys (scatter -> rank fix-up), behind them
+// the fluid's masses by slot (rank fix-up -> displacement). The chunk places
+// (rank fix-up -> density, xsph) are the array the stateless grid build
+// scatters into.
 __device__ __forceinline__ uint32_t* cell_keys(const SimView& v) { return reinterpret_cast<uint32_t*>(v.smove); }
-__device__ __forceinline__ float* slot_mass(const SimView& v) { return reinterpret_cast<float*>(v.svel) + 3 * (size_t)v.N; }
-__device__ __forceinline__ uint2* bucket_pairs(const SimView& v) { return reinterpret_cast<uint2*>(v.svel); }
-__device__ __forceinline__ uint32_t* chunk_places(const SimView& v) {
-  return reinterpret_cast<uint32_t*>(v.svel) + 2 * (size_t)v.N;
-}
+__device__ __forceinline__ float* slot_mass(const SimView& v) { return reinterpret_cast<float*>(v.pvrow) + 2 * (size_t)v.N; }
+__device__ __forceinline__ uint2* bucket_pairs(const SimView& v) { return reinterpret_cast<uint2*>(v.pvrow); }
+__device__ __forceinline__ uint32_t* chunk_places(const SimView& v) { return v.tmp; }
 
 // std::max / std::min / clamp with the operand order of the oracle (so -0.0
 // and NaN resolve the same way on both sides).

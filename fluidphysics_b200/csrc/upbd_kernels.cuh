@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(256) k_solid_visc(SimView v, const DevParams* 
   b_solid_visc(v, P, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_solid_visc_apply(SimView v) { b_solid_visc_apply(v, blockIdx.x); }
-template <bool APPLY, int ROLE = 0>
-__global__ void __launch_bounds__(256) k_xsph(SimView v, const DevParams* __restrict__ P) {
-  b_xsph<APPLY, ROLE>(v, P, blockIdx.x);
+// 4 CTAs of 256 per SM: four list entries in flight without spills (5 CTAs and
+// 48 registers: 26.3 us instead of 23.0 on the default scene)
+template <bool APPLY>
+__global__ void __launch_bounds__(256, 4) k_xsph(SimView v, const DevParams* __restrict__ P, uint32_t window) {
+  b_xsph<APPLY>(v, P, window, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_count_active(SimView v) { b_count_active(v, blockIdx.x, gridDim.x); }
 

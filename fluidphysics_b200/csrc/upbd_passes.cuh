@@ -341,65 +341,107 @@ __device__ __forceinline__ int thread_index() {
   return t;
 }
 
-// One round's copies: candidates q0 .. of the sequence whose bucket k starts at
-// place off (lane k) and slot s0 and ends at end. CLIP: only those below q0 +
-// STAGE, else all there are.
-template <bool CLIP>
-__device__ __forceinline__ void stage_rows(const SimView& v, real4* sx, int L, uint32_t s0, uint32_t off, uint32_t end,
-                                           uint32_t q0) {
+// One round's copies: copy(row, slot) for candidates q0 .. of the sequence whose
+// bucket k starts at place off (lane k) and slot s0 and ends at end, ROWS of them
+// a round (CLIP: where there is more than one).
+template <uint32_t ROWS, bool CLIP, class Copy>
+__device__ __forceinline__ void stage_rows(int L, uint32_t s0, uint32_t off, uint32_t end, uint32_t q0, Copy&& copy) {
   const unsigned FULL = 0xffffffffu;
-  const real4* __restrict__ spos = v.spos;
-  const uint32_t NS = (uint32_t)v.N;
 #pragma unroll
   for (int r = 0; r < 4; r++) {  // buckets 8 r + L / 4, rows L mod 4 and every fourth after it
-    const int src = 8 * r + L / 4;
-    uint32_t o = __shfl_sync(FULL, off, src), hi = __shfl_sync(FULL, end, src);
-    const uint32_t sb = __shfl_sync(FULL, s0, src) - o;
+    const int owner = 8 * r + L / 4;
+    uint32_t o = __shfl_sync(FULL, off, owner), hi = __shfl_sync(FULL, end, owner);
+    const uint32_t sb = __shfl_sync(FULL, s0, owner) - o;
     if (CLIP) {
       o = max(o, q0);
-      hi = min(hi, q0 + STAGE);
+      hi = min(hi, q0 + ROWS);
     }
     uint32_t k = o + (uint32_t)(L & 3);
     do {
 #pragma unroll
       for (int m = 0; m < 2; m++, k += 4)
-        if (k < hi) {
-          if (UPBD_IDX_OK(v, sb + k, NS)) copy_row_async(&sx[CLIP ? k - q0 : k], &spos[sb + k]);
-          else sx[CLIP ? k - q0 : k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never listed (reported)
-        }
+        if (k < hi) copy(CLIP ? k - q0 : k, sb + k);
     } while (__any_sync(FULL, k < hi));
   }
+}
+
+// The chunks that start among the window places from `first` on, listed in
+// s_chunk as (place - first | size << 8); returns how many. Every thread of the
+// block calls it.
+struct ChunkList {
+  uint32_t chunk[WINDOW_MAX], fill[WINDOW_MAX / 32], next;
+};
+__device__ __forceinline__ uint32_t list_chunks(const SimView& v, ChunkList& s, uint32_t first, uint32_t window,
+                                                uint32_t nact, int tid) {
+  const int L = tid & 31, wid = tid >> 5;
+  const uint32_t place = first + (uint32_t)tid;
+  uint32_t word = 0, before = 0;
+  if ((uint32_t)wid * 32u < window) {
+    if ((uint32_t)tid < window && place < nact) word = chunk_places(v)[place] >> CHUNK_SHIFT;
+    const unsigned b = __ballot_sync(0xffffffffu, word != 0u);
+    if (L == 0) s.fill[wid] = (uint32_t)__popc(b);
+    before = (uint32_t)__popc(b & ((1u << L) - 1u));
+  }
+  if (tid == 0) s.next = blockDim.x >> 5;
+  __syncthreads();
+  uint32_t chunks = 0;
+#pragma unroll
+  for (int w = 0; w < (int)(WINDOW_MAX / 32); w++)
+    if ((uint32_t)w * 32u < window) {
+      if (w == wid && word) s.chunk[chunks + before] = (uint32_t)tid | (word << 8);
+      chunks += s.fill[w];
+    }
+  __syncthreads();
+  return chunks;
+}
+// the warp's next chunk after c
+__device__ __forceinline__ uint32_t next_chunk(ChunkList& s, uint32_t c, int L) {
+  if (L == 0) c = atomicAdd(&s.next, 1u);
+  return __shfl_sync(0xffffffffu, c, 0);
+}
+
+// Lanes (all four of a group) whose particle lies in the cell of the group
+// that starts at lane ll; ca: the lane's cell coordinate (x, y, z, z).
+__device__ __forceinline__ unsigned same_cell(double ca, int ll, int lane) {
+  const unsigned FULL = 0xffffffffu;
+  const bool other = !(ca == __shfl_sync(FULL, ca, ll + lane));
+  unsigned turn = ~__ballot_sync(FULL, other);
+  turn &= (turn >> 1) & (turn >> 2) & 0x11111111u;  // groups with all three coordinates equal
+  return (turn * 15u) | (15u << ll);
+}
+
+// Bucket L (of 27) of the cells around that group's, CellHash::init's values.
+__device__ __forceinline__ uint32_t turn_bucket(double ca, int ll, int L, uint32_t mask) {
+  const unsigned FULL = 0xffffffffu;
+  const int axis = (L < 9) ? L / 3 : 2;  // lane j < 9: component j, axis j / 3, cell offset j % 3 - 1
+  const double cl = __shfl_sync(FULL, ca, ll + axis);
+  const double K = (axis == 0) ? 92837111.0 : ((axis == 1) ? 689287499.0 : 283923481.0);
+  const int32_t comp = js_toint32(__dmul_rn(__dadd_rn(cl, (double)(L - 3 * axis - 1)), K));
+  const int ka = L / 9, kb = (L - 9 * ka) / 3, kc = L - 9 * ka - 3 * kb;
+  return (uint32_t)(__shfl_sync(FULL, comp, ka) ^ __shfl_sync(FULL, comp, 3 + kb) ^ __shfl_sync(FULL, comp, 6 + kc)) & mask;
+}
+
+// inclusive scan over the warp
+__device__ __forceinline__ uint32_t warp_scan(uint32_t x, int L) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (L >= o) x += y;
+  }
+  return x;
 }
 
 // window <= min(WINDOW_MAX, blockDim), at most 256 threads a block.
 __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __restrict__ P, uint32_t window,
                                           uint32_t vb) {
   extern __shared__ __align__(16) unsigned char s_stage[];
-  __shared__ uint32_t s_chunk[WINDOW_MAX], s_fill[WINDOW_MAX / 32], s_next;
+  __shared__ ChunkList s_list;
   const unsigned FULL = 0xffffffffu;
   const int tid = thread_index();
   const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1), g = L / GLF;
-  // the window's chunks
   const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
   if (first >= nact) return;
-  const uint32_t place = first + (uint32_t)tid;
-  uint32_t word = 0, before = 0;
-  if ((uint32_t)wid * 32u < window) {
-    if ((uint32_t)tid < window && place < nact) word = chunk_places(v)[place] >> CHUNK_SHIFT;
-    const unsigned b = __ballot_sync(FULL, word != 0u);
-    if (L == 0) s_fill[wid] = (uint32_t)__popc(b);
-    before = (uint32_t)__popc(b & ((1u << L) - 1u));
-  }
-  if (tid == 0) s_next = blockDim.x >> 5;
-  __syncthreads();
-  uint32_t chunks = 0;
-#pragma unroll
-  for (int w = 0; w < (int)(WINDOW_MAX / 32); w++)
-    if ((uint32_t)w * 32u < window) {
-      if (w == wid && word) s_chunk[chunks + before] = (uint32_t)tid | (word << 8);
-      chunks += s_fill[w];
-    }
-  __syncthreads();
+  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid);
   real4* __restrict__ sx = reinterpret_cast<real4*>(s_stage + wid * STAGE_WARP);
   const double inv = P->inv_cell;
   const real H = P->fluid_h, H2 = H * H;
@@ -408,8 +450,8 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
 #ifndef UPBD_PARITY_BUILD
   const real invH = 1.0f / H;
 #endif
-  for (uint32_t c = (uint32_t)wid; c < chunks;) {
-    const uint32_t d = s_chunk[c];
+  for (uint32_t c = (uint32_t)wid; c < chunks; c = next_chunk(s_list, c, L)) {
+    const uint32_t d = s_list.chunk[c];
     const bool act = (uint32_t)g < (d >> 8);
     const uint32_t myslot = act ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
     const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
@@ -422,35 +464,23 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
     do {
       // the first remaining particle and those of its cell
       const int ll = __ffs((int)rem) - 1;
-      const bool other = !(ca == __shfl_sync(FULL, ca, ll + lane));
-      unsigned turn = ~__ballot_sync(FULL, other);
-      turn &= (turn >> 1) & (turn >> 2) & 0x11111111u;  // groups with all three coordinates equal
-      turn = ((turn * 15u) | (15u << ll)) & rem;
+      const unsigned turn = same_cell(ca, ll, lane) & rem;
       rem &= ~turn;
-      // its cell's hash components, one per lane (CellHash::init's values), and
-      // the range of bucket L
-      const int axis = (L < 9) ? L / 3 : 2;
-      const double cl = __shfl_sync(FULL, ca, ll + axis);
-      const double K = (axis == 0) ? 92837111.0 : ((axis == 1) ? 689287499.0 : 283923481.0);
-      const int32_t comp = js_toint32(__dmul_rn(__dadd_rn(cl, (double)(L - 3 * axis - 1)), K));
-      const int ka = L / 9, kb = (L - 9 * ka) / 3, kc = L - 9 * ka - 3 * kb;
-      const uint32_t hb = (uint32_t)(__shfl_sync(FULL, comp, ka) ^ __shfl_sync(FULL, comp, 3 + kb) ^
-                                     __shfl_sync(FULL, comp, 6 + kc)) & ((uint32_t)v.T - 1u);
+      const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
       uint32_t s0 = 0, n = 0;
       if (L < 27) {
         s0 = __ldg(&v.start[hb]);
         n = __ldg(&v.fend[hb]) - s0;
       }
-      uint32_t end = n;  // inclusive scan in cell order
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, end, o);
-        if (L >= o) end += y;
-      }
+      const uint32_t end = warp_scan(n, L);  // in cell order
       const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
       for (uint32_t q0 = 0; q0 < total; q0 += STAGE) {
-        if (total <= STAGE) stage_rows<false>(v, sx, L, s0, off, end, 0u);
-        else stage_rows<true>(v, sx, L, s0, off, end, q0);
+        auto copy = [&](uint32_t k, uint32_t e) {
+          if (UPBD_IDX_OK(v, e, NS)) copy_row_async(&sx[k], &v.spos[e]);
+          else sx[k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never listed (reported)
+        };
+        if (total <= STAGE) stage_rows<STAGE, false>(L, s0, off, end, 0u, copy);
+        else stage_rows<STAGE, true>(L, s0, off, end, q0, copy);
         copy_rows_wait();
         __syncwarp();
         const uint32_t len = min(total - q0, STAGE);
@@ -525,8 +555,6 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
       v.density[v.entries[myslot]] = dd;
       v.sdens[myslot] = dd;
     }
-    if (L == 0) c = atomicAdd(&s_next, 1u);
-    c = __shfl_sync(FULL, c, 0);
   }
 }
 
@@ -1357,8 +1385,6 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
   }
   if (stage < 2) {
     v.pos[i] = p;
-    if (!iSolid) record_move(v, P, i, sl, o, p);
-    v.spos[sl] = p;
     return;
   }
   // bounds
@@ -1391,13 +1417,12 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
   }
   p.x = px; p.y = py; p.z = pz;
   v.pos[i] = p;
-  if (!iSolid) record_move(v, P, i, sl, o, p);
-  v.spos[sl] = p;
   if (stage < 3) return;
+  if (!iSolid) record_move(v, P, i, sl, o, p);
   if (culled) {
     // xsph still reads a culled neighbour's velocity (src/gpu/wgsl.js:761
     // does not test its flag): its slot keeps the unchanged velocity
-    v.svel[sl] = ov;
+    store_row_pair(&v.pvrow[2 * (size_t)sl], make_real4(p.x, p.y, p.z, slot_pack(real(0), sl)), ov);
     return;
   }
   // velocityUpdate
@@ -1415,7 +1440,7 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
   if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz)) atomicOr(&v.scratch[SCR_HEALTH], 1u);
   const real4 nv = make_real4(vx, vy, vz, ov.w);
   v.vel[i] = nv;
-  v.svel[sl] = nv;
+  if (!iSolid) store_row_pair(&v.pvrow[2 * (size_t)sl], make_real4(p.x, p.y, p.z, slot_pack(real(0), sl)), nv);  // xsph's neighbours
 }
 
 // solidVisc, src/gpu/wgsl.js:717-735
@@ -1454,143 +1479,160 @@ __device__ __forceinline__ void b_solid_visc_apply(const SimView& v, uint32_t vb
   v.vel[i] = make_real4(d.x, d.y, d.z, w);
 }
 
-// xsph, src/gpu/wgsl.js:745-771 (slot-ordered groups, as b_density). The
-// grid still holds the particles bounds culled this substep: they are
-// neighbours (the reference does not test their flag) but have no pass of
-// their own. Neighbour velocities come from the slot copies (svel), so with
-// APPLY the blended velocity goes straight to vel[i] (xsphApply's result,
-// src/gpu/wgsl.js:773-778) and the copy pass is not needed; without it the
-// result waits in delta, where the reference's xsph pass leaves it.
-// A group whose particle passes the list test (XSKIN) reads its lanes'
-// density-pass lists instead of walking the 27 buckets: each lane's listed
-// candidates are a subsequence, in order, of its walk share that holds every
-// candidate within H now, so both forms add the same terms in the same order.
-// list entries whose loads are in flight together: 2 in the list-only
-// launch (48 registers: more warps hide the latency), 4 where one launch also
-// walks
-constexpr int XCH_LIST = 2, XCH_BOTH = 4;
-constexpr int XWU = 4;  // candidates in flight per step of a walk beside the lists
-// ROLE 0 runs both forms; ROLE 1 only the groups that read lists, ROLE 2
-// only those that walk (two launches that run side by side, each with the
-// registers its own form needs).
-template <bool APPLY, int ROLE = 0>
-__device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const uint32_t t = UPBD_VTID;
-  const int lane = threadIdx.x & (GLF - 1);
-  const uint32_t NS = (uint32_t)v.N, myslot = t / GLF, eld = min(myslot, NS - 1u);
-  const uint32_t nact = __ldg(&v.start[v.T]), i = v.entries[eld];
-  real4 pi = v.spos[eld];
-  float sm = v.smove[eld];
-  uint32_t cnt = v.ncount[(size_t)lane * NS + eld];
-  issued(nact);
-  issued(i);
-  issued(pi);
-  issued(sm);
-  issued(cnt);
-  const bool fluid = myslot < nact && i >= (uint32_t)v.S;
-  const bool act = fluid && (v.flags[i] & F_ACTIVE);
-  if (!__any_sync(0xffffffffu, act)) return;
-  real sx = 0.f, sy = 0.f, sz = 0.f, m = 0.f;
-  if (!act) {
-    pi = make_real4(0.f, 0.f, 0.f, 0.f);
-    sm = 0.f;
-    cnt = 0u;
-  }
+// xsph, src/gpu/wgsl.js:745-771, over the density pass's chunks. The grid still
+// holds the particles bounds culled this substep: they are neighbours (the
+// reference does not test their flag) but have no pass of their own. Neighbour
+// rows (position, velocity) are slot copies, so with APPLY the blended velocity
+// goes straight to vel[i] (xsphApply's result, src/gpu/wgsl.js:773-778) and the
+// copy pass is not needed; without it the result waits in delta, where the
+// reference's xsph pass leaves it.
+// A particle that passes the list test (XSKIN) has its lanes read their
+// density-pass lists: each lane's listed candidates are a subsequence, in order,
+// of its walk share that holds every candidate within H now. For the others the
+// warp stages the candidates' positions and velocities around their present
+// cell, as the density pass does, and the lanes walk the bits of those within H.
+// Either way a lane adds the same terms in the same order (a candidate out of
+// range would add +0 to a sum that starts at +0).
+// Bound by latency (list entry -> row) where the fluid has settled, by the
+// staged walks where it moves. With each group of lanes walking its own buckets
+// in a launch of its own beside the list readers, the default scene's settled
+// pool took 31.5 us (both forms in one launch, B200, event-timed), the large
+// scene's splash 115, a batch of 48 scenes 283; now 23.0, 88 and 228. Position and
+// velocity come as one 32-byte row: with two 16-byte rows 25.7, 103 us.
+constexpr uint32_t XROWS = STAGE / 2;  // candidates staged a round: positions and velocities in the same bytes
+constexpr int XCH = 4;                 // list entries whose loads are in flight together
+template <bool APPLY>
+__device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __restrict__ P, uint32_t window, uint32_t vb) {
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  __shared__ ChunkList s_list;
+  const unsigned FULL = 0xffffffffu;
+  const int tid = thread_index();
+  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1), g = L / GLF;
+  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  if (first >= nact) return;
+  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid);
+  real4* __restrict__ sx = reinterpret_cast<real4*>(s_stage + wid * STAGE_WARP);
+  real4* __restrict__ sv = sx + XROWS;
+  const double inv = P->inv_cell;
   const real H = P->fluid_h, H2 = H * H;
-  const real4* __restrict__ spos = v.spos;
-  const real4* __restrict__ svel = v.svel;
-  // position and velocity of every candidate are loaded together, before the
-  // range test, and out-of-range ones add zero (the sums start at +0, so +0
-  // leaves them unchanged): no load waits on the test
-  struct PV {
-    real4 p, v;
-  };
-  auto load = [&](uint32_t e) { return PV{spos[e], svel[e]}; };
-  auto use = [&](uint32_t e, const PV& c) {
-    const real ex = c.p.x - pi.x, ey = c.p.y - pi.y, ez = c.p.z - pi.z;
-    const bool in = (e != myslot) && (dot3(ex, ey, ez, ex, ey, ez) < H2);
-    sx = sx + (in ? c.v.x : 0.f); sy = sy + (in ? c.v.y : 0.f); sz = sz + (in ? c.v.z : 0.f);
-    m = m + (in ? 1.0f : 0.f);
-  };
-  // the list test: the particle kept its cell (smove finite), it and every
-  // particle of its 27 buckets moved within the allowance, and no lane's list
-  // overflowed. The scene's largest recorded movement bounds every bucket's,
-  // so when it passes the buckets are not looked at (nor hashed, unless the
-  // group walks).
+  const real4* __restrict__ rows = v.pvrow;
+  const uint32_t NS = (uint32_t)v.N;
   const real allow = xsph_allowance(P), rec = XMOVE_REC * allow;
-  uint32_t over = (cnt > NL) ? 1u : 0u;
+  const real scene = r_fmax(rec, (real)__uint_as_float(v.scratch[SCR_XMOVE]));
+  for (uint32_t c = (uint32_t)wid; c < chunks; c = next_chunk(s_list, c, L)) {
+    const uint32_t d = s_list.chunk[c];
+    const bool mem = (uint32_t)g < (d >> 8);
+    const uint32_t myslot = mem ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
+    const uint32_t i = v.entries[myslot];
+    const real4 pi = rows[2 * (size_t)myslot];
+    const real sm = v.smove[myslot];
+    uint32_t cnt = v.ncount[(size_t)lane * NS + myslot];
+    const bool act = mem && (v.flags[i] & F_ACTIVE);
+    // the list test: the particle kept its cell (smove finite), it and every
+    // particle of its 27 buckets moved within the allowance, and no lane's list
+    // overflowed. The scene's largest recorded movement bounds every bucket's,
+    // so when it passes the buckets are not looked at.
+    const unsigned full = __ballot_sync(FULL, cnt > NL);
+    const bool over = (full >> (L & ~(GLF - 1)) & ((1u << GLF) - 1u)) != 0u;
+    bool listed = act && !over && sm + scene <= allow;
+    real sx_ = 0.f, sy_ = 0.f, sz_ = 0.f, m = 0.f;
+    unsigned rem = __ballot_sync(FULL, act && !listed);
+    if (rem) {
+      const double ca = floor(__dmul_rn((double)(lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z)), inv));
+      do {
+        const int ll = __ffs((int)rem) - 1;
+        const unsigned turn = same_cell(ca, ll, lane) & rem;
+        rem &= ~turn;
+        const bool mine_turn = (turn >> L & 1u) != 0u;
+        const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
+        const uint32_t bm = __reduce_max_sync(FULL, (L < 27) ? v.bmove[hb] : 0u);  // a finite distance or +inf
+        if (mine_turn) listed = !over && sm + r_fmax(rec, (real)__uint_as_float(bm)) <= allow;
+        const bool walks = mine_turn && !listed;
+        if (!__any_sync(FULL, walks)) continue;
+        uint32_t s0 = 0, n = 0;
+        if (L < 27) {
+          s0 = __ldg(&v.start[hb]);
+          n = __ldg(&v.fend[hb]) - s0;
+        }
+        const uint32_t end = warp_scan(n, L);  // in cell order
+        const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
+        for (uint32_t q0 = 0; q0 < total; q0 += XROWS) {
+          auto copy = [&](uint32_t k, uint32_t e) {
+            if (UPBD_IDX_OK(v, e, NS)) {
+              copy_row_async(&sx[k], &rows[2 * (size_t)e]);
+              copy_row_async(&sv[k], &rows[2 * (size_t)e + 1]);
+            } else {
+              sx[k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never in range (reported)
+            }
+          };
+          if (total <= XROWS) stage_rows<XROWS, false>(L, s0, off, end, 0u, copy);
+          else stage_rows<XROWS, true>(L, s0, off, end, q0, copy);
+          copy_rows_wait();
+          __syncwarp();
+          const uint32_t len = min(total - q0, XROWS);
+          const uint32_t own = walks ? (len + (GLF - 1) - lane) / GLF : 0u;  // this lane's share, at most 32
+          const uint32_t steps = (len + (GLF - 1)) / GLF;
+          uint32_t bits = 0;  // within H, the first candidate's bit on top
+          const real4* __restrict__ r4 = sx + lane;
+          for (uint32_t u = 0; u < steps; u += 4, r4 += 4 * GLF) {  // reads past the share stay in the warp's rows
 #pragma unroll
-  for (int d = 1; d < GLF; d <<= 1) over |= __shfl_xor_sync(0xffffffffu, over, d);
-  const bool quick = act && over == 0u && sm + r_fmax(rec, (real)__uint_as_float(v.scratch[SCR_XMOVE])) <= allow;
-  const bool need = act && !quick;  // its buckets' movement, or the walk
-  CellHash ch;
-  bool listed = quick;
-  if (__any_sync(0xffffffffu, need)) {
-    group_cell_hash<GLF>(pi.x, pi.y, pi.z, P->inv_cell, ch);
-    uint32_t bm = 0;
-    if (need) {
-      const uint32_t mask = (uint32_t)v.T - 1u;
+            for (int k = 0; k < 4; k++) {
+              const real4 pj = r4[k * GLF];
+              const bool in = slot_unpack(pj.w) != myslot && dist2(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z) < H2;
+              bits = (bits << 1) | (in ? 1u : 0u);
+            }
+          }
+          bits <<= (32u - ((steps + 3u) & ~3u)) & 31u;
+          if (own < 32u) bits &= ~(0xffffffffu >> own);
+          while (bits) {
+            const int k = __clz((int)bits);
+            bits &= ~(0x80000000u >> k);
+            const real4 w = sv[lane + k * GLF];
+            sx_ = sx_ + w.x; sy_ = sy_ + w.y; sz_ = sz_ + w.z;
+            m = m + 1.0f;
+          }
+          __syncwarp();  // the next round rewrites the rows
+        }
+      } while (rem);
+    }
+    if (listed) {
+      const uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
+      for (uint32_t k = 0; k < cnt; k += XCH) {
+        uint32_t e[XCH];
+        real4 p[XCH], w[XCH];
 #pragma unroll
-      for (int r = 0; r < (27 + GLF - 1) / GLF; r++) {
-        const int k = lane + GLF * r;
-        if (k < 27) bm = max(bm, v.bmove[ch.bucket_k(k, mask)]);
+        for (int q = 0; q < XCH; q++) {
+          e[q] = (k + q < cnt) ? (__ldg(&nbr[(k + q) * NS]) & ~NBR_IN) : myslot;
+          if (!UPBD_IDX_OK(v, e[q], NS)) e[q] = myslot;  // out of range: the own slot (skipped, reported)
+        }
+#pragma unroll
+        for (int q = 0; q < XCH; q++) load_row_pair(&rows[2 * (size_t)e[q]], p[q], w[q]);
+#pragma unroll
+        for (int q = 0; q < XCH; q++) {
+          const bool in = e[q] != myslot && dist2(p[q].x - pi.x, p[q].y - pi.y, p[q].z - pi.z) < H2;
+          sx_ = sx_ + (in ? w[q].x : 0.f); sy_ = sy_ + (in ? w[q].y : 0.f); sz_ = sz_ + (in ? w[q].z : 0.f);
+          m = m + (in ? 1.0f : 0.f);
+        }
       }
     }
-#pragma unroll
-    for (int d = 1; d < GLF; d <<= 1) bm = max(bm, __shfl_xor_sync(0xffffffffu, bm, d));
-    // bm holds a finite distance or +inf
-    listed = quick || (need && over == 0u && sm + r_fmax(rec, (real)__uint_as_float(bm)) <= allow);
-  }
-  const bool walks = act && !listed;
-  const bool mine = (ROLE == 0) ? act : ((ROLE == 1) ? listed : walks);
-  if (ROLE != 0 && !__any_sync(0xffffffffu, mine)) return;
-  // with both forms in one launch the groups that walk keep XWU candidates'
-  // loads in flight: while most groups read lists, the few walks are the
-  // kernel's tail
-  if (ROLE == 0 && __any_sync(0xffffffffu, walks)) lane_strided<0, GLF, XWU>(v, ch, lane, walks, load, use);
-  // the walking launch: where one or two groups of a warp walk, the warp's
-  // lanes load their candidates for them; where more do, each walks its own
-  // (staged walks take turns, so they cost more than they save there)
-  if (ROLE == 2) {
-    const unsigned wg = __ballot_sync(0xffffffffu, walks && lane == 0);
-    if (wg != 0u && __popc(wg) <= 2) lane_staged<0, GLF>(v, ch, lane, walks, load, use);
-    else if (wg != 0u) lane_strided<0, GLF, 1>(v, ch, lane, walks, load, use);
-  }
-  if (ROLE != 2 && listed) {
-    constexpr int XCH = (ROLE == 1) ? XCH_LIST : XCH_BOTH;
-    const uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
-    for (uint32_t c = 0; c < cnt; c += XCH) {  // XCH entries' loads in flight
-      uint32_t e[XCH];
-      PV pv[XCH];
-#pragma unroll
-      for (int w = 0; w < XCH; w++) {
-        e[w] = (c + w < cnt) ? (__ldg(&nbr[(c + w) * NS]) & ~NBR_IN) : myslot;
-        if (!UPBD_IDX_OK(v, e[w], NS)) e[w] = myslot;  // out of range: the own slot (skipped, reported)
+    sx_ = lane_sum<GLF>(sx_);
+    sy_ = lane_sum<GLF>(sy_);
+    sz_ = lane_sum<GLF>(sz_);
+    m = lane_sum<GLF>(m);
+    if (act && lane == 0) {
+      const real4 vi = v.vel[i];
+      real vx = vi.x, vy = vi.y, vz = vi.z;
+      if (m > 0.f) {
+        const real mu = P->viscosity;
+        vx = vx + mu * (sx_ / m - vx);
+        vy = vy + mu * (sy_ / m - vy);
+        vz = vz + mu * (sz_ / m - vz);
       }
-#pragma unroll
-      for (int w = 0; w < XCH; w++) pv[w] = load(e[w]);
-#pragma unroll
-      for (int w = 0; w < XCH; w++)
-        if (c + w < cnt) use(e[w], pv[w]);
+      if (APPLY)
+        v.vel[i] = make_real4(vx, vy, vz, 0.f);
+      else
+        v.delta[i] = make_real4(vx, vy, vz, m);
     }
-  }
-  sx = lane_sum<GLF>(sx);
-  sy = lane_sum<GLF>(sy);
-  sz = lane_sum<GLF>(sz);
-  m = lane_sum<GLF>(m);
-  if (mine && lane == 0) {
-    const real4 vi = v.vel[i];
-    real vx = vi.x, vy = vi.y, vz = vi.z;
-    if (m > 0.f) {
-      const real mu = P->viscosity;
-      vx = vx + mu * (sx / m - vx);
-      vy = vy + mu * (sy / m - vy);
-      vz = vz + mu * (sz / m - vz);
-    }
-    if (APPLY)
-      v.vel[i] = make_real4(vx, vy, vz, 0.f);
-    else
-      v.delta[i] = make_real4(vx, vy, vz, m);
   }
 }
 

@@ -189,7 +189,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.mark = cv.take<uint32_t>(v.N);
   L.spos = cv.take<real4>(v.N);
   L.sdens = cv.take<real2>(v.N);
-  L.svel = cv.take<real4>(v.N);
+  L.pvrow = cv.take<real4>(2 * (size_t)v.N);
   L.slot = cv.take<uint32_t>(v.N);
   L.fend = cv.take<uint32_t>(v.T);
   L.nbr = cv.take<uint32_t>(std::max<size_t>((size_t)v.N * GLF * NL, 1));
@@ -201,7 +201,6 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.trec = cv.take<uint4>(tets ? std::max<size_t>(4 * (size_t)v.NT, 1) : 1);
   L.tscl = cv.take<float>(tets ? std::max<size_t>(4 * (size_t)v.NT, 1) : 1);
   L.sbuf = cv.take<real4>(2 * (size_t)std::max(v.S, 1));
-  L.sfp = cv.take<real4>(v.N);
   L.smove = cv.take<float>(v.N);
   L.bmove = cv.take<uint32_t>(v.T);
   L.scr = cv.take<uint32_t>(SCR_WORDS);
@@ -238,7 +237,7 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.mark = (uint32_t*)(base + L.mark);
   v.spos = (real4*)(base + L.spos);
   v.sdens = (real2*)(base + L.sdens);
-  v.svel = (real4*)(base + L.svel);
+  v.pvrow = (real4*)(base + L.pvrow);
   v.slot = (uint32_t*)(base + L.slot);
   v.fend = (uint32_t*)(base + L.fend);
   v.nbr = (uint32_t*)(base + L.nbr);
@@ -250,7 +249,7 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.ccount = (uint32_t*)(base + L.ccount);
   v.clist = (uint32_t*)(base + L.clist);
   v.sbuf = (real4*)(base + L.sbuf);
-  v.sfp = (real4*)(base + L.sfp);
+  v.sfp = v.pvrow + v.N;
   v.smove = (float*)(base + L.smove);
   v.bmove = (uint32_t*)(base + L.bmove);
   v.scratch = (uint32_t*)(base + L.scr);
