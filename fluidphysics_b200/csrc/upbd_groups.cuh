@@ -133,15 +133,25 @@ __global__ void __launch_bounds__(256) k_groups_tree(int S, GroupScratch g) {
   g.tree[v] = x;
 }
 
-// Alive constraints between different trees.
+// Alive constraints between different trees, the first of each pair of trees
+// in a warp's 32 (a later one of the same pair finds them joined).
 __global__ void __launch_bounds__(256) k_groups_cross(const uint4* __restrict__ cons, int C, int S, GroupScratch g) {
+  const unsigned FULL = 0xffffffffu;
   const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  bool cross = false;
+  unsigned long long pair = 0ull;  // no pair: a tree with itself
   if (c < C) {
     const uint4 k = cons[c];
-    cross = k.w != 0u && k.x < (uint32_t)S && k.y < (uint32_t)S && g.tree[k.x] != g.tree[k.y];
+    if (k.w != 0u && k.x < (uint32_t)S && k.y < (uint32_t)S) {
+      const uint32_t ta = (uint32_t)g.tree[k.x], tb = (uint32_t)g.tree[k.y];
+      if (ta != tb) pair = ((unsigned long long)max(ta, tb) << 32) | min(ta, tb);
+    }
   }
-  const unsigned w = __ballot_sync(0xffffffffu, cross);
+  bool cross = pair != 0ull;
+  if (__any_sync(FULL, cross)) {
+    const unsigned same = __match_any_sync(FULL, pair);
+    cross = cross && (int)(threadIdx.x & 31) == __ffs((int)same) - 1;
+  }
+  const unsigned w = __ballot_sync(FULL, cross);
   if ((threadIdx.x & 31) == 0 && c < C) g.bits[c >> 5] = w;
 }
 
