@@ -133,7 +133,9 @@ struct SimView {
   // a candidate's data with one load at its slot instead of entries -> pos.
   // Every pass that moves a particle also writes its slot's copy.
   real4* spos;         // position + inverse mass (fluid: + slot)
-  real2* sdens;        // (rho, rho_near) of the density pass
+  // Row pairs of the density pass (2 N rows, fluid): its position + slot at 2 e
+  // and (rho, rho_near, mass, 0) at 2 e + 1, for the displacement.
+  real4* drow;
   // Row pairs (2 N rows): position + slot and velocity of the fluid particle at
   // slot e after the bounds pass, at 2 e and 2 e + 1, for xsph. Until that
   // pass the memory serves earlier ones (bucket_pairs, slot_mass, sfp).
@@ -245,7 +247,7 @@ __device__ __forceinline__ bool idx_ok(uint32_t* scratch, uint64_t idx, uint64_t
 // cell boundaries in all.
 constexpr int GL = 8;
 constexpr int GLF = 4;
-constexpr uint32_t NL = 32;  // density-pass neighbour-list entries kept per fluid lane (GLF * NL per particle)
+constexpr uint32_t NL = 28;  // density-pass neighbour-list entries kept per fluid lane (GLF * NL per particle)
 constexpr int DL = 2;        // threads per particle in the displacement pass
 constexpr uint32_t CHUNK = 32 / GLF;  // fluid particles of one cell that a warp takes in the density pass
 constexpr int CHUNK_SHIFT = 28;       // chunk place: slot, above it the size of the chunk that starts there
@@ -462,12 +464,12 @@ __device__ __forceinline__ void store_row_pair(real4* dst, const real4& a, const
 // Words of the grid build and the density pass that live in arrays the bounds
 // pass writes: smove holds the cell keys by particle (count -> rank fix-up),
 // pvrow the bucket members with their keys (scatter -> rank fix-up), behind them
-// the fluid's masses by slot (rank fix-up -> displacement). The chunk places
+// the fluid's masses by slot (rank fix-up -> density). The chunk places
 // (rank fix-up -> density, xsph) are the array the stateless grid build
 // scatters into.
 __device__ __forceinline__ uint32_t* cell_keys(const SimView& v) { return reinterpret_cast<uint32_t*>(v.smove); }
-__device__ __forceinline__ float* slot_mass(const SimView& v) { return reinterpret_cast<float*>(v.pvrow) + 2 * (size_t)v.N; }
 __device__ __forceinline__ uint2* bucket_pairs(const SimView& v) { return reinterpret_cast<uint2*>(v.pvrow); }
+__device__ __forceinline__ real* slot_mass(const SimView& v) { return reinterpret_cast<real*>(bucket_pairs(v) + v.N); }
 __device__ __forceinline__ uint32_t* chunk_places(const SimView& v) { return v.tmp; }
 
 // std::max / std::min / clamp with the operand order of the oracle (so -0.0

@@ -262,7 +262,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   if (i >= v.S) {
     const uint32_t n = (rank_in % CHUNK == 0u) ? min(CHUNK, mates - rank_in) : 0u;
     chunk_places(v)[s + before + rank_in] = slot | (n << CHUNK_SHIFT);
-    slot_mass(v)[slot] = (float)p.w;
+    slot_mass(v)[slot] = p.w;
     p.w = slot_pack(real(0), slot);
   } else {
     chunk_places(v)[slot] = 0u;  // solids follow the fluid: no chunk starts there
@@ -455,6 +455,7 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
     const bool act = (uint32_t)g < (d >> 8);
     const uint32_t myslot = act ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
     const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
+    const real mass = slot_mass(v)[myslot];
     // lane l's c-th listed candidate goes to row l*NL + c, column myslot
     uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
     uint32_t cnt = 0;
@@ -551,9 +552,8 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
     rho = lane_sum<GLF>(rho);
     rhoNear = lane_sum<GLF>(rhoNear);
     if (act && lane == 0) {
-      const real2 dd = make_real2(rho, rhoNear);
-      v.density[v.entries[myslot]] = dd;
-      v.sdens[myslot] = dd;
+      v.density[v.entries[myslot]] = make_real2(rho, rhoNear);
+      store_row_pair(&v.drow[2 * (size_t)myslot], pi, make_real4(rho, rhoNear, mass, 0.f));
     }
   }
 }
@@ -591,20 +591,17 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
   constexpr int LPT = GLF / DL;  // lanes' lists per thread
   const uint32_t e0 = UPBD_VTID / DL;
   const int h = (int)(threadIdx.x & (DL - 1));
-  const real4* __restrict__ spos = v.spos;
-  const real2* __restrict__ sdens = v.sdens;
+  const real4* __restrict__ rows = v.drow;
   const uint32_t NS = (uint32_t)v.N, eld = min(e0, NS - 1u);
   const uint32_t nact = __ldg(&v.start[v.T]);
   const uint32_t i = v.entries[eld];
-  const real4 pi = spos[eld];
-  const real2 di = sdens[eld];
+  real4 pi, di;
+  load_row_pair(&rows[2 * (size_t)eld], pi, di);
   uint32_t cnt[LPT];
 #pragma unroll
   for (int u = 0; u < LPT; u++) cnt[u] = v.ncount[(size_t)(h * LPT + u) * NS + eld];
   issued(nact);
   issued(i);
-  issued(pi);
-  issued(di);
 #pragma unroll
   for (int u = 0; u < LPT; u++) issued(cnt[u]);
   const bool act = e0 < nact && i >= (uint32_t)v.S;
@@ -623,7 +620,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
 #ifndef UPBD_PARITY_BUILD
     const real invH = 1.0f / H;
 #endif
-    auto pair = [&](const real4& pj, const real2& dj) {
+    auto pair = [&](const real4& pj, const real4& dj) {
       const real ex = pj.x - pi.x, ey = pj.y - pi.y, ez = pj.z - pi.z;
       const real d2 = dot3(ex, ey, ez, ex, ey, ez);
       if (d2 >= H2 || d2 < 1e-12f) return;
@@ -658,8 +655,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
         // in flight together (a lane list holds ~4)
         for (uint32_t c = 0; c < cnt[u]; c += 4) {
           uint32_t e[4];
-          real4 pj[4];
-          real2 dj[4];
+          real4 pj[4], dj[4];
 #pragma unroll
           for (int w = 0; w < 4; w++) {
             // entries beyond H (listed for xsph) and past the count become the
@@ -669,10 +665,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
             if (!UPBD_IDX_OK(v, e[w], NS)) e[w] = e0;  // out of range: the own slot (skipped, reported)
           }
 #pragma unroll
-          for (int w = 0; w < 4; w++) {
-            pj[w] = spos[e[w]];
-            dj[w] = sdens[e[w]];
-          }
+          for (int w = 0; w < 4; w++) load_row_pair(&rows[2 * (size_t)e[w]], pj[w], dj[w]);
 #pragma unroll
           for (int w = 0; w < 4; w++)
             if (c + w < cnt[u]) pair(pj[w], dj[w]);
@@ -689,7 +682,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
           const uint32_t hb = ch.bucket_k(kk, mask);
           const uint32_t s0 = __ldg(&v.start[hb]), s1 = __ldg(&v.fend[hb]);
           for (uint32_t e = s0; e < s1; e++, c++)
-            if ((c & (GLF - 1)) == (uint32_t)l && e != e0) pair(spos[e], sdens[e]);
+            if ((c & (GLF - 1)) == (uint32_t)l && e != e0) pair(rows[2 * (size_t)e], rows[2 * (size_t)e + 1]);
         }
       }
     }
@@ -701,11 +694,6 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
     sz = sz + __shfl_xor_sync(0xffffffffu, sz, d);
   }
   if (!act || h != 0) return;
-#ifdef UPBD_FP64_BUILD
-  const real w = v.pos[i].w;
-#else
-  const real w = slot_mass(v)[e0];
-#endif
   const real maxTotal = 0.35f * H;
   const real s2 = dot3(sx, sy, sz, sx, sy, sz);
   if (s2 > maxTotal * maxTotal) {
@@ -713,7 +701,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
     sx = sx * f; sy = sy * f; sz = sz * f;
   }
   if (APPLY) {  // pi is pos[i] (but for its w): the grid build copied it and nothing moved it since
-    const real4 p = make_real4(pi.x + sx, pi.y + sy, pi.z + sz, w);
+    const real4 p = make_real4(pi.x + sx, pi.y + sy, pi.z + sz, di.z);
     v.pos[i] = p;
     v.sfp[e0] = p;
     mark_if_cell_changed(v, P, (int)i, pi, p);

@@ -188,7 +188,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.tadj = cv.take<uint32_t>(hs.tet_adj.size());
   L.mark = cv.take<uint32_t>(v.N);
   L.spos = cv.take<real4>(v.N);
-  L.sdens = cv.take<real2>(v.N);
+  L.drow = cv.take<real4>(2 * (size_t)v.N);
   L.pvrow = cv.take<real4>(2 * (size_t)v.N);
   L.slot = cv.take<uint32_t>(v.N);
   L.fend = cv.take<uint32_t>(v.T);
@@ -236,7 +236,7 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.tet_adj = (const uint32_t*)(base + L.tadj);
   v.mark = (uint32_t*)(base + L.mark);
   v.spos = (real4*)(base + L.spos);
-  v.sdens = (real2*)(base + L.sdens);
+  v.drow = (real4*)(base + L.drow);
   v.pvrow = (real4*)(base + L.pvrow);
   v.slot = (uint32_t*)(base + L.slot);
   v.fend = (uint32_t*)(base + L.fend);
