@@ -24,7 +24,7 @@ namespace upbd {
 constexpr uint32_t F_ACTIVE = 1u;
 constexpr uint32_t F_GRABBED = 2u;
 constexpr uint32_t C_K = 40u;           // solid contact cache width, src/gpu/wgsl.js:25
-constexpr int SCAN_THREADS = 256;       // 8 counts per thread (SCAN_TILE / 8)
+constexpr int SCAN_THREADS = 512;       // 4 counts per thread (SCAN_TILE / 4)
 
 // scratch words (device)
 constexpr int SCR_PICK = 0;        // pick blocks finished (last-block pattern)
