@@ -75,6 +75,10 @@ struct upbd_sim {
   // second stream of the substep: the solid solve's first iterations run
   // there beside the grid build and the fluid gathers (fork / join events)
   cudaStream_t side = nullptr;
+  // frames are captured on this stream, of higher priority than the side
+  // stream; the graph keeps each kernel's priority, so that the main chain's
+  // blocks are placed before the solve's when both become ready at once
+  cudaStream_t cap = nullptr;
   cudaEvent_t fork_ev = nullptr, grid_ev = nullptr, join_ev = nullptr;
   // asynchronous readback: device staging copy, copy stream, events
   void* rb_stage = nullptr;  // float4 pos[N] then uint32 flags[N]
@@ -202,7 +206,9 @@ int launch_substep(upbd_sim* s, int last) {
   const bool overlap = fold && !s->prof_on && s->side;
   const int early = scc ? per - 1 : phases - 1;  // phases that need no grid
   const int solid_pad = ((v.S * GL + 31) / 32) * 32;  // lane threads of the solve, whole warps
-  const unsigned blk_gl = blocks_for((long long)v.S * GL), blk_gt = blocks_for((long long)v.S * GT);
+  const unsigned blk_gl = blocks_for((long long)v.S * GL), blk_gt = blocks_for((long long)v.S * GT),
+                 blk_32 = blocks_for((long long)v.S * 32);
+  const bool wide_tets = blk_32 <= (unsigned)s->num_sms;  // b_solve_tets: a block an SM at most
   auto solid_phase = [&](cudaStream_t ss, int q, bool mark) {
     const int kind = q % per;
     const bool lastq = q == phases - 1;
@@ -211,8 +217,13 @@ int launch_substep(upbd_sim* s, int last) {
       else if (mark) PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_LAST><<<blocks_for(solid_pad), 256, 0, ss>>>(v, P, solid_pad, q));
       else PROF(s, K_SOLID_SOLVE, k_solid_solve<false, SOLVE_FINAL><<<blocks_for(solid_pad), 256, 0, ss>>>(v, P, solid_pad, q));
     } else if (tets && kind == 1) {
-      if (!lastq) PROF(s, K_SOLVE_TETS, k_solve_tets<false><<<blk_gt, 256, 0, ss>>>(v, P, q));
-      else PROF(s, K_SOLVE_TETS, k_solve_tets<true><<<blk_gt, 256, 0, ss>>>(v, P, q));
+      if (wide_tets) {
+        if (!lastq) PROF(s, K_SOLVE_TETS, k_solve_tets<false, 32><<<blk_32, 256, 0, ss>>>(v, P, q));
+        else PROF(s, K_SOLVE_TETS, k_solve_tets<true, 32><<<blk_32, 256, 0, ss>>>(v, P, q));
+      } else {
+        if (!lastq) PROF(s, K_SOLVE_TETS, k_solve_tets<false, GT><<<blk_gt, 256, 0, ss>>>(v, P, q));
+        else PROF(s, K_SOLVE_TETS, k_solve_tets<true, GT><<<blk_gt, 256, 0, ss>>>(v, P, q));
+      }
     } else {
       if (!lastq) PROF(s, K_SOLID_CONTACTS, k_solid_contacts<false><<<blk_gl, 256, 0, ss>>>(v, P, q));
       else PROF(s, K_SOLID_CONTACTS, k_solid_contacts<true><<<blk_gl, 256, 0, ss>>>(v, P, q));
@@ -402,15 +413,18 @@ int enqueue_frame(upbd_sim* s, double h, int nsub, bool profile = false) {
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
       cudaGraph_t g;
-      UPBD_CK(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+      const cudaStream_t user = s->stream;
+      UPBD_CK(s, cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal));
       const uint64_t before = s->launches;
+      s->stream = s->cap;
       rc = launch_frame(s, nsub, emit_blocks, cut);
-      cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
+      s->stream = user;
+      cudaError_t ce = cudaStreamEndCapture(s->cap, &g);
       s->launches = before;
       if (rc) return rc;
       if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
       cudaGraphExec_t ge;
-      ce = cudaGraphInstantiate(&ge, g, 0);
+      ce = cudaGraphInstantiate(&ge, g, cudaGraphInstantiateFlagUseNodePriority);
       const uint64_t nk = count_graph_kernels(g);
       cudaGraphDestroy(g);
       if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ce));
@@ -513,7 +527,10 @@ int upbd_create(const upbd_scene_desc* desc, const upbd_params* params, upbd_sim
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
     return cleanup_fail(UPBD_ERR_CUDA, "stream creation failed");
   s->own_stream = true;
-  if (cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess ||
+  int least = 0, greatest = 0;
+  if (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, least) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&s->cap, cudaStreamNonBlocking, greatest) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->grid_ev, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->join_ev, cudaEventDisableTiming) != cudaSuccess)
@@ -569,6 +586,7 @@ int upbd_destroy(upbd_sim* s) {
     cudaStreamSynchronize(s->side);
     cudaStreamDestroy(s->side);
   }
+  if (s->cap) cudaStreamDestroy(s->cap);
   if (s->rb_stream) {
     cudaStreamSynchronize(s->rb_stream);
     cudaStreamDestroy(s->rb_stream);

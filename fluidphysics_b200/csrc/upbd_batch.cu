@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) kb_apply_fluid(BatchArgs a) {
 template <bool APPLY_FLUID, int OUT>
 __global__ void __launch_bounds__(256, 6) kb_solid_solve(BatchArgs a, int q) {
   batch_loop<APPLY_FLUID ? D_SOLVE0 : D_SOLVE, false, true>(
-      a, UPBD_BODY { b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad_of(v.S), q, vb); });
+      a, UPBD_BODY { b_solid_solve<APPLY_FLUID, OUT, 2>(v, P, solid_pad_of(v.S), q, vb); });
 }
 __global__ void __launch_bounds__(256) kb_apply_solid(BatchArgs a) {
   batch_loop<D_SGL, false>(a, UPBD_BODY { b_apply_solid(v, P, vb); });

@@ -252,7 +252,7 @@ constexpr int DL = 2;        // threads per particle in the displacement pass
 constexpr uint32_t CHUNK = 32 / GLF;  // fluid particles of one cell that a warp takes in the density pass
 constexpr int CHUNK_SHIFT = 28;       // chunk place: slot, above it the size of the chunk that starts there
 constexpr uint32_t CHUNK_SLOT = (1u << CHUNK_SHIFT) - 1u;  // a scene of 2^28 slots would need 240 GB
-constexpr int GT = 16;       // lanes per solid in the tet solve
+constexpr int GT = 16;       // lanes per solid in the tet solve (32 for small bodies)
 constexpr uint32_t CL_NEAR = 0x80000000u;  // contact cache entry flag: a lattice neighbour (solids stay below 2^31)
 
 // xsph sums over the fluid candidates within H at its own time, after the

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) k_apply_fluid(SimView v, const DevParams*
 }
 template <bool APPLY_FLUID, int OUT>
 __global__ void __launch_bounds__(256) k_solid_solve(SimView v, const DevParams* __restrict__ P, int solid_pad, int q) {
-  b_solid_solve<APPLY_FLUID, OUT>(v, P, solid_pad, q, blockIdx.x);
+  b_solid_solve<APPLY_FLUID, OUT, 4>(v, P, solid_pad, q, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_apply_solid(SimView v, const DevParams* __restrict__ P) {
   b_apply_solid(v, P, blockIdx.x);
@@ -99,9 +99,9 @@ template <bool LAST>
 __global__ void __launch_bounds__(256) k_solid_contacts(SimView v, const DevParams* __restrict__ P, int q) {
   b_solid_contacts<LAST>(v, P, q, blockIdx.x);
 }
-template <bool LAST>
+template <bool LAST, int G>
 __global__ void __launch_bounds__(256) k_solve_tets(SimView v, const DevParams* __restrict__ P, int q) {
-  b_solve_tets<LAST>(v, P, q, blockIdx.x);
+  b_solve_tets<LAST, G>(v, P, q, blockIdx.x);
 }
 __global__ void __launch_bounds__(256) k_bond_contacts(SimView v, const DevParams* __restrict__ P, int nb, int nt,
                                                        int nb_pad, int nc) {

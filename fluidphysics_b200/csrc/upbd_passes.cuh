@@ -302,13 +302,21 @@ __device__ __forceinline__ void copy_row_async(real4* dst, const real4* src) {
 __device__ __forceinline__ void copy_rows_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Squared distance inside the gathers: the product build's rounding is spelled
-// out (the compiler may fuse either product first), the parity build's
-// operations are the reference's.
+// out (the compiler may fuse the x or the y product into the first sum, and
+// chooses anew with every change around it), the parity build's operations are
+// the reference's. The fluid gathers fuse x, the distance solve y.
 __device__ __forceinline__ real dist2(real ex, real ey, real ez) {
 #ifdef UPBD_PARITY_BUILD
   return dot3(ex, ey, ez, ex, ey, ez);
 #else
   return r_fma(ez, ez, r_fma(ex, ex, ey * ey));
+#endif
+}
+__device__ __forceinline__ real dist2_xy(real ex, real ey, real ez) {
+#ifdef UPBD_PARITY_BUILD
+  return dot3(ex, ey, ez, ex, ey, ez);
+#else
+  return r_fma(ez, ez, r_fma(ey, ey, ex * ex));
 #endif
 }
 
@@ -747,6 +755,11 @@ __device__ __forceinline__ void mark_fluid_near(const SimView& v, const DevParam
 // incident constraints k = st+l, st+l+GL, ... of the static CSR, whose other
 // endpoint and pair scale 1/max(deg_i, deg_j) are precomputed (both are fixed
 // for the life of the scene); the partials combine like lane_sum.
+// U constraints' loads are in flight together. Bound by the latency of its
+// loads (offsets -> constraint ids and other ends -> constraint and position):
+// with two in flight behind one another's branches a launch took 10.7 us on
+// 8,512 solids, with four at once 8.7 (B200, event-timed, about 4 of which are
+// the launch). The batch, bound by occupancy, keeps two and 40 registers.
 // Threads from solid_pad on (a warp multiple, so the solve's warps are whole)
 // apply the fluid displacement when APPLY_FLUID (applyDeltaFluid,
 // src/gpu/wgsl.js:318-323): the solve reads solid positions only.
@@ -785,7 +798,7 @@ __device__ __forceinline__ void solid_store(const SimView& v, int q, int i, bool
   }
 }
 
-template <bool APPLY_FLUID, int OUT = SOLVE_DELTA>
+template <bool APPLY_FLUID, int OUT, int U>
 __device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams* __restrict__ P, int solid_pad, int q,
                                               uint32_t vb) {
   const int t = UPBD_VTID;
@@ -825,24 +838,43 @@ __device__ __forceinline__ void b_solid_solve(const SimView& v, const DevParams*
     const real alpha = P->compliance / (h * h);
     const uint32_t* __restrict__ ids = v.adj + v.S + 1;
     const uint4* __restrict__ cons = v.cons;
-#pragma unroll 2
-    for (uint32_t k = st + lane; k < en; k += GL) {
-      const uint32_t ci = __ldg(&ids[k]);
-      const uint32_t other = __ldg(&v.adj_other[k]);
-      if (!UPBD_IDX_OK(v, ci, v.C) || !UPBD_IDX_OK(v, other, v.S)) continue;
-      const real s = __ldg(&v.adj_scale[k]);
-      const real4 po = pos[other];
-      const uint2 rw = *reinterpret_cast<const uint2*>(&cons[ci].z);  // rest bits, alive
-      if (rw.y == 0u) continue;
-      const real rest = __uint_as_float(rw.x);
-      const real ex = pi.x - po.x, ey = pi.y - po.y, ez = pi.z - po.z;
-      const real d = r_sqrt(dot3(ex, ey, ez, ex, ey, ez));
-      if (d < 1e-9f) continue;
-      const real wsum = wi + po.w;
-      if (wsum == 0.f) continue;
-      const real dl = -(d - rest) / (wsum + alpha);
-      const real f = dl * wi / d * s;
-      cx = cx + ex * f; cy = cy + ey * f; cz = cz + ez * f;
+    // U constraints at a time: their loads are in flight together (a lane has
+    // at most four of an inner solid's 26)
+    for (uint32_t k0 = st + lane; k0 < en; k0 += GL * U) {
+      uint32_t ci[U], other[U];
+      real s[U];
+      real4 po[U];
+      uint2 rw[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const uint32_t k = min(k0 + (uint32_t)(u * GL), en - 1u);
+        ci[u] = __ldg(&ids[k]);
+        other[u] = __ldg(&v.adj_other[k]);
+        s[u] = __ldg(&v.adj_scale[k]);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (!UPBD_IDX_OK(v, ci[u], v.C) || !UPBD_IDX_OK(v, other[u], v.S)) {
+          rw[u] = make_uint2(0u, 0u);
+          po[u] = pi;
+          continue;
+        }
+        po[u] = pos[other[u]];
+        rw[u] = *reinterpret_cast<const uint2*>(&cons[ci[u]].z);  // rest bits, alive
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (k0 + (uint32_t)(u * GL) >= en || rw[u].y == 0u) continue;
+        const real rest = __uint_as_float(rw[u].x);
+        const real ex = pi.x - po[u].x, ey = pi.y - po[u].y, ez = pi.z - po[u].z;
+        const real d = r_sqrt(dist2_xy(ex, ey, ez));
+        if (d < 1e-9f) continue;
+        const real wsum = wi + po[u].w;
+        if (wsum == 0.f) continue;
+        const real dl = -(d - rest) / (wsum + alpha);
+        const real f = dl * wi / d * s[u];
+        cx = cx + ex * f; cy = cy + ey * f; cz = cz + ez * f;
+      }
     }
   }
   cx = lane_sum(cx);
@@ -1120,17 +1152,20 @@ __device__ __forceinline__ void tet_corner(const DevParams* __restrict__ P, cons
   ox = c1x; oy = c1y; oz = c1z;
 }
 
-// solveTets + its apply, a phase of the folded solve: GT lanes per solid
-// compute the corrections of its next GT tets side by side (corners and pair
+// solveTets + its apply, a phase of the folded solve: G lanes per solid
+// compute the corrections of its next G tets side by side (corners and pair
 // scale in one row per incidence), then every lane adds them up in the CSR's
 // order, so the sum is the one-thread loop's. Bound by latency (record ->
 // corners -> arithmetic): inner solids have 8 or 32 tets, so one or two rounds
 // of 16 lanes; one thread per solid, 32 tets in a chain, took 34 us a launch
-// on 8,512 solids (B200, event-timed).
-template <bool LAST>
+// on 8,512 solids (B200, event-timed), 16 lanes take 10.7. One round of 32
+// lanes is faster where the launch fits one block an SM (793 solids: 8.5
+// against 8.8 us), slower where half its lanes' issue slots are missed (8,512:
+// 12.7).
+template <bool LAST, int G = GT>
 __device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* __restrict__ P, int q, uint32_t vb) {
   const unsigned FULL = 0xffffffffu;
-  const int i = (int)(UPBD_VTID / GT), lane = (int)(threadIdx.x & (GT - 1));
+  const int i = (int)(UPBD_VTID / G), lane = (int)(threadIdx.x & (G - 1));
   const real4* __restrict__ pos = solid_src(v, q);
   const uint32_t* __restrict__ ids = v.tet_adj + v.S + 1;
   real4 pi = make_real4(0.f, 0.f, 0.f, 0.f);
@@ -1148,7 +1183,7 @@ __device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* 
   const bool act = (fl & F_ACTIVE) != 0u;
   if (!act) en = st;
   real cx = 0.f, cy = 0.f, cz = 0.f;
-  for (uint32_t k0 = st; __any_sync(FULL, k0 < en); k0 += GT) {
+  for (uint32_t k0 = st; __any_sync(FULL, k0 < en); k0 += G) {
     const uint32_t k = k0 + (uint32_t)lane;
     real ox = 0.f, oy = 0.f, oz = 0.f;
     if (k < en) {
@@ -1162,10 +1197,10 @@ __device__ __forceinline__ void b_solve_tets(const SimView& v, const DevParams* 
       }
     }
 #pragma unroll
-    for (int l = 0; l < GT; l++) {
-      cx = cx + __shfl_sync(FULL, ox, l, GT);
-      cy = cy + __shfl_sync(FULL, oy, l, GT);
-      cz = cz + __shfl_sync(FULL, oz, l, GT);
+    for (int l = 0; l < G; l++) {
+      cx = cx + __shfl_sync(FULL, ox, l, G);
+      cy = cy + __shfl_sync(FULL, oy, l, G);
+      cz = cz + __shfl_sync(FULL, oz, l, G);
     }
   }
   if (i < v.S && lane == 0) solid_store<LAST>(v, q, i, act, act ? apply_clamped(P, pi, cx, cy, cz) : pi);
