@@ -142,8 +142,8 @@ struct SimView {
   real4* pvrow;
   uint32_t* slot;      // slot of particle i in this substep's grid
   // Inside a bucket, entries run in descending index, so fluid (indices >= S)
-  // precede solids: fend[h] splits bucket h into [start[h], fend[h]) fluid and
-  // [fend[h], start[h+1]) solid.
+  // precede solids: fend[h] splits an occupied bucket h into [start[h], fend[h])
+  // fluid and [fend[h], start[h+1]) solid.
   uint32_t* fend;
   // Density-pass neighbour lists: lane l (of GLF) of the fluid particle at
   // slot e records the slots of its fluid candidates within the list radius
@@ -154,7 +154,7 @@ struct SimView {
   // Movement between the density pass and xsph (written by the bounds pass):
   // smove[e] for the fluid particle at slot e (+inf when it left its cell),
   // bmove[h] the largest movement above XMOVE_REC * the allowance among the
-  // particles of bucket h (float bits; cleared by the scan).
+  // particles of bucket h (float bits; the rank fix-up clears the occupied ones').
   float* smove;
   uint32_t* bmove;
   const uint32_t* adj_other;  // CSR-parallel: the other endpoint of constraint ids[k]
@@ -324,6 +324,16 @@ __device__ __forceinline__ void group_cell_hash(real px, real py, real pz, doubl
 static __shared__ uint32_t s_walk_base[256 / GLF][28];  // slot of candidate 0 of cell k, minus its offset
 static __shared__ uint32_t s_walk_off[256 / GLF][28];   // sequence offset of cell k ([27] = total)
 
+// First slot and length of bucket h's fluid (PART 0) or solids (PART 1). Only
+// occupied buckets have a valid fend (the rank fix-up writes it): writing all
+// of them in the scan is a sweep over the table a substep.
+template <int PART>
+__device__ __forceinline__ uint2 bucket_range(const SimView& v, uint32_t h) {
+  const uint32_t s = __ldg(&v.start[h]), e = __ldg(&v.start[h + 1]), f = __ldg(&v.fend[h]);
+  if (e == s) return make_uint2(s, 0u);
+  return PART == 0 ? make_uint2(s, f - s) : make_uint2(f, e - f);
+}
+
 // The shared tables of a walk: row g (this lane's group) gets the slot base
 // and sequence offset of each of the 27 cells; returns the sequence length.
 template <int PART, int G>
@@ -339,14 +349,9 @@ __device__ __forceinline__ uint32_t walk_tables(const SimView& v, const CellHash
     uint32_t s = 0, n = 0;
     if (walk && k < 27) {
       const uint32_t hb = ch.bucket_k(k, mask);
-      const uint32_t f = __ldg(&v.fend[hb]);
-      if (PART == 0) {
-        s = __ldg(&v.start[hb]);
-        n = f - s;
-      } else {
-        s = f;
-        n = __ldg(&v.start[hb + 1]) - f;
-      }
+      const uint2 r = bucket_range<PART>(v, hb);
+      s = r.x;
+      n = r.y;
     }
     uint32_t x = n;  // inclusive scan over the group's lanes (cell order within the round)
 #pragma unroll

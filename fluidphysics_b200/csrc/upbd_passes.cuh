@@ -97,7 +97,8 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
 // scanBlocks/scanPartials/scanApply (src/gpu/wgsl.js:180-236) as one launch:
 // block b scans its own SCAN_TILE counts (SCAN_PER consecutive ones per
 // thread), adds the totals of tiles < b (the count's tile counters, all
-// replicas), writes start[], and clears the counts it read. The counts and the
+// replicas) and writes start[]; the rank fix-up clears the occupied buckets'
+// counts, movement and fluid ends, so that the table is swept once. The counts and the
 // earlier totals are loaded up front so that their latencies overlap, and one
 // block barrier publishes both per-warp sums. COUNTS: the counts themselves go
 // to counts_out. Four counts a thread: with eight (256 threads a block) the
@@ -116,7 +117,7 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
   // be a caller's buffer at any 4-byte offset)
   const bool vec = t0 + SCAN_PER <= (long long)v.T &&
                    ((reinterpret_cast<uintptr_t>(v.counts) | reinterpret_cast<uintptr_t>(v.start) |
-                     reinterpret_cast<uintptr_t>(v.fend) | reinterpret_cast<uintptr_t>(counts_out)) & 15u) == 0;
+                     reinterpret_cast<uintptr_t>(counts_out)) & 15u) == 0;
   uint4 c = make_uint4(0u, 0u, 0u, 0u);
   if (vec) {
     c = *reinterpret_cast<const uint4*>(v.counts + t0);
@@ -155,13 +156,9 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
     if (w < wid) run += s_scan[w];
   }
   const uint4 r = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
   if (vec) {
     *reinterpret_cast<uint4*>(v.start + t0) = r;
-    if (v.fend) *reinterpret_cast<uint4*>(v.fend + t0) = r;  // empty buckets; rankfix sets occupied ones
     if (COUNTS) *reinterpret_cast<uint4*>(counts_out + t0) = c;
-    *reinterpret_cast<uint4*>(v.counts + t0) = z;             // ready for the next count
-    if (v.bmove) *reinterpret_cast<uint4*>(v.bmove + t0) = z;  // no movement recorded yet this substep
   } else {
     const uint32_t cs[4] = {c.x, c.y, c.z, c.w}, rs[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
@@ -169,10 +166,7 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
       const long long idx = t0 + k;
       if (idx < v.T) {
         v.start[idx] = rs[k];
-        if (v.fend) v.fend[idx] = rs[k];
         if (COUNTS) counts_out[idx] = cs[k];
-        v.counts[idx] = 0u;
-        if (v.bmove) v.bmove[idx] = 0u;
       }
     }
   }
@@ -227,6 +221,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   if (!v.spos) {  // the stateless grid build has no bucket-ordered copies
     for (uint32_t k = s; k < e; k++) rank += (v.tmp[k] > (uint32_t)i) ? 1u : 0u;
     if (UPBD_IDX_OK(v, s + rank, v.N)) v.entries[s + rank] = (uint32_t)i;
+    if (rank == 0u) v.counts[h] = 0u;  // ready for the next count
     return;
   }
   const uint32_t key = cell_keys(v)[i];
@@ -245,7 +240,11 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   if (!UPBD_IDX_OK(v, slot, v.N)) return;
   v.entries[slot] = (uint32_t)i;
   v.slot[i] = slot;
-  v.fend[h] = e - solids;  // every member writes the same value
+  if (rank == 0u) {
+    v.fend[h] = e - solids;
+    v.counts[h] = 0u;  // ready for the next count
+    v.bmove[h] = 0u;   // no movement recorded yet this substep
+  }
   if (i >= v.S) {
     const uint32_t n = (rank_in % CHUNK == 0u) ? min(CHUNK, mates - rank_in) : 0u;
     chunk_places(v)[s + before + rank_in] = slot | (n << CHUNK_SHIFT);
@@ -465,8 +464,9 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
       const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
       uint32_t s0 = 0, n = 0;
       if (L < 27) {
-        s0 = __ldg(&v.start[hb]);
-        n = __ldg(&v.fend[hb]) - s0;
+        const uint2 r = bucket_range<0>(v, hb);
+        s0 = r.x;
+        n = r.y;
       }
       const uint32_t end = warp_scan(n, L);  // in cell order
       const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
@@ -675,8 +675,8 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
         uint32_t c = 0;
         for (int kk = 0; kk < 27; kk++) {
           const uint32_t hb = ch.bucket_k(kk, mask);
-          const uint32_t s0 = __ldg(&v.start[hb]), s1 = __ldg(&v.fend[hb]);
-          for (uint32_t e = s0; e < s1; e++, c++)
+          const uint2 r = bucket_range<0>(v, hb);
+          for (uint32_t e = r.x; e < r.x + r.y; e++, c++)
             if ((c & (GLF - 1)) == (uint32_t)l && e != e0) pair(rows[2 * (size_t)e], rows[2 * (size_t)e + 1]);
         }
       }
@@ -1555,15 +1555,18 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
         rem &= ~turn;
         const bool mine_turn = (turn >> L & 1u) != 0u;
         const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
-        const uint32_t bm = __reduce_max_sync(FULL, (L < 27) ? v.bmove[hb] : 0u);  // a finite distance or +inf
+        uint32_t s0 = 0, n = 0, bm = 0;  // the bucket's fluid; a finite distance or +inf
+        if (L < 27) {
+          const uint2 r = bucket_range<0>(v, hb);
+          s0 = r.x;
+          n = r.y;
+          bm = v.bmove[hb];
+          if (n == 0u) bm = 0u;
+        }
+        bm = __reduce_max_sync(FULL, bm);
         if (mine_turn) listed = !over && sm + r_fmax(rec, (real)__uint_as_float(bm)) <= allow;
         const bool walks = mine_turn && !listed;
         if (!__any_sync(FULL, walks)) continue;
-        uint32_t s0 = 0, n = 0;
-        if (L < 27) {
-          s0 = __ldg(&v.start[hb]);
-          n = __ldg(&v.fend[hb]) - s0;
-        }
         const uint32_t end = warp_scan(n, L);  // in cell order
         const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
         for (uint32_t q0 = 0; q0 < total; q0 += XROWS) {
