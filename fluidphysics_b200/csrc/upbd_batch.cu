@@ -421,11 +421,27 @@ int upload_table(upbd_batch* b) {
   return UPBD_OK;
 }
 
+// Virtual blocks of a domain over all live scenes, as the table has them.
+uint32_t total_blocks(const upbd_batch* b, int d) {
+  const uint32_t* pre = (const uint32_t*)(b->h_tab + b->off_prefix);
+  return pre[(size_t)d * b->stride + b->scenes.size()];
+}
+// x rounded up to three significant bits: at most an eighth more, and few
+// distinct values for scenes that come and go
+uint32_t quantized(uint32_t x) {
+  uint32_t step = 1;
+  while (x / step >= 16u) step *= 2u;
+  return (x + step - 1u) / step * step;
+}
+
 // The frame's launch sequence (GpuSim.encode's pass order, src/gpu/sim.js:
 // 354-391), each pass one persistent launch over every scene.
 int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
   const BatchArgs a = batch_args(b);
   const unsigned G = (unsigned)(b->cps * b->num_sms);
+  auto grid = [&](int d) {  // CTAs of a launch over domain d: no more than it has tiles
+    return std::max(1u, std::min(G, quantized(total_blocks(b, d))));
+  };
   const unsigned BT = (unsigned)b->bt;
   cudaStream_t st = b->stream;
   const bool tets = (b->desc.features & UPBD_FEAT_TETS) != 0;
@@ -437,45 +453,45 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
   const bool mark_in_apply = iters > 0 && per == 1;
   const bool fold = phases >= 2;
   for (int k = 0; k < nsub; k++) {
-    BLAUNCH(b, K_INTEGRATE, kb_integrate_count<true, true><<<G, BT, 0, st>>>(a));
-    BLAUNCH(b, K_SCAN, kb_scan<<<G, SCAN_THREADS, 0, st>>>(a));
-    BLAUNCH(b, K_SCATTER, kb_scatter<<<G, BT, 0, st>>>(a));
-    BLAUNCH(b, K_RANKFIX, kb_rankfix<<<G, BT, 0, st>>>(a));
-    BLAUNCH(b, K_DENSITY, kb_density<<<G, BT, (BT / 32) * STAGE_WARP, st>>>(a));
+    BLAUNCH(b, K_INTEGRATE, kb_integrate_count<true, true><<<grid(D_N), BT, 0, st>>>(a));
+    BLAUNCH(b, K_SCAN, kb_scan<<<grid(D_TILES), SCAN_THREADS, 0, st>>>(a));
+    BLAUNCH(b, K_SCATTER, kb_scatter<<<grid(D_SCATTER), BT, 0, st>>>(a));
+    BLAUNCH(b, K_RANKFIX, kb_rankfix<<<grid(D_N), BT, 0, st>>>(a));
+    BLAUNCH(b, K_DENSITY, kb_density<<<grid(D_CHUNK), BT, (BT / 32) * STAGE_WARP, st>>>(a));
     if (fold)  // the displacement pass applies the fluid's move (b_disp<true>)
-      BLAUNCH(b, K_DISP, kb_disp<true><<<G, BT, 0, st>>>(a));
+      BLAUNCH(b, K_DISP, kb_disp<true><<<grid(D_DISP), BT, 0, st>>>(a));
     else
-      BLAUNCH(b, K_DISP, kb_disp<false><<<G, BT, 0, st>>>(a));
-    if (iters == 0) BLAUNCH(b, K_APPLY_FLUID, kb_apply_fluid<<<G, BT, 0, st>>>(a));
-    if (scc && fold) BLAUNCH(b, K_COLLECT, kb_collect_contacts<<<G, BT, 0, st>>>(a));
+      BLAUNCH(b, K_DISP, kb_disp<false><<<grid(D_DISP), BT, 0, st>>>(a));
+    if (iters == 0) BLAUNCH(b, K_APPLY_FLUID, kb_apply_fluid<<<grid(D_F), BT, 0, st>>>(a));
+    if (scc && fold) BLAUNCH(b, K_COLLECT, kb_collect_contacts<<<grid(D_SW), BT, 0, st>>>(a));
     for (int q = 0; q < phases && fold; q++) {
       const int kind = q % per;
       const bool lastq = q == phases - 1;
       if (kind == 0) {
-        if (!lastq) BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_STEP><<<G, BT, 0, st>>>(a, q)));
-        else BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_LAST><<<G, BT, 0, st>>>(a, q)));
+        if (!lastq) BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_STEP><<<grid(D_SOLVE), BT, 0, st>>>(a, q)));
+        else BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<false, SOLVE_LAST><<<grid(D_SOLVE), BT, 0, st>>>(a, q)));
       } else if (tets && kind == 1) {
-        if (!lastq) BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<false><<<G, BT, 0, st>>>(a, q));
-        else BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<true><<<G, BT, 0, st>>>(a, q));
+        if (!lastq) BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<false><<<grid(D_STL), BT, 0, st>>>(a, q));
+        else BLAUNCH(b, K_SOLVE_TETS, kb_solve_tets<true><<<grid(D_STL), BT, 0, st>>>(a, q));
       } else {
-        if (!lastq) BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<false><<<G, BT, 0, st>>>(a, q));
-        else BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<true><<<G, BT, 0, st>>>(a, q));
+        if (!lastq) BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<false><<<grid(D_SGL), BT, 0, st>>>(a, q));
+        else BLAUNCH(b, K_SOLID_CONTACTS, kb_solid_contacts<true><<<grid(D_SGL), BT, 0, st>>>(a, q));
       }
     }
     if (phases == 1) {  // one plain iteration: split
-      BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<true, SOLVE_DELTA><<<G, BT, 0, st>>>(a, 0)));
-      BLAUNCH(b, K_APPLY_SOLID, kb_apply_solid<<<G, BT, 0, st>>>(a));
+      BLAUNCH(b, K_SOLID_SOLVE, (kb_solid_solve<true, SOLVE_DELTA><<<grid(D_SOLVE0), BT, 0, st>>>(a, 0)));
+      BLAUNCH(b, K_APPLY_SOLID, kb_apply_solid<<<grid(D_SGL), BT, 0, st>>>(a));
     }
-    if (!mark_in_apply) BLAUNCH(b, K_APPLY_SOLID, kb_contact_mark<<<G, BT, 0, st>>>(a));
-    BLAUNCH(b, K_BOND_CONTACTS, kb_bond_contacts<<<G, BT, 0, st>>>(a, tets ? 1 : 0));
-    BLAUNCH(b, K_APPLY_BOUNDS_VEL, kb_apply_bounds_vel<<<G, BT, 0, st>>>(a));
+    if (!mark_in_apply) BLAUNCH(b, K_APPLY_SOLID, kb_contact_mark<<<grid(D_SGL), BT, 0, st>>>(a));
+    BLAUNCH(b, K_BOND_CONTACTS, kb_bond_contacts<<<grid(D_BC), BT, 0, st>>>(a, tets ? 1 : 0));
+    BLAUNCH(b, K_APPLY_BOUNDS_VEL, kb_apply_bounds_vel<<<grid(D_N), BT, 0, st>>>(a));
     if (visc) {
-      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc<<<G, BT, 0, st>>>(a));
-      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc_apply<<<G, BT, 0, st>>>(a));
+      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc<<<grid(D_S), BT, 0, st>>>(a));
+      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc_apply<<<grid(D_S), BT, 0, st>>>(a));
     }
-    BLAUNCH(b, K_XSPH, kb_xsph<<<G, BT, (BT / 32) * STAGE_WARP, st>>>(a));  // writes the blended velocity itself
+    BLAUNCH(b, K_XSPH, kb_xsph<<<grid(D_CHUNK), BT, (BT / 32) * STAGE_WARP, st>>>(a));  // writes the blended velocity itself
   }
-  BLAUNCH(b, K_COUNT_ACTIVE, kb_count_active<<<G, BT, 0, st>>>(a));
+  BLAUNCH(b, K_COUNT_ACTIVE, kb_count_active<<<grid(D_F), BT, 0, st>>>(a));
   const cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) return bfail(b, UPBD_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   return UPBD_OK;
@@ -509,7 +525,10 @@ int enqueue_batch_frame(upbd_batch* b, double dt, int nsub, bool profile) {
   bool visc = false;
   for (auto& kv : b->scenes) visc = visc || kv.second.prm.solid_viscosity > 0;
   if (!profile) {
-    const uint64_t key = (uint64_t)nsub | ((uint64_t)b->bt << 16) | ((uint64_t)b->cps << 32) | ((uint64_t)visc << 48);
+    // a graph's grids are those of the scenes at its capture; any grid covers
+    // any table, so the key follows the size in coarse steps only
+    const uint64_t key = (uint64_t)nsub | ((uint64_t)(b->bt / 64) << 10) | ((uint64_t)b->cps << 14) | ((uint64_t)visc << 23) |
+                         ((uint64_t)quantized(total_blocks(b, D_N)) << 24);
     auto it = b->graphs.find(key);
     if (it == b->graphs.end()) {
       cudaGraph_t g;
