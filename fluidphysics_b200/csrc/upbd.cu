@@ -318,16 +318,27 @@ int launch_substep(upbd_sim* s, int last) {
   }
   UPBD_KCK(s);
   if (last < UPBD_PASS_SOLID_VISC) return UPBD_OK;
-  if (s->prm.solid_viscosity > 0) {
-    PROF(s, K_SOLID_VISC, k_solid_visc<<<blocks_for(v.S), 256, 0, st>>>(v, P));
-    PROF(s, K_SOLID_VISC, k_solid_visc_apply<<<blocks_for(v.S), 256, 0, st>>>(v));
+  // solid viscosity touches the solids' velocities alone and xsph the fluid's:
+  // in a full substep they run side by side
+  const bool visc = s->prm.solid_viscosity > 0;
+  const bool visc_beside = visc && last >= UPBD_PASS_XSPH && !s->prof_on && s->side;
+  if (visc) {
+    cudaStream_t vs = visc_beside ? s->side : st;
+    if (visc_beside) {
+      UPBD_CK(s, cudaEventRecord(s->fork_ev, st));
+      UPBD_CK(s, cudaStreamWaitEvent(s->side, s->fork_ev, 0));
+    }
+    PROF(s, K_SOLID_VISC, k_solid_visc<<<blk_gl, 256, 0, vs>>>(v, P));
+    PROF(s, K_SOLID_VISC, k_solid_visc_apply<<<blocks_for(v.S), 256, 0, vs>>>(v));
     L += 2;
+    if (visc_beside) UPBD_CK(s, cudaEventRecord(s->join_ev, s->side));
   }
   if (last < UPBD_PASS_XSPH) return UPBD_OK;
   if (last < UPBD_PASS_XSPH_APPLY)  // stop with the result in delta, as the reference's xsph pass leaves it
     PROF(s, K_XSPH, k_xsph<false><<<blocks_for(v.N, (int)window), 256, 8 * STAGE_WARP, st>>>(v, P, window));
   else
     PROF(s, K_XSPH, k_xsph<true><<<blocks_for(v.N, (int)window), 256, 8 * STAGE_WARP, st>>>(v, P, window));
+  if (visc_beside) UPBD_CK(s, cudaStreamWaitEvent(st, s->join_ev, 0));
   L++;
   UPBD_KCK(s);
   return UPBD_OK;

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) kb_apply_bounds_vel(BatchArgs a) {
   batch_loop<D_N, false>(a, UPBD_BODY { b_apply_bounds_vel(v, P, 3, vb); });
 }
 __global__ void __launch_bounds__(256) kb_solid_visc(BatchArgs a) {
-  batch_loop<D_S, false>(a, UPBD_BODY {
+  batch_loop<D_SGL, false>(a, UPBD_BODY {
     if (P->solid_viscosity > 0.f) b_solid_visc(v, P, vb);
   });
 }
@@ -486,7 +486,7 @@ int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
     BLAUNCH(b, K_BOND_CONTACTS, kb_bond_contacts<<<grid(D_BC), BT, 0, st>>>(a, tets ? 1 : 0));
     BLAUNCH(b, K_APPLY_BOUNDS_VEL, kb_apply_bounds_vel<<<grid(D_N), BT, 0, st>>>(a));
     if (visc) {
-      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc<<<grid(D_S), BT, 0, st>>>(a));
+      BLAUNCH(b, K_SOLID_VISC, kb_solid_visc<<<grid(D_SGL), BT, 0, st>>>(a));
       BLAUNCH(b, K_SOLID_VISC, kb_solid_visc_apply<<<grid(D_S), BT, 0, st>>>(a));
     }
     BLAUNCH(b, K_XSPH, kb_xsph<<<grid(D_CHUNK), BT, (BT / 32) * STAGE_WARP, st>>>(a));  // writes the blended velocity itself

@@ -1453,22 +1453,51 @@ __device__ __forceinline__ void b_apply_bounds_vel(const SimView& v, const DevPa
   if (!iSolid) store_row_pair(&v.pvrow[2 * (size_t)sl], make_real4(p.x, p.y, p.z, slot_pack(real(0), sl)), nv);  // xsph's neighbours
 }
 
-// solidVisc, src/gpu/wgsl.js:717-735
+// solidVisc, src/gpu/wgsl.js:717-735, GL lanes per solid: they load its next GL
+// neighbours' velocities side by side, then every lane adds the bonded ones up
+// in the CSR's order (the one-thread loop's sums). Bound by latency: one thread
+// a solid, 26 neighbours in a chain, took 9.7 us a launch on 793 solids, 7.6 now
+// (B200, event-timed).
 __device__ __forceinline__ void b_solid_visc(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
-  const int i = UPBD_VTID;
-  if (i >= v.S) return;
-  if (!(v.flags[i] & F_ACTIVE)) return;
-  const uint32_t* ids = v.adj + v.S + 1;
-  real sx = 0.f, sy = 0.f, sz = 0.f, m = 0.f;
-  for (uint32_t k = v.adj[i]; k < v.adj[i + 1]; k++) {
-    const uint4 c = v.cons[ids[k]];
-    if (c.w == 0u) continue;
-    const uint32_t other = (c.x == (uint32_t)i) ? c.y : c.x;
-    const real4 vo = v.vel[other];
-    sx = sx + vo.x; sy = sy + vo.y; sz = sz + vo.z;
-    m = m + 1.0f;
+  const unsigned FULL = 0xffffffffu;
+  const int i = (int)(UPBD_VTID / GL), lane = (int)(threadIdx.x & (GL - 1)), group = (int)(threadIdx.x & 31) & ~(GL - 1);
+  uint32_t fl = 0, st = 0, en = 0;
+  real4 vi = make_real4(0.f, 0.f, 0.f, 0.f);
+  if (i < v.S) {
+    fl = v.flags[i];
+    st = v.adj[i];
+    en = v.adj[i + 1];
+    vi = v.vel[i];
+    issued(fl);
+    issued(st);
+    issued(en);
+    issued(vi);
   }
-  const real4 vi = v.vel[i];
+  const bool act = (fl & F_ACTIVE) != 0u;
+  if (!act) en = st;
+  real sx = 0.f, sy = 0.f, sz = 0.f, m = 0.f;
+  for (uint32_t k0 = st; __any_sync(FULL, k0 < en); k0 += GL) {
+    const uint32_t k = k0 + (uint32_t)lane;
+    bool bonded = false;
+    real4 vo = make_real4(0.f, 0.f, 0.f, 0.f);
+    if (k < en) {
+      const uint32_t ci = v.adj[v.S + 1 + k], other = v.adj_other[k];
+      if (UPBD_IDX_OK(v, ci, v.C) && UPBD_IDX_OK(v, other, v.S)) {
+        bonded = v.cons[ci].w != 0u;
+        vo = v.vel[other];
+      }
+    }
+    const unsigned bonds = __ballot_sync(FULL, bonded) >> group;
+#pragma unroll
+    for (int l = 0; l < GL; l++) {
+      const real x = __shfl_sync(FULL, vo.x, l, GL), y = __shfl_sync(FULL, vo.y, l, GL), z = __shfl_sync(FULL, vo.z, l, GL);
+      if (bonds >> l & 1u) {
+        sx = sx + x; sy = sy + y; sz = sz + z;
+        m = m + 1.0f;
+      }
+    }
+  }
+  if (!act || lane != 0) return;
   real vx = vi.x, vy = vi.y, vz = vi.z;
   if (m > 0.f) {
     const real mu = P->solid_viscosity;

@@ -50,3 +50,41 @@ def test_solid_phases_bit_exact(features, iters, dim, dim2, squeeze, cut):
     if features & L.FEAT_SOLID_CONTACTS and squeeze < 0.6:
         assert o2.read_contact_cache()[0].max() == 40  # the cache was full somewhere
     sim.close()
+
+
+@pytest.mark.parametrize("dim,dim2", [(1, 0), (2, 0), (5, 2), (9, 4)])
+def test_solid_viscosity_bit_exact_and_batched(dim, dim2):
+    """Solid viscosity on its lanes: single scene against the oracle (cut body,
+    stirred velocities), and the same scene in a batch beside one without it."""
+    from fluidphysics_b200 import batch as B
+    d, p, opts = S.gpu_scene(dim, 300, 30, iters=2)
+    d.solid_dim2 = dim2
+    d.cube2_center[:] = [0.9, 1.0, 0.7]
+    S.set_params(p, {"solidViscosity": 0.3})
+    fp = S.jittered_block(8, 5, 8, 0.066, 0.1, 4)[:300]
+    sc = S.Scene("visc", d, p, fp, np.zeros_like(fp), opts["fluidMass"], 1 / 60, 5, 1)
+    sim, o2 = sim_from_scene(sc, "parity"), o2_from_scene(sc)
+    st, cons = sim.read_state(), sim.read_constraints()
+    n = sc.solid_n
+    rng = np.random.default_rng(dim)
+    st["vel"][:n, :3] = rng.normal(0, 1, (n, 3))
+    side = st["pos"][:n, 0] > st["pos"][:n, 0].mean() + 0.001
+    cons[side[cons[:, 0]] != side[cons[:, 1]], 3] = 0
+    load_state(sim, st, cons)
+    o2.write_state(**st)
+    o2.write_constraints(cons)
+    sim.step(1 / 60, 3)
+    o2.step(1 / 60, 3)
+    g = sim.read_state()
+    assert_states_equal(g, o2.read_state(), "visc")
+    with B.Batch(solid_iters=2, max_scenes=2, variant="parity") as b:
+        sid = b.add_scene(sc)
+        b.add_scene(B.batch_scene(4, 500, 3, iters=2))
+        b.write_state(sid, **st)
+        b.write_constraints(sid, cons)
+        b.step(1 / 60, 3)
+        b.sync()
+        h = b.read_state(sid)
+    for k in ("pos", "vel", "flags"):
+        assert np.array_equal(g[k], h[k]), k
+    sim.close()
