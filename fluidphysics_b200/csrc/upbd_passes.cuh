@@ -938,16 +938,6 @@ __device__ __forceinline__ real lattice_rest(const SimView& v, real spacing, uin
   return spacing * r_sqrt(dx * dx + dy * dy + dz * dz);
 }
 
-// latticeAdjacent, src/gpu/wgsl.js:409-416
-__device__ __forceinline__ bool lattice_adjacent(const SimView& v, uint32_t i, uint32_t j) {
-  if ((i >= (uint32_t)v.N1) != (j >= (uint32_t)v.N1)) return false;
-  uint32_t a = i, b = j, D = (uint32_t)v.dim1;
-  if (i >= (uint32_t)v.N1) { a = i - v.N1; b = j - v.N1; D = (uint32_t)(v.dim2 > 1 ? v.dim2 : 1); }
-  const int ax = (int)(a / (D * D)), ay = (int)((a / D) % D), az = (int)(a % D);
-  const int bx = (int)(b / (D * D)), by = (int)((b / D) % D), bz = (int)(b % D);
-  return abs(ax - bx) <= 1 && abs(ay - by) <= 1 && abs(az - bz) <= 1;
-}
-
 // solidRsum: the contact distance of two solids, lattice neighbours or not
 __device__ __forceinline__ real solid_rsum(const DevParams* __restrict__ P, bool near) {
   const real rsum = 2.0f * P->solid_radius;
@@ -960,12 +950,14 @@ __device__ __forceinline__ real solid_rsum(const DevParams* __restrict__ P, bool
 // order, and a ballot gives each kept one its place, so the cache holds what
 // one invocation of the reference would list (the first C_K kept candidates).
 // A candidate's position is its slot copy (the solve writes the copies only at
-// its end). The solid's alive neighbours (at most 26, one per lane) are looked
-// up by shuffles. Entries carry CL_NEAR for lattice neighbours, whose contact
-// distance differs (solid_rsum), so the iterations need no index arithmetic.
-// Bound by the latency of its three or four dependent loads. One thread per
-// solid, as a chain of ~70 candidates with a constraint scan for each in
-// range, took 710 us a launch on 8,512 solids (B200, event-timed).
+// its end). The solid's lattice neighbours (at most 26, ascending, one per lane)
+// are searched by shuffles: a candidate found there is adjacent, and bonded if
+// its constraint is alive. Entries carry CL_NEAR for lattice neighbours, whose
+// contact distance differs (solid_rsum), so the iterations need no index
+// arithmetic. Bound by the latency of its three or four dependent loads. One
+// thread per solid, as a chain of ~70 candidates with a constraint scan for each
+// in range, took 710 us a launch on 8,512 solids (B200, event-timed); a warp with
+// lattice coordinates by division and 26 shuffles a round 24.9, this 14.8.
 __device__ __forceinline__ void b_collect_contacts(const SimView& v, const DevParams* __restrict__ P, uint32_t vb) {
   const unsigned FULL = 0xffffffffu;
   const int i = (int)(UPBD_VTID >> 5), lane = (int)(threadIdx.x & 31);
@@ -979,14 +971,24 @@ __device__ __forceinline__ void b_collect_contacts(const SimView& v, const DevPa
   group_cell_hash<32>(pi.x, pi.y, pi.z, P->inv_cell, ch);
   const int row = (int)(threadIdx.x >> 5) * (32 / GLF);
   const uint32_t run = walk_tables<1, 32>(v, ch, lane, true, row);
-  const uint32_t st = v.adj[i], en = v.adj[i + 1];
+  // the solid's lattice neighbours, one a lane in ascending index, and which of
+  // their constraints are alive
+  const uint32_t st = v.adj[i], deg = v.adj[i + 1] - st;
+  uint32_t neighbour = 0xffffffffu;
+  bool tied = false;
+  if ((uint32_t)lane < deg) {
+    const uint32_t ci = v.adj[v.S + 1 + st + lane];
+    neighbour = v.adj_other[st + lane];
+    tied = UPBD_IDX_OK(v, ci, v.C) && v.cons[ci].w != 0u;
+  }
+  const unsigned bonds = __ballot_sync(FULL, tied);
   const real margin = 2.0f * P->solid_radius;
-  const real wide = 2.0f * P->solid_radius + margin, wide2 = wide * wide;  // no contact distance is larger
+  const real lim_near = solid_rsum(P, true) + margin, lim_far = solid_rsum(P, false) + margin;
   uint32_t cnt = 0, k = 0, next = s_walk_off[row][1], base = s_walk_base[row][0];
   for (uint32_t c0 = 0; c0 < run && cnt < C_K; c0 += 32) {
     const uint32_t c = c0 + (uint32_t)lane;
-    uint32_t j = (uint32_t)i;
-    bool keep = false, near = false;
+    uint32_t j = 0xffffffffu;
+    real d2 = 0.f;
     if (c < run) {
       while (c >= next) {
         k++;
@@ -995,38 +997,26 @@ __device__ __forceinline__ void b_collect_contacts(const SimView& v, const DevPa
       }
       const uint32_t e = base + c;
       if (UPBD_IDX_OK(v, e, v.N)) {
-        const uint32_t jj = v.entries[e];
+        j = v.entries[e];
         const real4 pj = v.spos[e];
         const real ex = pi.x - pj.x, ey = pi.y - pj.y, ez = pi.z - pj.z;
-        const real d2 = dot3(ex, ey, ez, ex, ey, ez);
-        if (jj != (uint32_t)i && jj < (uint32_t)v.S && !(d2 >= wide2)) {
-          near = lattice_adjacent(v, (uint32_t)i, jj);
-          const real lim = solid_rsum(P, near) + margin;
-          j = jj;
-          keep = !(d2 >= lim * lim);
-        }
+        d2 = dot3(ex, ey, ez, ex, ey, ez);
       }
     }
-    // isBonded, src/gpu/wgsl.js:599-607: only lattice neighbours are
-    if (__any_sync(FULL, keep && near)) {
-      bool bonded = false;
-      for (uint32_t q0 = st; q0 < en; q0 += 32) {
-        uint32_t other = 0xffffffffu;
-        if (q0 + (uint32_t)lane < en) {
-          const uint32_t ci = v.adj[v.S + 1 + q0 + lane];
-          if (UPBD_IDX_OK(v, ci, v.C) && v.cons[ci].w != 0u) other = v.adj_other[q0 + lane];
-        }
-        const int m = (int)min(32u, en - q0);
-        for (int l = 0; l < m; l++) {  // every lane takes part in every shuffle
-          const uint32_t o = __shfl_sync(FULL, other, l);
-          bonded = bonded | (o == j);
-        }
-      }
-      keep = keep && !bonded;
-    }
+    const bool other = j != (uint32_t)i && j < (uint32_t)v.S;
+    // latticeAdjacent (src/gpu/wgsl.js:409-416) is the 26-neighbourhood, which
+    // is what the constraints tie; isBonded (599-607) asks for an alive one.
+    // The place of j among the neighbours, five halvings:
+    uint32_t at = 0;
+#pragma unroll
+    for (uint32_t h = 16; h > 0; h >>= 1)
+      if (__shfl_sync(FULL, neighbour, (int)(at + h - 1u)) < j) at += h;
+    const bool near = __shfl_sync(FULL, neighbour, (int)at) == j && other;
+    const real lim = near ? lim_near : lim_far;
+    const bool keep = other && !(d2 >= lim * lim) && !(near && (bonds >> at & 1u));
     const unsigned kept = __ballot_sync(FULL, keep);
-    const uint32_t at = cnt + (uint32_t)__popc(kept & ((1u << lane) - 1u));
-    if (keep && at < C_K) v.clist[(size_t)i * C_K + at] = j | (near ? CL_NEAR : 0u);
+    const uint32_t place = cnt + (uint32_t)__popc(kept & ((1u << lane) - 1u));
+    if (keep && place < C_K) v.clist[(size_t)i * C_K + place] = j | (near ? CL_NEAR : 0u);
     cnt = min(cnt + (uint32_t)__popc(kept), C_K);
   }
   if (lane == 0) v.ccount[i] = cnt;
