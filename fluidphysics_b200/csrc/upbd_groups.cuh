@@ -23,11 +23,11 @@
 //
 // An intact or sliced body has a handful of seeds and few crossing
 // constraints, so the sequential part all but vanishes: the work is five
-// parallel passes and one block's replay of the joins (about 0.4 us each).
+// parallel passes and one block's replay of the joins (about 0.3 us each).
 // The passes are chains of a few dependent loads over L2-resident data, and
 // at this size their six launches are most of the time. Replaying every
 // constraint in one warp took 2,806 us on the default body after two cuts
-// (93,556 constraints, B200); this takes 49 us.
+// (93,556 constraints, B200); this takes 37 to 44 us.
 #pragma once
 #include "upbd_device.cuh"
 
@@ -177,37 +177,32 @@ __device__ __forceinline__ int32_t grp_find(int32_t* par, int32_t x) {
 __global__ void __launch_bounds__(GRP_BLOCK) k_groups_join(const uint4* __restrict__ cons, int C, int S, GroupScratch g) {
   __shared__ uint32_t s_warp[GRP_BLOCK / 32];
   __shared__ uint32_t s_total;
+  __shared__ int32_t s_from, s_to;
   const unsigned FULL = 0xffffffffu;
   const int tid = (int)threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) s_total = 0u;
-  __syncthreads();
-  // the crossing constraints as an ascending list
-  const int words = (C + 31) / 32;
-  for (int w0 = 0; w0 < words; w0 += GRP_BLOCK) {
-    const int w = w0 + tid;
-    uint32_t m = (w < words) ? g.bits[w] : 0u;
-    const uint32_t n = (uint32_t)__popc(m);
-    uint32_t x = n;
+  // the crossing constraints as an ascending list: each thread a run of words
+  const int words = (C + 31) / 32, per = (words + GRP_BLOCK - 1) / GRP_BLOCK;
+  const int w0 = tid * per, w1 = min(w0 + per, words);
+  uint32_t n = 0;
+  for (int w = w0; w < w1; w++) n += (uint32_t)__popc(g.bits[w]);
+  uint32_t x = n;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(FULL, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) s_warp[wid] = x;
-    __syncthreads();
-    uint32_t at = s_total + x - n, all = 0;
-    for (int q = 0; q < GRP_BLOCK / 32; q++) {
-      if (q < wid) at += s_warp[q];
-      all += s_warp[q];
-    }
-    while (m) {
-      g.list[at++] = (uint32_t)(w * 32 + __ffs(m) - 1);
-      m &= m - 1u;
-    }
-    __syncthreads();
-    if (tid == 0) s_total += all;
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, x, o);
+    if (lane >= o) x += y;
   }
+  if (lane == 31) s_warp[wid] = x;
+  __syncthreads();
+  uint32_t at = x - n;
+  {
+    const uint32_t mine = s_warp[lane];  // GRP_BLOCK / 32 = 32 warps
+    at += __reduce_add_sync(FULL, lane < wid ? mine : 0u);
+    if (tid == GRP_BLOCK - 1) s_total = at + n;
+  }
+  if (n)
+    for (int w = w0; w < w1; w++)
+      for (uint32_t m = g.bits[w]; m; m &= m - 1u) g.list[at++] = (uint32_t)(w * 32 + __ffs((int)m) - 1);
+  __syncthreads();
   const uint32_t total = s_total;
   // replay: all constraints of a batch look up their parts at once; the first
   // one with two different parts is the next join
@@ -218,14 +213,10 @@ __global__ void __launch_bounds__(GRP_BLOCK) k_groups_join(const uint4* __restri
     int32_t ra = 0, rb = 0;
     if (have) {
       const uint4 k = cons[e];
-      ra = g.tree[k.x];
-      rb = g.tree[k.y];
+      ra = grp_find<true>(g.par, g.tree[k.x]);
+      rb = grp_find<true>(g.par, g.tree[k.y]);
     }
     for (;;) {
-      if (have) {
-        ra = grp_find<true>(g.par, ra);
-        rb = grp_find<true>(g.par, rb);
-      }
       const unsigned diff = __ballot_sync(FULL, have && ra != rb);
       if (lane == 0) s_warp[wid] = diff ? (uint32_t)(wid * 32 + __ffs(diff) - 1) : GRP_NONE;
       __syncthreads();
@@ -240,9 +231,13 @@ __global__ void __launch_bounds__(GRP_BLOCK) k_groups_join(const uint4* __restri
         g.ke[joins] = e;
         g.cur[rb] = node;
         g.par[ra] = rb;
+        s_from = ra;
+        s_to = rb;
       }
       joins++;
       __syncthreads();
+      if (ra == s_from) ra = s_to;  // the other ends now rooted there
+      if (rb == s_from) rb = s_to;
     }
     __syncthreads();
   }
