@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -104,6 +106,7 @@ struct upbd_sim {
   };
   std::map<uint64_t, Graph> graphs;
   uint64_t launches = 0;  // kernels enqueued (graph replays count their nodes)
+  uint32_t pick_calls = 0;
   std::string err;
   // per-kernel timing of an eager frame
   bool prof_on = false;
@@ -859,11 +862,17 @@ int upbd_pick(upbd_sim* s, const double ro[3], const double rd[3], double max_pe
   if (s->v.S > 0) {
     // the blocks' results go to the density pass's list memory (free between substeps)
     const unsigned blocks = std::min(blocks_for(s->v.S), 2u * (unsigned)s->num_sms);
-    k_pick<<<blocks, 256, 0, s->stream>>>(s->v, ray, reinterpret_cast<PickBest*>(s->v.nbr));
+    k_pick<<<blocks, 256, 0, s->stream>>>(s->v, ray, reinterpret_cast<PickBest*>(s->v.nbr), ++s->pick_calls);
     s->launches++;
     UPBD_KCK(s);
-    UPBD_CK(s, cudaStreamSynchronize(s->stream));
+    // the result arrives in mapped memory a few microseconds before the stream
+    // reports; a longer queue, or a fault, is left to the stream
     const volatile uint32_t* hm = s->hmapped;
+    const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+    while (hm[HM_PICK_CALL] != s->pick_calls && std::chrono::steady_clock::now() < until) {
+    }
+    if (hm[HM_PICK_CALL] != s->pick_calls) UPBD_CK(s, cudaStreamSynchronize(s->stream));
+    std::atomic_thread_fence(std::memory_order_acquire);
     bits = (uint64_t)hm[HM_PICK_T] | ((uint64_t)hm[HM_PICK_T + 1] << 32);
     best = hm[HM_PICK_I];
   } else {

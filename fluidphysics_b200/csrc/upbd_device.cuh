@@ -39,6 +39,7 @@ constexpr int HM_ACTIVE = 0;
 constexpr int HM_HEALTH = 1;
 constexpr int HM_PICK_T = 2;  // pick: uint64 bits of the smallest t (words 2-3)
 constexpr int HM_PICK_I = 4;  // and the index there
+constexpr int HM_PICK_CALL = 5;  // number of the pick whose result this is
 constexpr int HM_WORDS = 8;
 
 // Scalar type of the particle state and of the pass arithmetic: float in
