@@ -426,12 +426,13 @@ uint32_t total_blocks(const upbd_batch* b, int d) {
   const uint32_t* pre = (const uint32_t*)(b->h_tab + b->off_prefix);
   return pre[(size_t)d * b->stride + b->scenes.size()];
 }
-// x rounded up to three significant bits: at most an eighth more, and few
-// distinct values for scenes that come and go
+// x rounded up to a power of two: scenes that come and go meet few distinct
+// values, each of which costs a capture once (with three significant bits the
+// served stream's waits at its 99th percentile went from 9 to 47 ms)
 uint32_t quantized(uint32_t x) {
-  uint32_t step = 1;
-  while (x / step >= 16u) step *= 2u;
-  return (x + step - 1u) / step * step;
+  uint32_t p = 1;
+  while (p < x && p < (1u << 31)) p *= 2u;
+  return p;
 }
 
 // The frame's launch sequence (GpuSim.encode's pass order, src/gpu/sim.js:

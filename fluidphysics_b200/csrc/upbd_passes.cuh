@@ -281,7 +281,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
 // places: 128 for large scenes (two to three chunks a warp in a settled pool,
 // so that uneven chunks even out), fewer where that would leave SMs idle.
 // Bound by the latency of the shared loads, square roots and shuffles between
-// its instructions (54 % of the issue slots of an active SM). On the default
+// its instructions (58 % of the issue slots of an active SM). On the default
 // scene's settled pool (65,536 fluid, 120 candidates and 22 listed each; B200,
 // event-timed) a launch takes 29.8 us; a walk of each group of GLF lanes with its
 // own cursor, 46 instructions a candidate, took 42.8 us; on the large scene 121
