@@ -285,12 +285,23 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
 // scene's settled pool (65,536 fluid, 120 candidates and 22 listed each; B200,
 // event-timed) a launch takes 29.8 us; a walk of each group of GLF lanes with its
 // own cursor, 46 instructions a candidate, took 42.8 us; on the large scene 121
-// against 173 us. With half a warp a chunk of 4 it took 40 us (the set-up is
-// shared by half as many), with a warp over 8 consecutive slots of several cells
-// 73 us.
+// against 173 us. With half a warp a chunk of 4 everywhere it took 40 us (the
+// set-up is shared by half as many), with a warp over 8 consecutive slots of
+// several cells 73 us.
+// Where fluid falls apart in drops of one or two particles a cell, a warp a chunk
+// leaves three lanes in four idle and the set-up, some 300 instructions, is
+// paid for two particles. There a warp takes two chunks of up to four, a half
+// each (W = 16): the large scene's first frames of the fall 147 us a warp a
+// chunk, 117 with halves (90 with a cursor a group), the default scene's 48.3
+// and 39.3.
 constexpr uint32_t STAGE = 4096 / sizeof(real4);     // 256 candidates a warp and round (FP64: 128)
 constexpr size_t STAGE_WARP = STAGE * sizeof(real4);  // dynamic shared bytes per warp
 constexpr uint32_t WINDOW_MAX = 128;                  // places of a block's window
+// Halves where fewer than one chunk in SPARSE of a window has more than four
+// particles. At one in two the default scene's settled pool takes 38.5 us instead
+// of 36.6 and the large scene's splash 2069 us a frame instead of 1966; at one in
+// eight and in 32 the fall's frames 6 to 15 take 1379 and 1399 us instead of 1324.
+constexpr uint32_t SPARSE = 4;
 
 __device__ __forceinline__ void copy_row_async(real4* dst, const real4* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -335,58 +346,95 @@ __device__ __forceinline__ int thread_index() {
   return t;
 }
 
-// One round's copies: copy(row, slot) for candidates q0 .. of the sequence whose
-// bucket k starts at place off (lane k) and slot s0 and ends at end, ROWS of them
-// a round (CLIP: where there is more than one).
-template <uint32_t ROWS, bool CLIP, class Copy>
-__device__ __forceinline__ void stage_rows(int L, uint32_t s0, uint32_t off, uint32_t end, uint32_t q0, Copy&& copy) {
+// A warp's W-lane parts (W = 32 or 16) each take a chunk of up to W / GLF
+// particles; a lane looks up buckets l and, with W = 16, l + 16 of its part's 27.
+template <int W>
+struct Buckets {
+  static constexpr int R = (27 + W - 1) / W;
+  uint32_t s0[R], off[R], end[R];  // first slot; the bucket's range of the sequence
+};
+
+// One round's copies: copy(row, slot) for candidates q0 .. of the part's
+// sequence, ROWS of them a round (CLIP: where there is more than one).
+template <int W, uint32_t ROWS, bool CLIP, class Copy>
+__device__ __forceinline__ void stage_rows(int L, const Buckets<W>& b, uint32_t q0, Copy&& copy) {
   const unsigned FULL = 0xffffffffu;
+  constexpr int LB = W / 8;  // lanes a bucket
+  const int l = L & (W - 1);
 #pragma unroll
-  for (int r = 0; r < 4; r++) {  // buckets 8 r + L / 4, rows L mod 4 and every fourth after it
-    const int owner = 8 * r + L / 4;
-    uint32_t o = __shfl_sync(FULL, off, owner), hi = __shfl_sync(FULL, end, owner);
-    const uint32_t sb = __shfl_sync(FULL, s0, owner) - o;
+  for (int r = 0; r < 4; r++) {  // buckets 8 r + l / LB, rows l mod LB and every LB-th after it
+    const int owner = (8 * r + l / LB) & (W - 1), q = 8 * r / W;
+    uint32_t o = __shfl_sync(FULL, b.off[q], owner, W), hi = __shfl_sync(FULL, b.end[q], owner, W);
+    const uint32_t sb = __shfl_sync(FULL, b.s0[q], owner, W) - o;
     if (CLIP) {
       o = max(o, q0);
       hi = min(hi, q0 + ROWS);
     }
-    uint32_t k = o + (uint32_t)(L & 3);
+    uint32_t k = o + (uint32_t)(l & (LB - 1));
     do {
 #pragma unroll
-      for (int m = 0; m < 2; m++, k += 4)
+      for (int m = 0; m < 2; m++, k += LB)
         if (k < hi) copy(CLIP ? k - q0 : k, sb + k);
     } while (__any_sync(FULL, k < hi));
   }
 }
 
 // The chunks that start among the window places from `first` on, listed in
-// s_chunk as (place - first | size << 8); returns how many. Every thread of the
-// block calls it.
+// chunk as (place - first | size << 8); returns how many entries the warps
+// share out. Where most chunks hold one or two particles (a fluid that falls
+// apart in drops) and there are more of them than warps, an entry is a pair of
+// chunks of up to four particles, one to each half of a warp; `halves` is then
+// their number, else 0. Every thread of the block calls it.
 struct ChunkList {
-  uint32_t chunk[WINDOW_MAX], fill[WINDOW_MAX / 32], next;
+  uint32_t chunk[WINDOW_MAX + CHUNK], fill[WINDOW_MAX / 32], next;
 };
 __device__ __forceinline__ uint32_t list_chunks(const SimView& v, ChunkList& s, uint32_t first, uint32_t window,
-                                                uint32_t nact, int tid) {
+                                                uint32_t nact, int tid, uint32_t& halves) {
   const int L = tid & 31, wid = tid >> 5;
   const uint32_t place = first + (uint32_t)tid;
-  uint32_t word = 0, before = 0;
+  uint32_t word = 0, before = 0, more = 0;
   if ((uint32_t)wid * 32u < window) {
     if ((uint32_t)tid < window && place < nact) word = chunk_places(v)[place] >> CHUNK_SHIFT;
-    const unsigned b = __ballot_sync(0xffffffffu, word != 0u);
-    if (L == 0) s.fill[wid] = (uint32_t)__popc(b);
+    const unsigned b = __ballot_sync(0xffffffffu, word != 0u), b4 = __ballot_sync(0xffffffffu, word > CHUNK / 2);
+    // chunks, those over four particles, particles
+    if (L == 0) s.fill[wid] = (uint32_t)__popc(b) | (uint32_t)__popc(b4) << 8;
     before = (uint32_t)__popc(b & ((1u << L) - 1u));
+    more = (uint32_t)__popc(b4 & ((1u << L) - 1u));
   }
   if (tid == 0) s.next = blockDim.x >> 5;
   __syncthreads();
-  uint32_t chunks = 0;
+  uint32_t all = 0, mine = 0;
 #pragma unroll
   for (int w = 0; w < (int)(WINDOW_MAX / 32); w++)
     if ((uint32_t)w * 32u < window) {
-      if (w == wid && word) s.chunk[chunks + before] = (uint32_t)tid | (word << 8);
-      chunks += s.fill[w];
+      if (w == wid) mine = all;
+      all += s.fill[w];
     }
+  const uint32_t chunks = all & 0xffu, big = all >> 8;
+  const bool sp = SPARSE * big < chunks && chunks > blockDim.x >> 5;
+  halves = sp ? chunks + big : 0u;
+  if (word) {
+    const uint32_t at = (mine & 0xffu) + before;
+    if (!sp) {
+      s.chunk[at] = (uint32_t)tid | (word << 8);
+    } else {
+      const uint32_t a = at + (mine >> 8) + more, h = min(word, CHUNK / 2);
+      s.chunk[a] = (uint32_t)tid | (h << 8);
+      if (word > h) s.chunk[a + 1] = ((uint32_t)tid + h) | ((word - h) << 8);
+    }
+  }
   __syncthreads();
-  return chunks;
+  return sp ? (halves + 1) / 2 : chunks;
+}
+// Entry c's chunk for this lane's part of the warp: the slot of group g's
+// particle (0 where it has none) and whether it has one.
+template <int W>
+__device__ __forceinline__ uint32_t chunk_slot(const SimView& v, const ChunkList& s, uint32_t c, int L, uint32_t first,
+                                               uint32_t halves, bool& act) {
+  const uint32_t k = (W == 32) ? c : 2 * c + (uint32_t)L / W, g = (uint32_t)(L & (W - 1)) / GLF;
+  const uint32_t d = (W == 32 || k < halves) ? s.chunk[k] : 0u;
+  act = g < (d >> 8);
+  return act ? (chunk_places(v)[first + (d & 0xffu) + g] & CHUNK_SLOT) : 0u;
 }
 // the warp's next chunk after c
 __device__ __forceinline__ uint32_t next_chunk(ChunkList& s, uint32_t c, int L) {
@@ -394,8 +442,9 @@ __device__ __forceinline__ uint32_t next_chunk(ChunkList& s, uint32_t c, int L) 
   return __shfl_sync(0xffffffffu, c, 0);
 }
 
-// Lanes (all four of a group) whose particle lies in the cell of the group
-// that starts at lane ll; ca: the lane's cell coordinate (x, y, z, z).
+// Of the part's lanes: those (all four of a group) whose particle lies in the
+// cell of the group that starts at lane ll; ca: the lane's cell coordinate (x, y, z, z).
+template <int W>
 __device__ __forceinline__ unsigned same_cell(double ca, int ll, int lane) {
   const unsigned FULL = 0xffffffffu;
   const bool other = !(ca == __shfl_sync(FULL, ca, ll + lane));
@@ -404,39 +453,76 @@ __device__ __forceinline__ unsigned same_cell(double ca, int ll, int lane) {
   return (turn * 15u) | (15u << ll);
 }
 
-// Bucket L (of 27) of the cells around that group's, CellHash::init's values.
-__device__ __forceinline__ uint32_t turn_bucket(double ca, int ll, int L, uint32_t mask) {
-  const unsigned FULL = 0xffffffffu;
-  const int axis = (L < 9) ? L / 3 : 2;  // lane j < 9: component j, axis j / 3, cell offset j % 3 - 1
-  const double cl = __shfl_sync(FULL, ca, ll + axis);
-  const double K = (axis == 0) ? 92837111.0 : ((axis == 1) ? 689287499.0 : 283923481.0);
-  const int32_t comp = js_toint32(__dmul_rn(__dadd_rn(cl, (double)(L - 3 * axis - 1)), K));
-  const int ka = L / 9, kb = (L - 9 * ka) / 3, kc = L - 9 * ka - 3 * kb;
-  return (uint32_t)(__shfl_sync(FULL, comp, ka) ^ __shfl_sync(FULL, comp, 3 + kb) ^ __shfl_sync(FULL, comp, 6 + kc)) & mask;
-}
-
-// inclusive scan over the warp
-__device__ __forceinline__ uint32_t warp_scan(uint32_t x, int L) {
+// inclusive scan over the W lanes of a part
+template <int W>
+__device__ __forceinline__ uint32_t part_scan(uint32_t x, int L) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (L >= o) x += y;
+  for (int o = 1; o < W; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o, W);
+    if ((L & (W - 1)) >= o) x += y;
   }
   return x;
 }
 
-// window <= min(WINDOW_MAX, blockDim), at most 256 threads a block.
-__device__ __forceinline__ void b_density(const SimView& v, const DevParams* __restrict__ P, uint32_t window,
-                                          uint32_t vb) {
-  extern __shared__ __align__(16) unsigned char s_stage[];
-  __shared__ ChunkList s_list;
+// The fluid of the 27 cells around that group's (CellHash::init's buckets);
+// each(length, bucket) sees them; none where the part has no work. Returns the
+// sequence's length.
+template <int W, class Each>
+__device__ __forceinline__ uint32_t part_buckets(const SimView& v, double ca, int ll, int L, bool work, Buckets<W>& b,
+                                                 Each&& each) {
   const unsigned FULL = 0xffffffffu;
-  const int tid = thread_index();
-  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1), g = L / GLF;
-  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
-  if (first >= nact) return;
-  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid);
-  real4* __restrict__ sx = reinterpret_cast<real4*>(s_stage + wid * STAGE_WARP);
+  const int l = L & (W - 1);
+  const int axis = (l < 9) ? l / 3 : 2;  // lane j < 9: component j, axis j / 3, cell offset j % 3 - 1
+  const double cl = __shfl_sync(FULL, ca, ll + axis);
+  const double K = (axis == 0) ? 92837111.0 : ((axis == 1) ? 689287499.0 : 283923481.0);
+  const int32_t comp = js_toint32(__dmul_rn(__dadd_rn(cl, (double)(l - 3 * axis - 1)), K));
+  const uint32_t mask = (uint32_t)v.T - 1u;
+  uint32_t n[Buckets<W>::R];
+#pragma unroll
+  for (int r = 0; r < Buckets<W>::R; r++) {
+    const int k = l + W * r;
+    const int ka = k / 9, kb = (k - 9 * ka) / 3, kc = k - 9 * ka - 3 * kb;
+    const uint32_t hb = (uint32_t)(__shfl_sync(FULL, comp, ka, W) ^ __shfl_sync(FULL, comp, 3 + kb, W) ^
+                                   __shfl_sync(FULL, comp, 6 + kc, W)) & mask;
+    b.s0[r] = 0;
+    n[r] = 0;
+    if (k < 27 && (W == 32 || work)) {
+      const uint2 q = bucket_range<0>(v, hb);
+      b.s0[r] = q.x;
+      n[r] = q.y;
+      each(q.y, hb);
+    }
+  }
+  uint32_t total = 0;
+#pragma unroll
+  for (int r = 0; r < Buckets<W>::R; r++) {
+    b.end[r] = total + part_scan<W>(n[r], L);  // in cell order
+    b.off[r] = b.end[r] - n[r];
+    total = __shfl_sync(FULL, b.end[r], W - 1, W);
+  }
+  return total;
+}
+template <int W>
+__device__ __forceinline__ uint32_t longest(uint32_t total) {
+  return W == 32 ? total : max(total, __shfl_xor_sync(0xffffffffu, total, 16));
+}
+template <int W>
+__device__ __forceinline__ bool parts_left(unsigned rem) {
+  return W == 32 ? rem != 0u : __any_sync(0xffffffffu, rem != 0u);
+}
+// the lane's part
+template <int W>
+__device__ __forceinline__ unsigned part_lanes(int L) {
+  return W == 32 ? 0xffffffffu : ((1u << (W & 31)) - 1u) << (L & ~(W - 1));
+}
+
+template <int W>
+__device__ __forceinline__ void density_chunks(const SimView& v, const DevParams* __restrict__ P, ChunkList& s_list,
+                                               real4* sx, uint32_t first, uint32_t chunks, uint32_t halves, int tid) {
+  const unsigned FULL = 0xffffffffu;
+  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1);
+  constexpr uint32_t ROWS = STAGE * W / 32;
+  sx += (L / W) * ROWS;
   const double inv = P->inv_cell;
   const real H = P->fluid_h, H2 = H * H;
   const real HS = H * (1.0f + XSKIN), HS2 = HS * HS;  // list radius (for xsph)
@@ -445,9 +531,8 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
   const real invH = 1.0f / H;
 #endif
   for (uint32_t c = (uint32_t)wid; c < chunks; c = next_chunk(s_list, c, L)) {
-    const uint32_t d = s_list.chunk[c];
-    const bool act = (uint32_t)g < (d >> 8);
-    const uint32_t myslot = act ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
+    bool act;
+    const uint32_t myslot = chunk_slot<W>(v, s_list, c, L, first, halves, act);
     const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
     const real mass = slot_mass(v)[myslot];
     // lane l's c-th listed candidate goes to row l*NL + c, column myslot
@@ -455,31 +540,26 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
     uint32_t cnt = 0;
     real rho = 0.f, rhoNear = 0.f;
     const double ca = floor(__dmul_rn((double)(lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z)), inv));
-    unsigned rem = __ballot_sync(FULL, act);  // particles whose cell has not had its turn
+    unsigned rem = __ballot_sync(FULL, act) & part_lanes<W>(L);  // the part's particles whose cell has not had its turn
     do {
       // the first remaining particle and those of its cell
-      const int ll = __ffs((int)rem) - 1;
-      const unsigned turn = same_cell(ca, ll, lane) & rem;
+      const bool work = W == 32 || rem != 0u;
+      const int ll = work ? __ffs((int)rem) - 1 : L & ~(W - 1);
+      const unsigned turn = same_cell<W>(ca, ll, lane) & rem;
       rem &= ~turn;
-      const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
-      uint32_t s0 = 0, n = 0;
-      if (L < 27) {
-        const uint2 r = bucket_range<0>(v, hb);
-        s0 = r.x;
-        n = r.y;
-      }
-      const uint32_t end = warp_scan(n, L);  // in cell order
-      const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
-      for (uint32_t q0 = 0; q0 < total; q0 += STAGE) {
+      Buckets<W> b;
+      const uint32_t total = part_buckets<W>(v, ca, ll, L, work, b, [](uint32_t, uint32_t) {});
+      const uint32_t most = longest<W>(total);
+      for (uint32_t q0 = 0; q0 < most; q0 += ROWS) {
         auto copy = [&](uint32_t k, uint32_t e) {
           if (UPBD_IDX_OK(v, e, NS)) copy_row_async(&sx[k], &v.spos[e]);
           else sx[k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never listed (reported)
         };
-        if (total <= STAGE) stage_rows<STAGE, false>(L, s0, off, end, 0u, copy);
-        else stage_rows<STAGE, true>(L, s0, off, end, q0, copy);
+        if (most <= ROWS) stage_rows<W, ROWS, false>(L, b, 0u, copy);
+        else stage_rows<W, ROWS, true>(L, b, q0, copy);
         copy_rows_wait();
         __syncwarp();
-        const uint32_t len = min(total - q0, STAGE);
+        const uint32_t len = (W == 32 || q0 < total) ? min(total - q0, ROWS) : 0u;
         const uint32_t mine = (turn >> L & 1u) ? (len + (GLF - 1) - lane) / GLF : 0u;  // this lane's share
         const real4* __restrict__ row = sx + lane;
         for (uint32_t u0 = 0; u0 * GLF < len; u0 += 32, row += 32 * GLF) {
@@ -542,7 +622,7 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
         }
         __syncwarp();  // the next round rewrites the rows
       }
-    } while (rem);
+    } while (parts_left<W>(rem));
     if (act) v.ncount[lane * NS + myslot] = cnt;
     rho = lane_sum<GLF>(rho);
     rhoNear = lane_sum<GLF>(rhoNear);
@@ -551,6 +631,21 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
       store_row_pair(&v.drow[2 * (size_t)myslot], pi, make_real4(rho, rhoNear, mass, 0.f));
     }
   }
+}
+
+// window <= min(WINDOW_MAX, blockDim), at most 256 threads a block.
+__device__ __forceinline__ void b_density(const SimView& v, const DevParams* __restrict__ P, uint32_t window,
+                                          uint32_t vb) {
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  __shared__ ChunkList s_list;
+  const int tid = thread_index();
+  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  if (first >= nact) return;
+  uint32_t halves;
+  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid, halves);
+  real4* sx = reinterpret_cast<real4*>(s_stage + (tid >> 5) * STAGE_WARP);
+  if (halves) density_chunks<16>(v, P, s_list, sx, first, chunks, halves, tid);
+  else density_chunks<32>(v, P, s_list, sx, first, chunks, halves, tid);
 }
 
 // Contact marks (mark_fluid_near below) find a fluid particle from the
@@ -1527,20 +1622,18 @@ __device__ __forceinline__ void b_solid_visc_apply(const SimView& v, uint32_t vb
 // in a launch of its own beside the list readers, the default scene's settled
 // pool took 31.5 us (both forms in one launch, B200, event-timed), the large
 // scene's splash 115, a batch of 48 scenes 283; now 23.0, 88 and 228. Position and
-// velocity come as one 32-byte row: with two 16-byte rows 25.7, 103 us.
+// velocity come as one 32-byte row: with two 16-byte rows 25.7, 103 us. Windows of
+// small chunks go by half-warps as in the density pass: in the large scene's fall
+// 68.7 us, a warp a chunk 90.8.
 constexpr uint32_t XROWS = STAGE / 2;  // candidates staged a round: positions and velocities in the same bytes
 constexpr int XCH = 4;                 // list entries whose loads are in flight together
-template <bool APPLY>
-__device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __restrict__ P, uint32_t window, uint32_t vb) {
-  extern __shared__ __align__(16) unsigned char s_stage[];
-  __shared__ ChunkList s_list;
+template <bool APPLY, int W>
+__device__ __forceinline__ void xsph_chunks(const SimView& v, const DevParams* __restrict__ P, ChunkList& s_list,
+                                            real4* sx, uint32_t first, uint32_t chunks, uint32_t halves, int tid) {
   const unsigned FULL = 0xffffffffu;
-  const int tid = thread_index();
-  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1), g = L / GLF;
-  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
-  if (first >= nact) return;
-  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid);
-  real4* __restrict__ sx = reinterpret_cast<real4*>(s_stage + wid * STAGE_WARP);
+  const int L = tid & 31, wid = tid >> 5, lane = L & (GLF - 1);
+  constexpr uint32_t ROWS = XROWS * W / 32;
+  sx += (L / W) * ROWS;
   real4* __restrict__ sv = sx + XROWS;
   const double inv = P->inv_cell;
   const real H = P->fluid_h, H2 = H * H;
@@ -1549,9 +1642,8 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
   const real allow = xsph_allowance(P), rec = XMOVE_REC * allow;
   const real scene = r_fmax(rec, (real)__uint_as_float(v.scratch[SCR_XMOVE]));
   for (uint32_t c = (uint32_t)wid; c < chunks; c = next_chunk(s_list, c, L)) {
-    const uint32_t d = s_list.chunk[c];
-    const bool mem = (uint32_t)g < (d >> 8);
-    const uint32_t myslot = mem ? (chunk_places(v)[first + (d & 0xffu) + (uint32_t)g] & CHUNK_SLOT) : 0u;
+    bool mem;
+    const uint32_t myslot = chunk_slot<W>(v, s_list, c, L, first, halves, mem);
     const uint32_t i = v.entries[myslot];
     const real4 pi = rows[2 * (size_t)myslot];
     const real sm = v.smove[myslot];
@@ -1567,28 +1659,31 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
     real sx_ = 0.f, sy_ = 0.f, sz_ = 0.f, m = 0.f;
     unsigned rem = __ballot_sync(FULL, act && !listed);
     if (rem) {
+      rem &= part_lanes<W>(L);
       const double ca = floor(__dmul_rn((double)(lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z)), inv));
       do {
-        const int ll = __ffs((int)rem) - 1;
-        const unsigned turn = same_cell(ca, ll, lane) & rem;
+        const bool work = W == 32 || rem != 0u;
+      const int ll = work ? __ffs((int)rem) - 1 : L & ~(W - 1);
+        const unsigned turn = same_cell<W>(ca, ll, lane) & rem;
         rem &= ~turn;
         const bool mine_turn = (turn >> L & 1u) != 0u;
-        const uint32_t hb = turn_bucket(ca, ll, L, (uint32_t)v.T - 1u);
-        uint32_t s0 = 0, n = 0, bm = 0;  // the bucket's fluid; a finite distance or +inf
-        if (L < 27) {
-          const uint2 r = bucket_range<0>(v, hb);
-          s0 = r.x;
-          n = r.y;
-          bm = v.bmove[hb];
-          if (n == 0u) bm = 0u;
+        uint32_t bm = 0;  // the buckets' fluid: a finite distance or +inf
+        Buckets<W> b;
+        const uint32_t total = part_buckets<W>(v, ca, ll, L, work, b, [&](uint32_t n, uint32_t hb) {
+          const uint32_t moved = v.bmove[hb];
+          if (n) bm = max(bm, moved);
+        });
+        const uint32_t most = longest<W>(total);
+        if (W == 32) {
+          bm = __reduce_max_sync(FULL, bm);
+        } else {
+#pragma unroll
+          for (int o = 1; o < W; o <<= 1) bm = max(bm, __shfl_xor_sync(FULL, bm, o));
         }
-        bm = __reduce_max_sync(FULL, bm);
         if (mine_turn) listed = !over && sm + r_fmax(rec, (real)__uint_as_float(bm)) <= allow;
         const bool walks = mine_turn && !listed;
         if (!__any_sync(FULL, walks)) continue;
-        const uint32_t end = warp_scan(n, L);  // in cell order
-        const uint32_t total = __shfl_sync(FULL, end, 31), off = end - n;
-        for (uint32_t q0 = 0; q0 < total; q0 += XROWS) {
+        for (uint32_t q0 = 0; q0 < most; q0 += ROWS) {
           auto copy = [&](uint32_t k, uint32_t e) {
             if (UPBD_IDX_OK(v, e, NS)) {
               copy_row_async(&sx[k], &rows[2 * (size_t)e]);
@@ -1597,11 +1692,11 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
               sx[k] = make_real4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);  // never in range (reported)
             }
           };
-          if (total <= XROWS) stage_rows<XROWS, false>(L, s0, off, end, 0u, copy);
-          else stage_rows<XROWS, true>(L, s0, off, end, q0, copy);
+          if (most <= ROWS) stage_rows<W, ROWS, false>(L, b, 0u, copy);
+          else stage_rows<W, ROWS, true>(L, b, q0, copy);
           copy_rows_wait();
           __syncwarp();
-          const uint32_t len = min(total - q0, XROWS);
+          const uint32_t len = (W == 32 || q0 < total) ? min(total - q0, ROWS) : 0u;
           const uint32_t own = walks ? (len + (GLF - 1) - lane) / GLF : 0u;  // this lane's share, at most 32
           const uint32_t steps = (len + (GLF - 1)) / GLF;
           uint32_t bits = 0;  // within H, the first candidate's bit on top
@@ -1625,7 +1720,7 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
           }
           __syncwarp();  // the next round rewrites the rows
         }
-      } while (rem);
+      } while (parts_left<W>(rem));
     }
     if (listed) {
       const uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
@@ -1666,6 +1761,19 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
         v.delta[i] = make_real4(vx, vy, vz, m);
     }
   }
+}
+template <bool APPLY>
+__device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __restrict__ P, uint32_t window, uint32_t vb) {
+  extern __shared__ __align__(16) unsigned char s_stage[];
+  __shared__ ChunkList s_list;
+  const int tid = thread_index();
+  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  if (first >= nact) return;
+  uint32_t halves;
+  const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid, halves);
+  real4* sx = reinterpret_cast<real4*>(s_stage + (tid >> 5) * STAGE_WARP);
+  if (halves) xsph_chunks<APPLY, 16>(v, P, s_list, sx, first, chunks, halves, tid);
+  else xsph_chunks<APPLY, 32>(v, P, s_list, sx, first, chunks, halves, tid);
 }
 
 // countActive (src/gpu/wgsl.js:874-879) with a last-block epilogue that
