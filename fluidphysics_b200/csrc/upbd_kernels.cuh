@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256) k_cut_tets(SimView v, const DevParams* __
 // into mapped host memory. The call is all latency: with the ray copied to the
 // uniform block, a memset, two launches (smallest t, then lowest index) and a
 // copy back it took 29.3 us on 8,000 solids (B200, host clock, through the Python
-// mirror), this takes 17.1: the host watches the call's number arrive instead of
+// mirror), this takes 16.2: the host watches the call's number arrive instead of
 // waiting for the stream (18.7).
 struct PickRay {
   double o[3], d[3], max_perp;
