@@ -33,6 +33,7 @@ constexpr int SCR_ACTIVE = 4;      // active-fluid partial sums
 constexpr int SCR_DONE = 5;        // blocks finished (last-block pattern)
 constexpr int SCR_HEALTH = 6;      // UPBD_HEALTH_* bits
 constexpr int SCR_XMOVE = 7;       // largest movement the bounds pass recorded this substep (float bits)
+constexpr int SCR_FAR = 8;         // a fluid particle is not within FAR of the origin in this substep's grid
 constexpr int SCR_WORDS = 16;
 // mapped host words
 constexpr int HM_ACTIVE = 0;
@@ -271,6 +272,8 @@ constexpr uint32_t CL_NEAR = 0x80000000u;  // contact cache entry flag: a lattic
 constexpr float XSKIN = 0.05f;
 constexpr float XMOVE_FRAC = 0.9f;
 constexpr float XMOVE_REC = 0.25f;
+// Within FAR of the origin (each coordinate) no squared distance overflows.
+constexpr float FAR = 1e18f;
 constexpr uint32_t NBR_IN = 0x80000000u;  // list entry flag: within H at density time (slots stay below 2^31)
 
 template <int G = GL>

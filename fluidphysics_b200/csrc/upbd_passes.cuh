@@ -171,7 +171,10 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
     }
   }
   if (vb == (uint32_t)v.num_tiles - 1u && tid == SCAN_THREADS - 1) v.start[v.T] = run + sum;
-  if (vb == 0 && tid == 0 && v.bmove) v.scratch[SCR_XMOVE] = 0u;
+  if (vb == 0 && tid == 0 && v.bmove) {
+    v.scratch[SCR_XMOVE] = 0u;
+    v.scratch[SCR_FAR] = 0u;
+  }
 }
 
 // Scatter by ticket (gridScatter, src/gpu/wgsl.js:238-245, without its
@@ -249,6 +252,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
     const uint32_t n = (rank_in % CHUNK == 0u) ? min(CHUNK, mates - rank_in) : 0u;
     chunk_places(v)[s + before + rank_in] = slot | (n << CHUNK_SHIFT);
     slot_mass(v)[slot] = p.w;
+    if (!(r_fabs(p.x) <= FAR && r_fabs(p.y) <= FAR && r_fabs(p.z) <= FAR)) v.scratch[SCR_FAR] = 1u;
     p.w = slot_pack(real(0), slot);
   } else {
     chunk_places(v)[slot] = 0u;  // solids follow the fluid: no chunk starts there
@@ -332,8 +336,10 @@ __device__ __forceinline__ real dist2_xy(real ex, real ey, real ez) {
 
 // bits << 1, plus 1 where d2 is below lim (the parity build: not at or above)
 __device__ __forceinline__ uint32_t push_listed(uint32_t bits, real d2, real lim) {
-#if defined(UPBD_PARITY_BUILD) || defined(UPBD_FP64_BUILD)
+#if defined(UPBD_PARITY_BUILD)
   return (bits << 1) | (d2 >= lim ? 0u : 1u);
+#elif defined(UPBD_FP64_BUILD)
+  return (bits << 1) | (d2 < lim ? 1u : 0u);
 #else
   return __funnelshift_l(__float_as_uint(d2 - lim), bits, 1);  // the sign of the difference (a NaN's is clear)
 #endif
@@ -529,6 +535,7 @@ __device__ __forceinline__ void density_chunks(const SimView& v, const DevParams
   const uint32_t NS = (uint32_t)v.N;
 #ifndef UPBD_PARITY_BUILD
   const real invH = 1.0f / H;
+  const bool far = v.scratch[SCR_FAR] != 0u || !(r_fabs(invH) <= 3.0e38f);
 #endif
   for (uint32_t c = (uint32_t)wid; c < chunks; c = next_chunk(s_list, c, L)) {
     bool act;
@@ -620,6 +627,17 @@ __device__ __forceinline__ void density_chunks(const SimView& v, const DevParams
 #endif
           }
         }
+#ifndef UPBD_PARITY_BUILD
+        // a candidate at no finite distance is not listed, but leaves the near
+        // density NaN: it adds 0 times its q, as every candidate out of range
+        // does in exact terms
+        if (far)
+          for (uint32_t u = 0; u < mine; u++) {
+            const real4 pj = sx[lane + u * GLF];
+            const real d2 = dist2(pj.x - pi.x, pj.y - pi.y, pj.z - pi.z);
+            rhoNear = r_fma(real(0.0f), r_fma(-approx_sqrt(d2), invH, real(1.0f)), rhoNear);
+          }
+#endif
         __syncwarp();  // the next round rewrites the rows
       }
     } while (parts_left<W>(rem));
