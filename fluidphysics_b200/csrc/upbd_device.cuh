@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "upbd_grid_layout.h"
+#include "upbd_index.h"
 
 namespace upbd {
 
@@ -247,13 +248,7 @@ __device__ __forceinline__ bool idx_ok(uint32_t* scratch, uint64_t idx, uint64_t
 // GL = 8 lanes; the fluid-fluid gathers (density, xsph) GLF = 4: each lane
 // walks the whole 27-cell sequence, so fewer lanes per particle cross fewer
 // cell boundaries in all.
-constexpr int GL = 8;
-constexpr int GLF = 4;
-constexpr uint32_t NL = 28;  // density-pass neighbour-list entries kept per fluid lane (GLF * NL per particle)
-constexpr int DL = 2;        // threads per particle in the displacement pass
-constexpr uint32_t CHUNK = 32 / GLF;  // fluid particles of one cell that a warp takes in the density pass
-constexpr int CHUNK_SHIFT = 28;       // chunk place: slot, above it the size of the chunk that starts there
-constexpr uint32_t CHUNK_SLOT = (1u << CHUNK_SHIFT) - 1u;  // a scene of 2^28 slots would need 240 GB
+// (GL, GLF, DL and the lists' and chunks' sizes: upbd_index.h.)
 constexpr int GT = 16;       // lanes per solid in the tet solve (32 for small bodies)
 constexpr uint32_t CL_NEAR = 0x80000000u;  // contact cache entry flag: a lattice neighbour (solids stay below 2^31)
 
@@ -480,6 +475,11 @@ __device__ __forceinline__ uint32_t* cell_keys(const SimView& v) { return reinte
 __device__ __forceinline__ uint2* bucket_pairs(const SimView& v) { return reinterpret_cast<uint2*>(v.pvrow); }
 __device__ __forceinline__ real* slot_mass(const SimView& v) { return reinterpret_cast<real*>(bucket_pairs(v) + v.N); }
 __device__ __forceinline__ uint32_t* chunk_places(const SimView& v) { return v.tmp; }
+
+// entry of a lane's list at `row`, from the column's first row
+__device__ __forceinline__ uint32_t* list_entry(uint32_t* column, uint32_t row, uint32_t slots) {
+  return reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(column) + list_row_bytes(row, slots));
+}
 
 // std::max / std::min / clamp with the operand order of the oracle (so -0.0
 // and NaN resolve the same way on both sides).

@@ -206,7 +206,7 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
 // one bucket of seven in a settled pool, would need candidates of their own).
 // Inside a bucket the fluid's slots are listed by (cell key, slot) at the
 // bucket's places of chunk_places, the first of each chunk with the chunk's
-// size in the bits above CHUNK_SHIFT. The slot copy of a fluid particle carries
+// size (chunk_word). The slot copy of a fluid particle carries
 // its slot where the mass would be, for the density pass's lists; the mass goes
 // to slot_mass.
 __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
@@ -250,7 +250,8 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   }
   if (i >= v.S) {
     const uint32_t n = (rank_in % CHUNK == 0u) ? min(CHUNK, mates - rank_in) : 0u;
-    chunk_places(v)[s + before + rank_in] = slot | (n << CHUNK_SHIFT);
+    const uint32_t place = s + before + rank_in;
+    chunk_places(v)[place] = chunk_word(place, slot, n);
     slot_mass(v)[slot] = p.w;
     if (!(r_fabs(p.x) <= FAR && r_fabs(p.y) <= FAR && r_fabs(p.z) <= FAR)) v.scratch[SCR_FAR] = 1u;
     p.w = slot_pack(real(0), slot);
@@ -400,7 +401,7 @@ __device__ __forceinline__ uint32_t list_chunks(const SimView& v, ChunkList& s, 
   const uint32_t place = first + (uint32_t)tid;
   uint32_t word = 0, before = 0, more = 0;
   if ((uint32_t)wid * 32u < window) {
-    if ((uint32_t)tid < window && place < nact) word = chunk_places(v)[place] >> CHUNK_SHIFT;
+    if ((uint32_t)tid < window && place < nact) word = chunk_word_size(chunk_places(v)[place]);
     const unsigned b = __ballot_sync(0xffffffffu, word != 0u), b4 = __ballot_sync(0xffffffffu, word > CHUNK / 2);
     // chunks, those over four particles, particles
     if (L == 0) s.fill[wid] = (uint32_t)__popc(b) | (uint32_t)__popc(b4) << 8;
@@ -440,7 +441,8 @@ __device__ __forceinline__ uint32_t chunk_slot(const SimView& v, const ChunkList
   const uint32_t k = (W == 32) ? c : 2 * c + (uint32_t)L / W, g = (uint32_t)(L & (W - 1)) / GLF;
   const uint32_t d = (W == 32 || k < halves) ? s.chunk[k] : 0u;
   act = g < (d >> 8);
-  return act ? (chunk_places(v)[first + (d & 0xffu) + g] & CHUNK_SLOT) : 0u;
+  const uint32_t place = first + (d & 0xffu) + g;
+  return act ? chunk_word_slot(place, chunk_places(v)[place]) : 0u;
 }
 // the warp's next chunk after c
 __device__ __forceinline__ uint32_t next_chunk(ChunkList& s, uint32_t c, int L) {
@@ -543,7 +545,7 @@ __device__ __forceinline__ void density_chunks(const SimView& v, const DevParams
     const real4 pi = act ? v.spos[myslot] : make_real4(0.f, 0.f, 0.f, 0.f);
     const real mass = slot_mass(v)[myslot];
     // lane l's c-th listed candidate goes to row l*NL + c, column myslot
-    uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
+    uint32_t* nbr = list_entry(v.nbr + myslot, lane * NL, NS);
     uint32_t cnt = 0;
     real rho = 0.f, rhoNear = 0.f;
     const double ca = floor(__dmul_rn((double)(lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z)), inv));
@@ -599,11 +601,11 @@ __device__ __forceinline__ void density_chunks(const SimView& v, const DevParams
             const bool use0 = e0 != myslot, use1 = two && e1 != myslot;
             const bool in0 = d0 < H2, in1 = d1 < H2;
             if (use0) {
-              if (cnt < NL) nbr[cnt * NS] = e0 | (in0 ? NBR_IN : 0u);  // for fluidDisp (same positions) and xsph
+              if (cnt < NL) *list_entry(nbr, cnt, NS) = e0 | (in0 ? NBR_IN : 0u);  // for fluidDisp (same positions) and xsph
               cnt++;
             }
             if (use1) {
-              if (cnt < NL) nbr[cnt * NS] = e1 | (in1 ? NBR_IN : 0u);
+              if (cnt < NL) *list_entry(nbr, cnt, NS) = e1 | (in1 ? NBR_IN : 0u);
               cnt++;
             }
 #ifdef UPBD_PARITY_BUILD
@@ -756,7 +758,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
 #pragma unroll
     for (int u = 0; u < LPT; u++) over = over || cnt[u] > NL;
     if (!over) {
-      const uint32_t* __restrict__ nbr = v.nbr + e0;
+      uint32_t* const nbr = v.nbr + e0;
 #pragma unroll
       for (int u = 0; u < LPT; u++) {
         // four entries at a time: their list, position and density loads are
@@ -768,7 +770,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
           for (int w = 0; w < 4; w++) {
             // entries beyond H (listed for xsph) and past the count become the
             // own slot, which pair() skips (d2 = 0)
-            const uint32_t r = (c + w < cnt[u]) ? __ldg(&nbr[((uint32_t)(l0 + u) * NL + c + w) * NS]) : e0;
+            const uint32_t r = (c + w < cnt[u]) ? __ldg(list_entry(nbr, (uint32_t)(l0 + u) * NL + c + w, NS)) : e0;
             e[w] = (r & NBR_IN) ? (r & ~NBR_IN) : e0;
             if (!UPBD_IDX_OK(v, e[w], NS)) e[w] = e0;  // out of range: the own slot (skipped, reported)
           }
@@ -1422,16 +1424,17 @@ __device__ __forceinline__ void contacts_lane(const SimView& v, const DevParams*
 // start on a warp boundary and whole warps reach lane_sum's shuffles.
 __device__ __forceinline__ void b_bond_contacts(const SimView& v, const DevParams* __restrict__ P,
                                                        int nb, int nt, int nb_pad, int nc, uint32_t vb) {
-  const int t = UPBD_VTID;
-  if (t < nb_pad) {
-    if (t < nb)
-      bond_update(v, P, t);
-    else if (t < nb + nt)
-      tet_update(v, P, t - nb);
+  // by groups of GL threads: the threads themselves pass 2^31 from 2^28 particles on
+  const uint32_t group = vb * (blockDim.x / GL) + threadIdx.x / GL, first = (uint32_t)nb_pad / GL;
+  if (group < first) {
+    const int k = (int)(group * GL + (threadIdx.x & (GL - 1)));
+    if (k < nb)
+      bond_update(v, P, k);
+    else if (k < nb + nt)
+      tet_update(v, P, k - nb);
     return;
   }
-  const int c = t - nb_pad;
-  contacts_lane(v, P, c / GL, c & (GL - 1), nc);
+  contacts_lane(v, P, (int)(group - first), (int)(threadIdx.x & (GL - 1)), nc);
 }
 
 // -------------------------------- apply + bounds + velocity (per particle)
@@ -1741,13 +1744,13 @@ __device__ __forceinline__ void xsph_chunks(const SimView& v, const DevParams* _
       } while (parts_left<W>(rem));
     }
     if (listed) {
-      const uint32_t* __restrict__ nbr = v.nbr + (size_t)lane * NL * NS + myslot;
+      uint32_t* const nbr = list_entry(v.nbr + myslot, lane * NL, NS);
       for (uint32_t k = 0; k < cnt; k += XCH) {
         uint32_t e[XCH];
         real4 p[XCH], w[XCH];
 #pragma unroll
         for (int q = 0; q < XCH; q++) {
-          e[q] = (k + q < cnt) ? (__ldg(&nbr[(k + q) * NS]) & ~NBR_IN) : myslot;
+          e[q] = (k + q < cnt) ? (__ldg(list_entry(nbr, k + q, NS)) & ~NBR_IN) : myslot;
           if (!UPBD_IDX_OK(v, e[q], NS)) e[q] = myslot;  // out of range: the own slot (skipped, reported)
         }
 #pragma unroll

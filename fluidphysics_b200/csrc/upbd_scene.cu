@@ -475,7 +475,7 @@ const char* check_desc(const upbd_scene_desc* d, const upbd_params* p) {
   if (!(p->cell_size > 0)) return "cell_size must be > 0";
   const long long total = (long long)d->solid_dim * d->solid_dim * d->solid_dim +
                           (long long)d->solid_dim2 * d->solid_dim2 * d->solid_dim2 + d->max_fluid;
-  if (total < 1 || total > (1ll << 29)) return "particle count out of range";
+  if (total < 1 || total > MAX_PARTICLES) return "particle count out of range";
   return nullptr;
 }
 
