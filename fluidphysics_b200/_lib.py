@@ -85,7 +85,7 @@ class BatchInfo(C.Structure):
         ("scenes", C.c_int32), ("max_scenes", C.c_int32), ("particles", C.c_int64), ("solids", C.c_int64),
         ("bytes_in_use", C.c_uint64), ("bytes_reserved", C.c_uint64), ("hbm_budget", C.c_uint64),
         ("frames", C.c_uint64), ("launches", C.c_uint64), ("block_threads", C.c_int32),
-        ("ctas_per_sm", C.c_int32), ("num_sms", C.c_int32), ("reserved0", C.c_int32),
+        ("ctas_per_sm", C.c_int32), ("num_sms", C.c_int32), ("captures", C.c_int32),
         ("reserved", C.c_int32 * 8),
     ]
 

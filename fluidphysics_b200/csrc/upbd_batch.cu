@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -300,6 +301,8 @@ struct ProfRec {
 
 thread_local std::string g_batch_error;
 
+using Grids = std::array<uint32_t, NUM_DOMAINS>;  // CTAs of a launch over each domain
+
 }  // namespace
 
 struct upbd_batch {
@@ -327,9 +330,11 @@ struct upbd_batch {
   struct Graph {
     cudaGraphExec_t exec;
     uint64_t kernels;
+    Grids grids;  // what it was captured with
   };
   std::map<uint64_t, Graph> graphs;
   uint64_t launches = 0, frames = 0;
+  int32_t captures = 0;
   std::string err;
   bool prof_on = false;
   std::vector<ProfRec> prof;
@@ -427,7 +432,7 @@ uint32_t total_blocks(const upbd_batch* b, int d) {
   return pre[(size_t)d * b->stride + b->scenes.size()];
 }
 // x rounded up to a power of two: scenes that come and go meet few distinct
-// values, each of which costs a capture once (with three significant bits the
+// values, each of which may cost a capture (with three significant bits the
 // served stream's waits at its 99th percentile went from 9 to 47 ms)
 uint32_t quantized(uint32_t x) {
   uint32_t p = 1;
@@ -435,14 +440,19 @@ uint32_t quantized(uint32_t x) {
   return p;
 }
 
+// The grids the live scenes ask for: no more CTAs than a domain has tiles.
+Grids frame_grids(const upbd_batch* b) {
+  Grids g;
+  for (int d = 0; d < NUM_DOMAINS; d++)
+    g[d] = std::max(1u, std::min((uint32_t)(b->cps * b->num_sms), quantized(total_blocks(b, d))));
+  return g;
+}
+
 // The frame's launch sequence (GpuSim.encode's pass order, src/gpu/sim.js:
 // 354-391), each pass one persistent launch over every scene.
-int launch_batch_frame(upbd_batch* b, int nsub, bool visc) {
+int launch_batch_frame(upbd_batch* b, int nsub, bool visc, const Grids& grids) {
   const BatchArgs a = batch_args(b);
-  const unsigned G = (unsigned)(b->cps * b->num_sms);
-  auto grid = [&](int d) {  // CTAs of a launch over domain d: no more than it has tiles
-    return std::max(1u, std::min(G, quantized(total_blocks(b, d))));
-  };
+  auto grid = [&](int d) { return (unsigned)grids[d]; };
   const unsigned BT = (unsigned)b->bt;
   cudaStream_t st = b->stream;
   const bool tets = (b->desc.features & UPBD_FEAT_TETS) != 0;
@@ -526,16 +536,26 @@ int enqueue_batch_frame(upbd_batch* b, double dt, int nsub, bool profile) {
   bool visc = false;
   for (auto& kv : b->scenes) visc = visc || kv.second.prm.solid_viscosity > 0;
   if (!profile) {
-    // a graph's grids are those of the scenes at its capture; any grid covers
-    // any table, so the key follows the size in coarse steps only
+    // Any grid covers any table, but a small one takes its time over it: a
+    // graph is captured again, with the larger grids of both, when the scenes
+    // ask for more CTAs in any domain than it has (a mix with the same number
+    // of particles and more solids, say). Grids only grow, by powers of two, so
+    // that ends; too many CTAs find no tile and cost little.
+    Grids need = frame_grids(b);
     const uint64_t key = (uint64_t)nsub | ((uint64_t)(b->bt / 64) << 10) | ((uint64_t)b->cps << 14) | ((uint64_t)visc << 23) |
                          ((uint64_t)quantized(total_blocks(b, D_N)) << 24);
     auto it = b->graphs.find(key);
-    if (it == b->graphs.end()) {
+    bool covers = it != b->graphs.end();
+    if (covers)
+      for (int d = 0; d < NUM_DOMAINS; d++) {
+        covers = covers && need[d] <= it->second.grids[d];
+        need[d] = std::max(need[d], it->second.grids[d]);
+      }
+    if (!covers) {
       cudaGraph_t g;
       BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
       const uint64_t before = b->launches;
-      const int rc = launch_batch_frame(b, nsub, visc);
+      const int rc = launch_batch_frame(b, nsub, visc, need);
       cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
       b->launches = before;
       if (rc) return rc;
@@ -545,13 +565,15 @@ int enqueue_batch_frame(upbd_batch* b, double dt, int nsub, bool profile) {
       const uint64_t nk = graph_kernels(g);
       cudaGraphDestroy(g);
       if (ce != cudaSuccess) return bfail(b, UPBD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ce));
-      it = b->graphs.emplace(key, upbd_batch::Graph{ge, nk}).first;
+      if (it != b->graphs.end()) cudaGraphExecDestroy(it->second.exec);  // (a frame in flight ends first)
+      it = b->graphs.insert_or_assign(key, upbd_batch::Graph{ge, nk, need}).first;
+      b->captures++;
     }
     BCK(b, cudaGraphLaunch(it->second.exec, b->stream));
     b->launches += it->second.kernels;
   } else {
     b->prof_on = true;
-    const int rc = launch_batch_frame(b, nsub, visc);
+    const int rc = launch_batch_frame(b, nsub, visc, frame_grids(b));
     b->prof_on = false;
     if (rc) return rc;
   }
@@ -741,6 +763,7 @@ int upbd_batch_get_info(upbd_batch* b, upbd_batch_info* info) {
   info->block_threads = b->bt;
   info->ctas_per_sm = b->cps;
   info->num_sms = b->num_sms;
+  info->captures = b->captures;
   return UPBD_OK;
 }
 

@@ -8,8 +8,9 @@
  * walk a per-scene offset table (tiles of scene 0, then scene 1, ...), so a
  * scene's arithmetic is the one of upbd_step and its results match a
  * single-scene handle's. The table lives in device memory and the frame is
- * a captured CUDA graph, so scenes join and leave between frames without a
- * new capture.
+ * a captured CUDA graph, so scenes join and leave between frames; the frame is
+ * captured again only where the live scenes outgrow the graph's launch grids,
+ * which follow their sizes in powers of two.
  *
  * Conventions are those of upbd.h: every call returns an int status
  * (UPBD_OK or a negative UPBD_ERR_*), host buffers are caller-owned and
@@ -49,7 +50,8 @@ typedef struct upbd_batch_info {
   uint64_t hbm_budget;
   uint64_t frames;
   uint64_t launches;       /* kernels enqueued (graph replays count their nodes) */
-  int32_t block_threads, ctas_per_sm, num_sms, reserved0;
+  int32_t block_threads, ctas_per_sm, num_sms;
+  int32_t captures;        /* frame graphs captured so far */
   int32_t reserved[8];
 } upbd_batch_info;
 
