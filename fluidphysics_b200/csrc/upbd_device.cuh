@@ -25,6 +25,7 @@ namespace upbd {
 constexpr uint32_t F_ACTIVE = 1u;
 constexpr uint32_t F_GRABBED = 2u;
 constexpr uint32_t C_K = 40u;           // solid contact cache width, src/gpu/wgsl.js:25
+constexpr uint32_t CELL_NONE = 0xffffffffu;  // bucket of an inactive particle in a stateless grid build
 constexpr int SCAN_THREADS = 512;       // 4 counts per thread (SCAN_TILE / 4)
 
 // scratch words (device)

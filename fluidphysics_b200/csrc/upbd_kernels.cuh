@@ -60,14 +60,19 @@ __global__ void __launch_bounds__(256) k_integrate_count(SimView v, const DevPar
 }
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan(SimView v) { b_scan(v, blockIdx.x); }
 // the stateless grid build's forms: the cell size in the arguments, the bucket
-// counts written by the scan that reads them
+// counts written by the scan that reads them. The count alone reads the caller's
+// flags: the passes after it go by the buckets it wrote.
 __global__ void __launch_bounds__(256) k_grid_count(SimView v, double inv_cell) {
   const int i = UPBD_TID;
-  if (i < v.N && (v.flags[i] & F_ACTIVE)) count_particle(v, inv_cell, i, v.pos[i]);
+  if (i >= v.N) return;
+  if (v.flags[i] & F_ACTIVE) count_particle(v, inv_cell, i, v.pos[i]);
+  else v.cell[i] = CELL_NONE;
 }
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_counts(SimView v, uint32_t* counts) {
   b_scan<true>(v, blockIdx.x, counts);
 }
+__global__ void __launch_bounds__(256) k_grid_scatter(SimView v) { b_scatter<false>(v, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_grid_rankfix(SimView v) { b_rankfix<false>(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_scatter(SimView v) { b_scatter(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_rankfix(SimView v) { b_rankfix(v, blockIdx.x); }
 // 5 CTAs of 256 per SM: 48 registers (with 6 and 40 a launch took 32.2 us instead of 31.1)

@@ -179,20 +179,30 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
 
 // Scatter by ticket (gridScatter, src/gpu/wgsl.js:238-245, without its
 // second atomic), and clear the tile totals for the next count.
-// In a scene the particle's cell key goes along, for the rank fix-up.
+// In a scene the particle's cell key goes along, for the rank fix-up. The
+// stateless grid build (SCENE false) goes by the buckets its count wrote, and clears every count here, four a thread, so that its
+// scratch, which outlives the call, is clear for the next one even where calls
+// overlapped (262,139 particles, 2^19 buckets, B200: with the scan storing the
+// zeros behind its reads the build took 35.8 us instead of 34.8).
+template <bool SCENE = true>
 __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i < tile_words(v.num_tiles)) v.tile_sum[i] = 0u;
+  if (!SCENE && i < (v.T + 3) / 4) {
+    if (4 * i + 3 < v.T) *reinterpret_cast<uint4*>(v.counts + 4 * i) = make_uint4(0u, 0u, 0u, 0u);
+    else for (int k = 4 * i; k < v.T; k++) v.counts[k] = 0u;
+  }
   if (i >= v.N) return;
-  const uint32_t f = v.flags[i], h = v.cell[i], ticket = v.ticket[i], key = v.spos ? cell_keys(v)[i] : 0u;
+  const uint32_t f = SCENE ? v.flags[i] : F_ACTIVE, h = v.cell[i], ticket = v.ticket[i],
+                 key = SCENE ? cell_keys(v)[i] : 0u;
   issued(f);
   issued(h);
   issued(ticket);
   issued(key);
-  if (!(f & F_ACTIVE)) return;
+  if (SCENE ? !(f & F_ACTIVE) : h == CELL_NONE) return;
   const uint32_t at = v.start[h] + ticket;
   if (!UPBD_IDX_OK(v, at, v.N)) return;
-  if (v.spos) bucket_pairs(v)[at] = make_uint2((uint32_t)i, key);
+  if (SCENE) bucket_pairs(v)[at] = make_uint2((uint32_t)i, key);
   else v.tmp[at] = (uint32_t)i;  // the stateless grid build
 }
 
@@ -209,22 +219,23 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
 // size (chunk_word). The slot copy of a fluid particle carries
 // its slot where the mass would be, for the density pass's lists; the mass goes
 // to slot_mass.
+template <bool SCENE = true>
 __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   const int i = UPBD_VTID;
   if (i >= v.N) return;
-  const uint32_t f = v.flags[i], h = v.cell[i];
-  real4 p = v.pos[i];
+  const uint32_t f = SCENE ? v.flags[i] : F_ACTIVE, h = v.cell[i];
+  real4 p = make_real4(0.f, 0.f, 0.f, 0.f);
+  if (SCENE) p = v.pos[i];
   issued(f);
   issued(h);
   issued(p);
-  if (!(f & F_ACTIVE)) return;
+  if (SCENE ? !(f & F_ACTIVE) : h == CELL_NONE) return;
   const uint32_t s = v.start[h], e = v.start[h + 1];
   if (!UPBD_IDX_OK(v, e, (uint32_t)v.N + 1u)) return;
   uint32_t rank = 0;
-  if (!v.spos) {  // the stateless grid build has no bucket-ordered copies
+  if (!SCENE) {  // the stateless grid build has no bucket-ordered copies
     for (uint32_t k = s; k < e; k++) rank += (v.tmp[k] > (uint32_t)i) ? 1u : 0u;
     if (UPBD_IDX_OK(v, s + rank, v.N)) v.entries[s + rank] = (uint32_t)i;
-    if (rank == 0u) v.counts[h] = 0u;  // ready for the next count
     return;
   }
   const uint32_t key = cell_keys(v)[i];

@@ -346,8 +346,9 @@ int upbd_groups_device(upbd_sim* sim, int32_t* d_group);
  * pool must not be captured into a CUDA graph (make one call of the largest
  * size first). Every call on a device shares that pool: calls whose work
  * overlaps on the GPU (different streams or threads) race on it, so order
- * them on one stream or with events. All work, including the counts, is
- * enqueued on `stream`; the call does not wait for it. */
+ * them on one stream or with events. `flags` is read by the first pass alone:
+ * what becomes of it later in the call changes nothing. All work, including
+ * the counts, is enqueued on `stream`; the call does not wait for it. */
 int upbd_grid_build(const void* pos4, const void* flags, int32_t n, int32_t table_size,
                     double cell_size, void* counts, void* offsets, void* entries,
                     void* stream);
