@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(256) k_cut_tets(SimView v, const DevParams* __
 }
 
 // Pick: smallest t (Solver.pickSolid, src/solver.js:502-515, in double), the
-// lowest index among the particles at it. t >= 0, so its IEEE bits order like
-// unsigned integers. One launch with the ray in its arguments: each block
+// lowest index among the particles at it. t >= 0 and never -0, so its IEEE bits
+// order like unsigned integers. One launch with the ray in its arguments: each block
 // leaves its best (t, index) in parts, the last one to finish reduces those
 // into mapped host memory. The call is all latency: with the ray copied to the
 // uniform block, a memset, two launches (smallest t, then lowest index) and a
@@ -229,6 +229,7 @@ __device__ __forceinline__ bool pick_t(const SimView& v, const PickRay& ray, int
                pz = __dsub_rn((double)p.z, ray.o[2]);
   t = __dadd_rn(__dadd_rn(__dmul_rn(px, dx), __dmul_rn(py, dy)), __dmul_rn(pz, dz));
   if (!(t >= 0.0)) return false;
+  t = __dadd_rn(t, 0.0);  // -0 (a particle at the origin of the ray) becomes +0
   const double qx = __dsub_rn(px, __dmul_rn(dx, t)), qy = __dsub_rn(py, __dmul_rn(dy, t)),
                qz = __dsub_rn(pz, __dmul_rn(dz, t));
   const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(qx, qx), __dmul_rn(qy, qy)), __dmul_rn(qz, qz));
