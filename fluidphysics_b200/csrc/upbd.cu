@@ -386,6 +386,28 @@ uint64_t count_graph_kernels(cudaGraph_t g) {
   return k;
 }
 
+// A frame as a graph, captured on the handle's own stream (see cap) whatever
+// the user's is.
+int capture_frame(upbd_sim* s, int nsub, uint32_t emit_blocks, bool cut, cudaGraph_t* g) {
+  const cudaStream_t user = s->stream;
+  UPBD_CK(s, cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal));
+  const uint64_t before = s->launches;
+  s->stream = s->cap;
+  const int rc = launch_frame(s, nsub, emit_blocks, cut);
+  s->stream = user;
+  const cudaError_t ce = cudaStreamEndCapture(s->cap, g);
+  s->launches = before;
+  if (rc) {
+    if (ce == cudaSuccess && *g) cudaGraphDestroy(*g);
+    return rc;
+  }
+  if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
+  return UPBD_OK;
+}
+cudaError_t instantiate_frame(cudaGraphExec_t* ge, cudaGraph_t g) {
+  return cudaGraphInstantiate(ge, g, cudaGraphInstantiateFlagUseNodePriority);
+}
+
 // One frame on the stream: GpuSim.encode (src/gpu/sim.js:333-398).
 int enqueue_frame(upbd_sim* s, double h, int nsub, bool profile = false) {
   if (nsub < 1 || nsub > 1000) return fail(s, UPBD_ERR_INVALID, "substeps out of range [1, 1000]");
@@ -426,19 +448,11 @@ int enqueue_frame(upbd_sim* s, double h, int nsub, bool profile = false) {
                          ((uint64_t)visc << 41);
     auto it = s->graphs.find(key);
     if (it == s->graphs.end()) {
-      cudaGraph_t g;
-      const cudaStream_t user = s->stream;
-      UPBD_CK(s, cudaStreamBeginCapture(s->cap, cudaStreamCaptureModeThreadLocal));
-      const uint64_t before = s->launches;
-      s->stream = s->cap;
-      rc = launch_frame(s, nsub, emit_blocks, cut);
-      s->stream = user;
-      cudaError_t ce = cudaStreamEndCapture(s->cap, &g);
-      s->launches = before;
+      cudaGraph_t g = nullptr;
+      rc = capture_frame(s, nsub, emit_blocks, cut, &g);
       if (rc) return rc;
-      if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
       cudaGraphExec_t ge;
-      ce = cudaGraphInstantiate(&ge, g, cudaGraphInstantiateFlagUseNodePriority);
+      const cudaError_t ce = instantiate_frame(&ge, g);
       const uint64_t nk = count_graph_kernels(g);
       cudaGraphDestroy(g);
       if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ce));
@@ -1299,16 +1313,9 @@ int upbd_profile_graph_floor(upbd_sim* s, double dt, int32_t substeps, int32_t r
   if (!s || !floor_ms || !kernel_nodes || substeps < 1 || substeps > 1000 || reps < 1) return UPBD_ERR_INVALID;
   cudaSetDevice(s->device);
   cudaGraph_t g = nullptr;
-  UPBD_CK(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  const uint64_t before = s->launches;
-  int rc = launch_frame(s, substeps, 0u, false);
-  cudaError_t ce = cudaStreamEndCapture(s->stream, &g);
-  s->launches = before;
-  if (rc) {
-    if (g) cudaGraphDestroy(g);
-    return rc;
-  }
-  if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
+  int rc = capture_frame(s, substeps, 0u, false, &g);
+  if (rc) return rc;
+  cudaError_t ce = cudaSuccess;
   size_t n = 0;
   cudaGraphGetNodes(g, nullptr, &n);
   std::vector<cudaGraphNode_t> nodes(n);
@@ -1333,7 +1340,7 @@ int upbd_profile_graph_floor(upbd_sim* s, double dt, int32_t substeps, int32_t r
     nk++;
   }
   cudaGraphExec_t ge;
-  ce = cudaGraphInstantiate(&ge, g, 0);
+  ce = instantiate_frame(&ge, g);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(s, UPBD_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ce));
   cudaEvent_t a = nullptr, b = nullptr;
