@@ -97,8 +97,9 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
 // scanBlocks/scanPartials/scanApply (src/gpu/wgsl.js:180-236) as one launch:
 // block b scans its own SCAN_TILE counts (SCAN_PER consecutive ones per
 // thread), adds the totals of tiles < b (the count's tile counters, all
-// replicas) and writes start[]; the rank fix-up clears the occupied buckets'
-// counts, movement and fluid ends, so that the table is swept once. The counts and the
+// replicas) and writes start[] and the buckets' rows (all empty: the rank
+// fix-up enters the occupied ones' fluid ends, and clears their counts and
+// movement). The counts and the
 // earlier totals are loaded up front so that their latencies overlap, and one
 // block barrier publishes both per-warp sums. COUNTS: the counts themselves go
 // to counts_out. Four counts a thread: with eight (256 threads a block) the
@@ -159,6 +160,11 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
   if (vec) {
     *reinterpret_cast<uint4*>(v.start + t0) = r;
     if (COUNTS) *reinterpret_cast<uint4*>(counts_out + t0) = c;
+    if (v.brow) {
+      uint4* row = reinterpret_cast<uint4*>(v.brow + t0);
+      row[0] = make_uint4(r.x, r.x, r.y, r.y);
+      row[1] = make_uint4(r.z, r.z, r.w, r.w);
+    }
   } else {
     const uint32_t cs[4] = {c.x, c.y, c.z, c.w}, rs[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
@@ -167,6 +173,7 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
       if (idx < v.T) {
         v.start[idx] = rs[k];
         if (COUNTS) counts_out[idx] = cs[k];
+        if (v.brow) v.brow[idx] = make_uint2(rs[k], rs[k]);
       }
     }
   }
@@ -255,7 +262,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   v.entries[slot] = (uint32_t)i;
   v.slot[i] = slot;
   if (rank == 0u) {
-    v.fend[h] = e - solids;
+    v.brow[h].y = e - solids;
     v.counts[h] = 0u;  // ready for the next count
     v.bmove[h] = 0u;   // no movement recorded yet this substep
   }

@@ -191,7 +191,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.drow = cv.take<real4>(2 * (size_t)v.N);
   L.pvrow = cv.take<real4>(2 * (size_t)v.N);
   L.slot = cv.take<uint32_t>(v.N);
-  L.fend = cv.take<uint32_t>(v.T);
+  L.brow = cv.take<uint2>(v.T);
   L.nbr = cv.take<uint32_t>(std::max<size_t>((size_t)v.N * GLF * NL, 1));
   L.ncount = cv.take<uint32_t>(std::max<size_t>((size_t)v.N * GLF, 1));
   L.aoth = cv.take<uint32_t>(std::max<size_t>(hs.adj_other.size(), 1));
@@ -239,7 +239,7 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.drow = (real4*)(base + L.drow);
   v.pvrow = (real4*)(base + L.pvrow);
   v.slot = (uint32_t*)(base + L.slot);
-  v.fend = (uint32_t*)(base + L.fend);
+  v.brow = (uint2*)(base + L.brow);
   v.nbr = (uint32_t*)(base + L.nbr);
   v.ncount = (uint32_t*)(base + L.ncount);
   v.adj_other = (const uint32_t*)(base + L.aoth);
