@@ -84,6 +84,16 @@ def measured_peaks() -> tuple[dict, str]:
     return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}, "fallback"
 
 
+# Kernels that a captured frame runs on the side stream beside the main chain:
+# their time is not the frame's, whatever their share of the eager launches.
+SIDE_STREAM = ("solid_solve",)
+
+
+def dominant_kernel(per_kernel: dict) -> str:
+    """The kernel of the frame's main chain with the largest share."""
+    return max((k for k in per_kernel if k in KERNEL_BYTES and k not in SIDE_STREAM), key=lambda k: per_kernel[k]["share"])
+
+
 def ncu_traffic(kernel: str, workload: str):
     """DRAM bytes per launch from a committed ncu summary, if one exists:
     profiles/traffic.txt lines `kernel workload bytes_per_launch`."""
@@ -764,7 +774,7 @@ def main() -> None:
             per_kernel[nm] = {"share": tot[k] / tot.sum(), "avg_us": avg_ms * 1e3,
                               "launches_per_frame": cnt[k] / P,
                               "gbs": (b / (avg_ms / 1e3) / 1e9) if b else None}
-    dom = max((nm for nm in per_kernel if nm in KERNEL_BYTES), key=lambda n: per_kernel[n]["share"])
+    dom = dominant_kernel(per_kernel)
     peaks, peak_src = measured_peaks()
     hbm = float(peaks.get("hbm_gbs", 6650.0))
     dk = per_kernel[dom]
