@@ -315,8 +315,7 @@ __device__ __forceinline__ void group_cell_hash(real px, real py, real pz, doubl
 // entries in bucket order (PART 0: its fluid entries, PART 1: its solids);
 // lane l of the G group takes candidates c = l, l+G, l+2G, ... so the
 // lanes' shares differ by at most one. For each slot e of its share, in
-// order, a lane calls use(e, load(e)); with U > 1 it issues the loads of U
-// slots before their uses. The bucket ranges are looked up by
+// order, a lane calls use(e, load(e)). The bucket ranges are looked up by
 // their round-robin lanes (cell k by lane k mod G), scanned into sequence
 // offsets by shuffles, and handed over in shared memory. Every lane of the
 // warp must call it; a group with `walk` false has an empty sequence. At most
@@ -327,8 +326,8 @@ static __shared__ uint32_t s_walk_off[256 / GLF][28];   // sequence offset of ce
 // First slot and length of bucket h's fluid (PART 0) or solids (PART 1). A
 // look-up is a scattered read, a cycle of the SM's L1 data path for each lane and
 // word, and the gathers do 27 a cell: with start[h], start[h + 1] and a fluid end
-// that only occupied buckets had, the large scene's first frames of a fall spent
-// 115 us a density launch, with one 8-byte row 106 (B200; settled pool 33.5, 33.1).
+// that only occupied buckets had, a density launch of the large scene's first
+// frames of a fall took 115 us, with one 8-byte row 106 (B200).
 template <int PART>
 __device__ __forceinline__ uint2 bucket_range(const SimView& v, uint32_t h) {
   const uint2 r = __ldg(&v.brow[h]);

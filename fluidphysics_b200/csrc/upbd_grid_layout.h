@@ -33,9 +33,9 @@ UPBD_HD constexpr int tile_words(int num_tiles) { return tile_reps(num_tiles) * 
 // Scratch of one stateless grid build sized for up to n_cap particles and
 // t_cap buckets, in 32-bit words from a 256-byte aligned base: bucket counts
 // [t_cap], arrival tickets, bucket of each particle and the unordered scatter
-// [n_cap each], the scan tile counters, then a params block of params_bytes.
-// The params block holds a double (1 / cell size), so it starts on a 64-word
-// (256-byte) boundary whatever n_cap is; tile_words() does not decrease with
+// [n_cap each], the scan tile counters, then params_bytes of a caller's own on a
+// 64-word (256-byte) boundary (the grid builds take their one constant as a
+// kernel argument and ask for none). tile_words() does not decrease with
 // the tile count, so the layout for the capacity covers every smaller call.
 struct GridScratchLayout {
   size_t counts, ticket, cell, tmp, tiles, params, words;

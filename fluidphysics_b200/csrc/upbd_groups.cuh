@@ -39,7 +39,7 @@ constexpr int GRP_LANES = 8;     // lanes that look for a vertex's first alive c
 
 // Scratch of one call, carved from the density pass's neighbour lists (free
 // between substeps): 11 S words and C + C / 32 + 1 more, C <= 13 S, of the
-// 128 N there are.
+// GLF * NL * N there are.
 struct GroupScratch {
   int32_t* p;       // smallest alive neighbour, or the vertex itself (seed)
   uint32_t* fe;     // first edge (constraint index), GRP_NONE for a seed

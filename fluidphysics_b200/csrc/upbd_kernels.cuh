@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_grid_scatter(SimView v) { b_scatter<fal
 __global__ void __launch_bounds__(256) k_grid_rankfix(SimView v) { b_rankfix<false>(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_scatter(SimView v) { b_scatter(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_rankfix(SimView v) { b_rankfix(v, blockIdx.x); }
-// 5 CTAs of 256 per SM: 48 registers (with 6 and 40 a launch took 32.2 us instead of 31.1)
+// 5 CTAs of 256 per SM: 48 registers (with 6 and 40 a launch took 3 % longer)
 __global__ void __launch_bounds__(256, 5) k_density(SimView v, const DevParams* __restrict__ P, uint32_t window) {
   b_density(v, P, window, blockIdx.x);
 }
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_solid_visc(SimView v, const DevParams* 
 }
 __global__ void __launch_bounds__(256) k_solid_visc_apply(SimView v) { b_solid_visc_apply(v, blockIdx.x); }
 // 4 CTAs of 256 per SM: four list entries in flight without spills (5 CTAs and
-// 48 registers: 26.3 us instead of 23.0 on the default scene)
+// 48 registers: a seventh longer on the default scene)
 template <bool APPLY>
 __global__ void __launch_bounds__(256, 4) k_xsph(SimView v, const DevParams* __restrict__ P, uint32_t window) {
   b_xsph<APPLY>(v, P, window, blockIdx.x);

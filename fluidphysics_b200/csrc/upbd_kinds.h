@@ -1,5 +1,8 @@
 // Kernel classes of the per-kernel timing (upbd_profile_frame,
-// upbd_batch_profile_frame); names through upbd_kernel_name.
+// upbd_batch_profile_frame); names through upbd_kernel_name. The numbers are part
+// of the interface: a class that no launch records any more
+// (K_APPLY_SOLID_CONTACTS, K_XSPH_APPLY: their passes apply their results
+// themselves) keeps its place.
 #pragma once
 
 namespace upbd {

@@ -306,24 +306,29 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
 // Bound by the latency of the shared loads, square roots and shuffles between
 // its instructions (58 % of the issue slots of an active SM). On the default
 // scene's settled pool (65,536 fluid, 120 candidates and 22 listed each; B200,
-// event-timed) a launch takes 29.8 us; a walk of each group of GLF lanes with its
-// own cursor, 46 instructions a candidate, took 42.8 us; on the large scene 121
-// against 173 us. With half a warp a chunk of 4 everywhere it took 40 us (the
-// set-up is shared by half as many), with a warp over 8 consecutive slots of
-// several cells 73 us.
+// an event pair around an eager launch, as all of the following) a launch takes
+// 33.2 us; a walk of each group of GLF lanes with its own cursor, 46 instructions
+// a candidate, took 51.4; in the large scene's splash 99.7 against 117.9. With
+// half a warp a chunk of 4 everywhere it took a third longer (the set-up is shared
+// by half as many), with a warp over 8 consecutive slots of several cells more
+// than twice as long.
 // Where fluid falls apart in drops of one or two particles a cell, a warp a chunk
 // leaves three lanes in four idle and the set-up, some 300 instructions, is
 // paid for two particles. There a warp takes two chunks of up to four, a half
 // each (W = 16): the large scene's first frames of the fall 147 us a warp a
-// chunk, 117 with halves (90 with a cursor a group), the default scene's 48.3
-// and 39.3.
+// chunk, 106 with halves, the default scene's 48.3 and 37.0. A cursor a group
+// took 89 and 34 there, in a kernel of 32 registers; within this one, at 48, it
+// takes 121 and 45, quarters of a warp 124 (a sequence is 64 long: two rounds),
+// lists of slots in shared memory 107 and 38. A launch of its own for such
+// windows would cost every other frame 2 to 3 us a substep.
 constexpr uint32_t STAGE = 4096 / sizeof(real4);     // 256 candidates a warp and round (FP64: 128)
 constexpr size_t STAGE_WARP = STAGE * sizeof(real4);  // dynamic shared bytes per warp
 constexpr uint32_t WINDOW_MAX = 128;                  // places of a block's window
 // Halves where fewer than one chunk in SPARSE of a window has more than four
-// particles. At one in two the default scene's settled pool takes 38.5 us instead
-// of 36.6 and the large scene's splash 2069 us a frame instead of 1966; at one in
-// eight and in 32 the fall's frames 6 to 15 take 1379 and 1399 us instead of 1324.
+// particles. Measured before the look-ups were one row each: at one in two the
+// default scene's settled pool took 38.5 us instead of 36.6 and the large scene's
+// splash 2069 us a frame instead of 1966; at one in eight and in 32 the fall's
+// frames 6 to 15 took 1379 and 1399 us instead of 1324.
 constexpr uint32_t SPARSE = 4;
 
 __device__ __forceinline__ void copy_row_async(real4* dst, const real4* src) {
@@ -1659,11 +1664,11 @@ __device__ __forceinline__ void b_solid_visc_apply(const SimView& v, uint32_t vb
 // Bound by latency (list entry -> row) where the fluid has settled, by the
 // staged walks where it moves. With each group of lanes walking its own buckets
 // in a launch of its own beside the list readers, the default scene's settled
-// pool took 31.5 us (both forms in one launch, B200, event-timed), the large
-// scene's splash 115, a batch of 48 scenes 283; now 23.0, 88 and 228. Position and
-// velocity come as one 32-byte row: with two 16-byte rows 25.7, 103 us. Windows of
-// small chunks go by half-warps as in the density pass: in the large scene's fall
-// 68.7 us, a warp a chunk 90.8.
+// pool took 34.7 us (both forms in one launch; B200, an event pair around an
+// eager launch), the large scene's splash 115.4; now 23.3 and 102.3. Position and
+// velocity come as one 32-byte row: with two 16-byte rows a tenth longer. Windows
+// of small chunks go by half-warps as in the density pass: in the large scene's
+// fall 68 us, a warp a chunk 91.
 constexpr uint32_t XROWS = STAGE / 2;  // candidates staged a round: positions and velocities in the same bytes
 constexpr int XCH = 4;                 // list entries whose loads are in flight together
 template <bool APPLY, int W>
