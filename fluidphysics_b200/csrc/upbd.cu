@@ -1066,9 +1066,11 @@ int upbd_read_grid(upbd_sim* s, uint32_t* counts, uint32_t* offsets, uint32_t* e
   if (!s) return UPBD_ERR_INVALID;
   cudaSetDevice(s->device);
   const size_t T = (size_t)s->v.T;
-  std::vector<uint32_t> off(T + 1);
-  UPBD_CK(s, cudaMemcpyAsync(off.data(), s->v.start, (T + 1) * 4, cudaMemcpyDeviceToHost, s->stream));
+  std::vector<uint2> rows(T + 1);
+  UPBD_CK(s, cudaMemcpyAsync(rows.data(), s->v.brow, (T + 1) * sizeof(uint2), cudaMemcpyDeviceToHost, s->stream));
   UPBD_CK(s, cudaStreamSynchronize(s->stream));
+  std::vector<uint32_t> off(T + 1);
+  for (size_t h = 0; h <= T; h++) off[h] = rows[h].x;
   const uint32_t n = off[T];
   if (n > (uint32_t)s->v.N) return fail(s, UPBD_ERR_INVALID, "grid not built");
   if (offsets) std::memcpy(offsets, off.data(), (T + 1) * 4);
@@ -1207,8 +1209,8 @@ GridPool g_pool;
 // build; this takes 34.8 back to back (B200).
 cudaError_t launch_grid_build(const SimView& v, double inv_cell, uint32_t* counts, cudaStream_t st) {
   k_grid_count<<<blocks_for(v.N), 256, 0, st>>>(v, inv_cell);
-  if (counts) k_scan_counts<<<v.num_tiles, SCAN_THREADS, 0, st>>>(v, counts);
-  else k_scan<<<v.num_tiles, SCAN_THREADS, 0, st>>>(v);
+  if (counts) k_grid_scan<true><<<v.num_tiles, SCAN_THREADS, 0, st>>>(v, counts);
+  else k_grid_scan<false><<<v.num_tiles, SCAN_THREADS, 0, st>>>(v, nullptr);
   k_grid_scatter<<<blocks_for(std::max({v.N, tile_words(v.num_tiles), (v.T + 3) / 4})), 256, 0, st>>>(v);
   k_grid_rankfix<<<blocks_for(v.N), 256, 0, st>>>(v);
   return cudaPeekAtLastError();

@@ -12,7 +12,7 @@
 //   cons[C]    uint4   {a, b, rest float bits, alive}
 //   adj        uint32  [S+1 offsets][2C constraint ids]  (static CSR)
 // Hash grid (rebuilt every substep):
-//   counts[T], start[T+1], entries[N], tmp[N], ticket[N], cell[N], tile_sum
+//   counts[T], brow[T+1], entries[N], tmp[N], ticket[N], cell[N], tile_sum
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -120,7 +120,7 @@ struct SimView {
   uint4* cons;
   const uint32_t* adj;
   uint32_t* counts;
-  uint32_t* start;
+  uint32_t* start;     // first slot of each bucket, T + 1 (the stateless grid build; a scene has brow)
   uint32_t* entries;
   uint32_t* tmp;
   uint32_t* ticket;
@@ -146,8 +146,9 @@ struct SimView {
   real4* pvrow;
   uint32_t* slot;      // slot of particle i in this substep's grid
   // Inside a bucket, entries run in descending index, so fluid (indices >= S)
-  // precede solids: brow[h] = {start[h], end of the fluid} splits bucket h into
-  // its fluid and [end of the fluid, start[h+1]) solid.
+  // precede solids: brow[h] = {first slot, end of the fluid} splits bucket h
+  // into its fluid and [end of the fluid, brow[h+1].x) solid; brow[T].x is the
+  // number of active particles.
   uint2* brow;
   // Density-pass neighbour lists: lane l (of GLF) of the fluid particle at
   // slot e records the slots of its fluid candidates within the list radius
@@ -325,15 +326,17 @@ static __shared__ uint32_t s_walk_off[256 / GLF][28];   // sequence offset of ce
 
 // First slot and length of bucket h's fluid (PART 0) or solids (PART 1). A
 // look-up is a scattered read, a cycle of the SM's L1 data path for each lane and
-// word, and the gathers do 27 a cell: with start[h], start[h + 1] and a fluid end
+// word, and the gathers do 27 a cell: with two bucket starts and a fluid end
 // that only occupied buckets had, a density launch of the large scene's first
 // frames of a fall took 115 us, with one 8-byte row 106 (B200).
 template <int PART>
 __device__ __forceinline__ uint2 bucket_range(const SimView& v, uint32_t h) {
   const uint2 r = __ldg(&v.brow[h]);
   if (PART == 0) return make_uint2(r.x, r.y - r.x);
-  return make_uint2(r.y, __ldg(&v.start[h + 1]) - r.y);
+  return make_uint2(r.y, __ldg(&v.brow[h + 1].x) - r.y);
 }
+// slots taken in this substep's grid
+__device__ __forceinline__ uint32_t active_slots(const SimView& v) { return __ldg(&v.brow[v.T].x); }
 
 // The shared tables of a walk: row g (this lane's group) gets the slot base
 // and sequence offset of each of the 27 cells; returns the sequence length.

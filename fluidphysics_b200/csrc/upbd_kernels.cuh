@@ -68,8 +68,9 @@ __global__ void __launch_bounds__(256) k_grid_count(SimView v, double inv_cell) 
   if (v.flags[i] & F_ACTIVE) count_particle(v, inv_cell, i, v.pos[i]);
   else v.cell[i] = CELL_NONE;
 }
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_counts(SimView v, uint32_t* counts) {
-  b_scan<true>(v, blockIdx.x, counts);
+template <bool COUNTS>
+__global__ void __launch_bounds__(SCAN_THREADS) k_grid_scan(SimView v, uint32_t* counts) {
+  b_scan<COUNTS, false>(v, blockIdx.x, counts);
 }
 __global__ void __launch_bounds__(256) k_grid_scatter(SimView v) { b_scatter<false>(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_grid_rankfix(SimView v) { b_rankfix<false>(v, blockIdx.x); }

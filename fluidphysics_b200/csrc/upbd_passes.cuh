@@ -97,9 +97,9 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
 // scanBlocks/scanPartials/scanApply (src/gpu/wgsl.js:180-236) as one launch:
 // block b scans its own SCAN_TILE counts (SCAN_PER consecutive ones per
 // thread), adds the totals of tiles < b (the count's tile counters, all
-// replicas) and writes start[] and the buckets' rows (all empty: the rank
-// fix-up enters the occupied ones' fluid ends, and clears their counts and
-// movement). The counts and the
+// replicas) and writes the buckets' rows (all empty: the rank fix-up enters the
+// occupied ones' fluid ends, and clears their counts and movement), or in the
+// stateless grid build (SCENE false) start[]. The counts and the
 // earlier totals are loaded up front so that their latencies overlap, and one
 // block barrier publishes both per-warp sums. COUNTS: the counts themselves go
 // to counts_out. Four counts a thread: with eight (256 threads a block) the
@@ -107,7 +107,7 @@ __device__ __forceinline__ void b_integrate_count(const SimView& v, const DevPar
 // which are the launch).
 constexpr int SCAN_PER = SCAN_TILE / SCAN_THREADS;
 static_assert(SCAN_PER == 4, "a thread's counts are one 16-byte row");
-template <bool COUNTS = false>
+template <bool COUNTS = false, bool SCENE = true>
 __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* __restrict__ counts_out = nullptr) {
   __shared__ uint32_t s_scan[SCAN_THREADS / 32];  // per-warp sums of this tile's counts
   __shared__ uint32_t s_prev[SCAN_THREADS / 32];  // per-warp sums of earlier tiles' totals
@@ -158,26 +158,30 @@ __device__ __forceinline__ void b_scan(const SimView& v, uint32_t vb, uint32_t* 
   }
   const uint4 r = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
   if (vec) {
-    *reinterpret_cast<uint4*>(v.start + t0) = r;
-    if (COUNTS) *reinterpret_cast<uint4*>(counts_out + t0) = c;
-    if (v.brow) {
+    if (SCENE) {
       uint4* row = reinterpret_cast<uint4*>(v.brow + t0);
       row[0] = make_uint4(r.x, r.x, r.y, r.y);
       row[1] = make_uint4(r.z, r.z, r.w, r.w);
+    } else {
+      *reinterpret_cast<uint4*>(v.start + t0) = r;
     }
+    if (COUNTS) *reinterpret_cast<uint4*>(counts_out + t0) = c;
   } else {
     const uint32_t cs[4] = {c.x, c.y, c.z, c.w}, rs[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
     for (int k = 0; k < SCAN_PER; k++) {
       const long long idx = t0 + k;
       if (idx < v.T) {
-        v.start[idx] = rs[k];
+        if (SCENE) v.brow[idx] = make_uint2(rs[k], rs[k]);
+        else v.start[idx] = rs[k];
         if (COUNTS) counts_out[idx] = cs[k];
-        if (v.brow) v.brow[idx] = make_uint2(rs[k], rs[k]);
       }
     }
   }
-  if (vb == (uint32_t)v.num_tiles - 1u && tid == SCAN_THREADS - 1) v.start[v.T] = run + sum;
+  if (vb == (uint32_t)v.num_tiles - 1u && tid == SCAN_THREADS - 1) {
+    if (SCENE) v.brow[v.T] = make_uint2(run + sum, run + sum);
+    else v.start[v.T] = run + sum;
+  }
   if (vb == 0 && tid == 0 && v.bmove) {
     v.scratch[SCR_XMOVE] = 0u;
     v.scratch[SCR_FAR] = 0u;
@@ -207,7 +211,7 @@ __device__ __forceinline__ void b_scatter(const SimView& v, uint32_t vb) {
   issued(ticket);
   issued(key);
   if (SCENE ? !(f & F_ACTIVE) : h == CELL_NONE) return;
-  const uint32_t at = v.start[h] + ticket;
+  const uint32_t at = (SCENE ? v.brow[h].x : v.start[h]) + ticket;
   if (!UPBD_IDX_OK(v, at, v.N)) return;
   if (SCENE) bucket_pairs(v)[at] = make_uint2((uint32_t)i, key);
   else v.tmp[at] = (uint32_t)i;  // the stateless grid build
@@ -237,7 +241,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
   issued(h);
   issued(p);
   if (SCENE ? !(f & F_ACTIVE) : h == CELL_NONE) return;
-  const uint32_t s = v.start[h], e = v.start[h + 1];
+  const uint32_t s = SCENE ? v.brow[h].x : v.start[h], e = SCENE ? v.brow[h + 1].x : v.start[h + 1];
   if (!UPBD_IDX_OK(v, e, (uint32_t)v.N + 1u)) return;
   uint32_t rank = 0;
   if (!SCENE) {  // the stateless grid build has no bucket-ordered copies
@@ -284,7 +288,7 @@ __device__ __forceinline__ void b_rankfix(const SimView& v, uint32_t vb) {
 // writes. They take the particles by grid slot: the particles of one bucket sit
 // in consecutive slots and share their 27 neighbour buckets. A particle's own
 // arithmetic does not depend on which group runs it. Groups whose slot holds a
-// solid, or lies past the active count start[T], have no work.
+// solid, or lies past the active count, have no work.
 
 // fluidDensity, src/gpu/wgsl.js:254-279. Every grid entry is active (the
 // grid is built from the active particles of this substep, before bounds).
@@ -682,7 +686,7 @@ __device__ __forceinline__ void b_density(const SimView& v, const DevParams* __r
   extern __shared__ __align__(16) unsigned char s_stage[];
   __shared__ ChunkList s_list;
   const int tid = thread_index();
-  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  const uint32_t nact = active_slots(v), first = vb * window;
   if (first >= nact) return;
   uint32_t halves;
   const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid, halves);
@@ -726,7 +730,7 @@ __device__ __forceinline__ void b_disp(const SimView& v, const DevParams* __rest
   const int h = (int)(threadIdx.x & (DL - 1));
   const real4* __restrict__ rows = v.drow;
   const uint32_t NS = (uint32_t)v.N, eld = min(e0, NS - 1u);
-  const uint32_t nact = __ldg(&v.start[v.T]);
+  const uint32_t nact = active_slots(v);
   const uint32_t i = v.entries[eld];
   real4 pi, di;
   load_row_pair(&rows[2 * (size_t)eld], pi, di);
@@ -1811,7 +1815,7 @@ __device__ __forceinline__ void b_xsph(const SimView& v, const DevParams* __rest
   extern __shared__ __align__(16) unsigned char s_stage[];
   __shared__ ChunkList s_list;
   const int tid = thread_index();
-  const uint32_t nact = __ldg(&v.start[v.T]), first = vb * window;
+  const uint32_t nact = active_slots(v), first = vb * window;
   if (first >= nact) return;
   uint32_t halves;
   const uint32_t chunks = list_chunks(v, s_list, first, window, nact, tid, halves);

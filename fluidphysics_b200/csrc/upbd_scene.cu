@@ -177,7 +177,6 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.cons = cv.take<uint4>(std::max(v.C, 1));
   L.adj = cv.take<uint32_t>(hs.adj.size());
   L.counts = cv.take<uint32_t>(v.T);
-  L.start = cv.take<uint32_t>(v.T + 1);
   L.entries = cv.take<uint32_t>(v.N);
   L.tmp = cv.take<uint32_t>(v.N);
   L.ticket = cv.take<uint32_t>(v.N);
@@ -191,7 +190,7 @@ SceneLayout layout_scene(const upbd_scene_desc& d, const HostScene& hs, SimView&
   L.drow = cv.take<real4>(2 * (size_t)v.N);
   L.pvrow = cv.take<real4>(2 * (size_t)v.N);
   L.slot = cv.take<uint32_t>(v.N);
-  L.brow = cv.take<uint2>(v.T);
+  L.brow = cv.take<uint2>((size_t)v.T + 1);
   L.nbr = cv.take<uint32_t>(std::max<size_t>((size_t)v.N * GLF * NL, 1));
   L.ncount = cv.take<uint32_t>(std::max<size_t>((size_t)v.N * GLF, 1));
   L.aoth = cv.take<uint32_t>(std::max<size_t>(hs.adj_other.size(), 1));
@@ -225,7 +224,6 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.cons = (uint4*)(base + L.cons);
   v.adj = (const uint32_t*)(base + L.adj);
   v.counts = (uint32_t*)(base + L.counts);
-  v.start = (uint32_t*)(base + L.start);
   v.entries = (uint32_t*)(base + L.entries);
   v.tmp = (uint32_t*)(base + L.tmp);
   v.ticket = (uint32_t*)(base + L.ticket);
@@ -239,6 +237,7 @@ void bind_scene(const SceneLayout& L, char* base, SimView& v, DevParams** params
   v.drow = (real4*)(base + L.drow);
   v.pvrow = (real4*)(base + L.pvrow);
   v.slot = (uint32_t*)(base + L.slot);
+  v.start = nullptr;
   v.brow = (uint2*)(base + L.brow);
   v.nbr = (uint32_t*)(base + L.nbr);
   v.ncount = (uint32_t*)(base + L.ncount);

@@ -32,7 +32,7 @@ void build_scene(const upbd_scene_desc& d, HostScene& out);
 
 // Byte offsets of one scene's arrays inside its arena (each 256-byte aligned).
 struct SceneLayout {
-  size_t pos, prev, vel, delta, dens, flags, cons, adj, counts, start, entries, tmp, ticket, cell, tiles;
+  size_t pos, prev, vel, delta, dens, flags, cons, adj, counts, entries, tmp, ticket, cell, tiles;
   size_t tidx, tvol, tadj, mark, spos, drow, pvrow, slot, brow, nbr, ncount, aoth, ascl, ccount, clist;
   size_t trec, tscl, sbuf, smove, bmove, scr, par, conv;
   size_t bytes;
