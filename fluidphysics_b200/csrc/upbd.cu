@@ -1066,11 +1066,22 @@ int upbd_read_grid(upbd_sim* s, uint32_t* counts, uint32_t* offsets, uint32_t* e
   if (!s) return UPBD_ERR_INVALID;
   cudaSetDevice(s->device);
   const size_t T = (size_t)s->v.T;
-  std::vector<uint2> rows(T + 1);
-  UPBD_CK(s, cudaMemcpyAsync(rows.data(), s->v.brow, (T + 1) * sizeof(uint2), cudaMemcpyDeviceToHost, s->stream));
-  UPBD_CK(s, cudaStreamSynchronize(s->stream));
   std::vector<uint32_t> off(T + 1);
-  for (size_t h = 0; h <= T; h++) off[h] = rows[h].x;
+  if (T + 1 <= (size_t)s->v.N * GLF * NL) {
+    // the rows' first words, gathered in the density pass's list memory (free
+    // between substeps): half the bytes to the host (2^18 buckets, 400 us a
+    // call instead of 750)
+    k_bucket_starts<<<blocks_for((long long)T + 1), 256, 0, s->stream>>>(s->v.brow, s->v.nbr, (int)T + 1);
+    s->launches++;
+    UPBD_KCK(s);
+    UPBD_CK(s, cudaMemcpyAsync(off.data(), s->v.nbr, (T + 1) * 4, cudaMemcpyDeviceToHost, s->stream));
+    UPBD_CK(s, cudaStreamSynchronize(s->stream));
+  } else {  // a table far larger than the scene
+    std::vector<uint2> rows(T + 1);
+    UPBD_CK(s, cudaMemcpyAsync(rows.data(), s->v.brow, (T + 1) * sizeof(uint2), cudaMemcpyDeviceToHost, s->stream));
+    UPBD_CK(s, cudaStreamSynchronize(s->stream));
+    for (size_t h = 0; h <= T; h++) off[h] = rows[h].x;
+  }
   const uint32_t n = off[T];
   if (n > (uint32_t)s->v.N) return fail(s, UPBD_ERR_INVALID, "grid not built");
   if (offsets) std::memcpy(offsets, off.data(), (T + 1) * 4);

@@ -9,10 +9,10 @@
 // pass body the single-scene kernels run (upbd_passes.cuh) on that tile.
 //
 // The table, the SimViews and the uniform blocks live in one device buffer
-// whose address never changes; the frame is captured once per shape into a
-// CUDA graph whose kernels read the scene count from that buffer, so adding
-// or removing scenes only rewrites the table (one stream-ordered copy before
-// the next replay). Scene arenas come from a first-fit pool of large device
+// whose address never changes; the frame is captured into a CUDA graph whose
+// kernels read the scene count from that buffer, so adding or removing scenes
+// only rewrites the table (one stream-ordered copy before the next replay),
+// unless they outgrow the graph's launch grids. Scene arenas come from a first-fit pool of large device
 // chunks, bounded by the HBM budget.
 #include <cuda_runtime.h>
 

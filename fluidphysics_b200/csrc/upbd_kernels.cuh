@@ -74,6 +74,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_grid_scan(SimView v, uint32_t*
 }
 __global__ void __launch_bounds__(256) k_grid_scatter(SimView v) { b_scatter<false>(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_grid_rankfix(SimView v) { b_rankfix<false>(v, blockIdx.x); }
+// the first words of n bucket rows
+__global__ void __launch_bounds__(256) k_bucket_starts(const uint2* __restrict__ rows, uint32_t* __restrict__ out, int n) {
+  const int h = UPBD_TID;
+  if (h < n) out[h] = rows[h].x;
+}
 __global__ void __launch_bounds__(256) k_scatter(SimView v) { b_scatter(v, blockIdx.x); }
 __global__ void __launch_bounds__(256) k_rankfix(SimView v) { b_rankfix(v, blockIdx.x); }
 // 5 CTAs of 256 per SM: 48 registers (with 6 and 40 a launch took 3 % longer)
